@@ -31,7 +31,7 @@ struct MatScratch {
     int id[kSlots];
     int count;                // distinct tuples inserted
     int err;                  // 1: a poll expired, 2: the table filled up
-    int nmat;                 // result: number of materials, 0 = index unusable
+    MaterialInfo info;        // result
 };
 
 __device__ __forceinline__ unsigned mix(uint4 k)
@@ -126,21 +126,27 @@ __global__ void k_mat_insert(const float *Ca, const float *Cb, const float *Da, 
 __global__ void k_mat_compact(MatScratch *S, float4 *tab)
 {
     int n = 0;
+    bool simple = true;
+    unsigned db = 0;
     for (int h = 0; h < kSlots; ++h) {
         if (S->state[h] != 2u) continue;
+        if (n == 0) db = S->key[h].w;
+        simple = simple && S->key[h].x == 0x3f800000u && S->key[h].z == 0x3f800000u && S->key[h].w == db;
         if (n < kMaxMaterials) {
             const uint4 k = S->key[h];
             tab[n] = make_float4(__uint_as_float(k.x), __uint_as_float(k.y), __uint_as_float(k.z), __uint_as_float(k.w));
         }
         S->id[h] = n++;
     }
-    S->nmat = (S->err || n > kMaxMaterials || n != S->count) ? 0 : n;
+    S->info.nmat = (S->err || n > kMaxMaterials || n != S->count) ? 0 : n;
+    S->info.simple = S->info.nmat > 0 && simple;
+    S->info.db = __uint_as_float(db);
 }
 
 __global__ void k_mat_index(const float *Ca, const float *Cb, const float *Da, const float *Db, Nodes N,
                             const MatScratch *S, unsigned char *mat)
 {
-    if (S->nmat == 0) return;
+    if (S->info.nmat == 0) return;
     const float *c[4] = {Ca, Cb, Da, Db};
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < N.n; q += stride) {
@@ -157,11 +163,11 @@ __global__ void k_mat_index(const float *Ca, const float *Cb, const float *Da, c
 
 }  // namespace
 
-int build_material_index(const float *const coef[4], const Layout &L, unsigned char *mat, float *tab, int *nmat,
+int build_material_index(const float *const coef[4], const Layout &L, unsigned char *mat, float *tab, MaterialInfo *info,
                          cudaStream_t s)
 {
-    PTK_CHECK_ARG(coef && mat && tab && nmat, "NULL argument");
-    *nmat = 0;
+    PTK_CHECK_ARG(coef && mat && tab && info, "NULL argument");
+    *info = MaterialInfo{};
     MatScratch *S = nullptr;
     int rc = pool_alloc(sizeof(MatScratch), s, (void **)&S);
     if (rc) return rc;
@@ -173,11 +179,11 @@ int build_material_index(const float *const coef[4], const Layout &L, unsigned c
     k_mat_index<<<grid, 256, 0, s>>>(coef[0], coef[1], coef[2], coef[3], N, S, mat);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(3);
-    int h = 0;
-    PTK_CUDA_TRY(cudaMemcpyAsync(&h, &S->nmat, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MaterialInfo h;
+    PTK_CUDA_TRY(cudaMemcpyAsync(&h, &S->info, sizeof h, cudaMemcpyDeviceToHost, s));
     PTK_CUDA_TRY(cudaStreamSynchronize(s));
     pool_free(S, s);
-    *nmat = h;
+    *info = h;
     return PTK_OK;
 }
 

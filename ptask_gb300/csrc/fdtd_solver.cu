@@ -85,12 +85,16 @@ struct ptk_solver {
     int tma_by = 0;
     unsigned char *mat = nullptr;   // material index of the coefficients (one byte per node)
     float *mat_tab = nullptr;       // its table, kMaxMaterials x (Ca, Cb, Da, Db)
-    int nmat = 0;                   // materials in the table; 0 = per-cell arrays only
+    MaterialInfo minfo{};           // materials in the table; nmat 0 = per-cell arrays only
     bool mat_enabled = true;
     long long *d_face0 = nullptr;   // {0, face nodes}: the staged path advances faces per chunk
     long long faces = 0;
     int *d_work = nullptr;          // staged path: tile counters, one per step of a chunk
     int total_tiles = 0;
+    bool resident = false;          // the grid fits on chip: staged shapes run whole runs in one launch
+    ResidentPlan rplan{};
+    ulonglong2 *d_xch = nullptr;    // its ghost rows in flight
+    unsigned *d_seq = nullptr;      // and sequence numbers
     InstDesc *d_desc = nullptr;
     int *d_tile0 = nullptr;
     cudaStream_t cap = nullptr;   // capture stream
@@ -107,7 +111,7 @@ namespace ptk {
 // the index).
 static bool use_mat(const ptk_solver *s)
 {
-    return s->stages > 0 && s->mat_enabled && s->nmat > 0 && yee_bulk_smem_bytes(s->by, s->stages, true) > 0;
+    return s->stages > 0 && s->mat_enabled && s->minfo.nmat > 0 && yee_bulk_smem_bytes(s->by, s->stages, true) > 0;
 }
 
 struct RunShape {
@@ -127,10 +131,10 @@ static RunShape run_shape(const ptk_solver *s)
 
 static int rebuild_material(ptk_solver *s, cudaStream_t st)
 {
-    s->nmat = 0;
+    s->minfo = MaterialInfo{};
     if (!s->mat_enabled) return PTK_OK;
     const float *const c[4] = {s->coef[0], s->coef[1], s->coef[2], s->coef[3]};
-    return build_material_index(c, s->L, s->mat, s->mat_tab, &s->nmat, st);
+    return build_material_index(c, s->L, s->mat, s->mat_tab, &s->minfo, st);
 }
 
 static InstDesc host_desc(const ptk_solver *s, int steps_left)
@@ -151,7 +155,7 @@ static InstDesc host_desc(const ptk_solver *s, int steps_left)
     if (rs.mat) {
         d.mat = s->mat;
         d.mat_tab = s->mat_tab;
-        d.nmat = s->nmat;
+        d.nmat = s->minfo.nmat;
     }
     plan_tiles(d, rs.by, s->kc, rs.stages > 0 ? yee_bulk_tile_vec(rs.by) : s->vec);
     if (rs.stages > 0) d.face_tiles = 0;   // faces: launch_yee_faces_steps, once per chunk
@@ -241,11 +245,45 @@ static int solver_graph(ptk_solver *s, int len, cudaGraphExec_t *out)
 
 static constexpr int kChunk = 32;   // fused steps per replayed graph
 
+// A run of this many steps or more on a grid that fits on chip is one resident launch
+// (fdtd_resident.cu) instead of a step kernel per time step.
+static constexpr int kResidentSteps = 8;
+
+static int run_resident(ptk_solver *s, int steps, cudaStream_t st)
+{
+    ResidentArgs a{};
+    const int p0 = s->step & 1, p1 = (s->step + steps) & 1;
+    for (int f = 0; f < 6; ++f) {
+        a.in[f] = s->buf[p0][f];
+        a.out[f] = s->buf[p1][f];
+    }
+    for (int c = 0; c < 4; ++c) a.coef[c] = s->coef[c];
+    const int coef = s->mat_enabled && s->minfo.simple ? COEF_SIMPLE : COEF_DENSE;
+    a.db = s->minfo.db;
+    a.wave = s->wave;
+    a.src = s->nwave > 0 ? s->src : -1;
+    a.nwave = s->nwave;
+    a.step = s->step;
+    a.steps = steps;
+    a.nx = s->L.nx; a.ny = s->L.ny; a.nz = s->L.nz; a.pitch = s->L.pitch;
+    a.plane = s->L.plane;
+    a.cx = s->p.Cx; a.cy = s->p.Cy; a.cz = s->p.Cz;
+    a.xch = s->d_xch;
+    a.seq = s->d_seq;
+    a.err = s->d_err;
+    int rc = launch_yee_resident(s->rplan, coef, a, st);
+    if (rc) return rc;
+    s->last_launches = 1;
+    s->step += steps;
+    return PTK_OK;
+}
+
 int solver_run(ptk_solver *s, int steps, cudaStream_t st)
 {
     if (steps < 0) return set_error(PTK_ERR_INVALID, "negative step count");
     s->last_launches = 0;
     if (steps == 0) return PTK_OK;
+    if (s->resident && s->stages > 0 && steps >= kResidentSteps) return run_resident(s, steps, st);
     int rc = solver_sync_desc(s, steps, st);
     if (rc) return rc;
     int left = steps;
@@ -311,6 +349,15 @@ try {
     if (rc == PTK_OK) cudaMemsetAsync(s->mat, 0, (size_t)s->L.total, st);
     if (rc == PTK_OK) rc = pool_alloc(2 * sizeof(long long), st, (void **)&s->d_face0);
     if (rc == PTK_OK) rc = pool_alloc(sizeof(int) * kChunk, st, (void **)&s->d_work);
+    if (rc == PTK_OK && plan_resident(p->Nx, p->Ny, p->Nz, &s->rplan)) {
+        const size_t nseq = sizeof(unsigned) * s->rplan.nby * s->rplan.nbz;
+        rc = pool_alloc(s->rplan.xch_bytes, st, (void **)&s->d_xch);
+        if (rc == PTK_OK) rc = pool_alloc(nseq, st, (void **)&s->d_seq);
+        if (rc == PTK_OK && (cudaMemsetAsync(s->d_xch, 0, s->rplan.xch_bytes, st) != cudaSuccess ||
+                             cudaMemsetAsync(s->d_seq, 0, nseq, st) != cudaSuccess))
+            rc = set_error(PTK_ERR_CUDA, "exchange buffer reset failed");
+        s->resident = rc == PTK_OK;
+    }
     if (rc == PTK_OK) {
         s->faces = face_nodes(p->Nx, p->Ny, p->Nz);
         const long long f0[2] = {0, s->faces};   // pageable: staged before the call returns
@@ -359,6 +406,8 @@ int ptk_solver_destroy(ptk_solver *s)
         pool_free(s->mat_tab, st);
         pool_free(s->d_face0, st);
         pool_free(s->d_work, st);
+        pool_free(s->d_xch, st);
+        pool_free(s->d_seq, st);
         if (s->cap) cudaStreamDestroy(s->cap);
     }
     cudaStreamSynchronize(st);
@@ -548,7 +597,7 @@ int ptk_solver_use_material_index(ptk_solver *s, int enable, void *stream)
 int ptk_solver_material_count(const ptk_solver *s, int *nmat)
 {
     PTK_CHECK_ARG(s && nmat, "NULL argument");
-    *nmat = s->mat_enabled ? s->nmat : 0;
+    *nmat = s->mat_enabled ? s->minfo.nmat : 0;
     return PTK_OK;
 }
 
@@ -715,6 +764,8 @@ try {
     const int staged[17][2] = {{4, 2}, {4, 3}, {4, 4}, {4, 5}, {4, 6}, {8, 2}, {8, 3}, {8, 4}, {8, 5}, {8, 6},
                                {10, 4}, {10, 5}, {11, 4}, {23, 3}, {23, 4}, {7, 3}, {7, 4}};
     for (const auto &bs : staged) {
+        // grids that fit on chip: a staged shape's runs are resident launches, whatever its tiles
+        if (s->resident && !(bs[0] == 11 && bs[1] == 4)) continue;
         const bool m = yee_bulk_smem_bytes(bs[0], bs[1], true) > 0;
         add(bs[0], yee_bulk_tile_vec(bs[0]), bs[1], yee_bulk_resident_ctas(bs[0], bs[1], m));
     }

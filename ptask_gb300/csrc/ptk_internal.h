@@ -96,9 +96,14 @@ constexpr int kMaxMaterials = 256;
 // Per-node material index of an instance's padded coefficient arrays (Ca, Cb, Da, Db): the
 // distinct tuples of the nodes (i <= Nx, j <= Ny, k <= Nz; row padding excluded) are gathered on
 // the device; if there are at most kMaxMaterials of them, `mat` (L.total bytes, padding left as
-// is) receives each node's id and `tab` (kMaxMaterials x 4 floats) the tuples, and *nmat their
-// count; otherwise *nmat = 0 and nothing else is written.  Synchronises `s`.
-int build_material_index(const float *const coef[4], const Layout &L, unsigned char *mat, float *tab, int *nmat,
+// is) receives each node's id and `tab` (kMaxMaterials x 4 floats) the tuples, and info->nmat their
+// count; otherwise info->nmat = 0 and the index must not be used.  Synchronises `s`.
+struct MaterialInfo {
+    int nmat;       // materials in the table, 0 = no index
+    int simple;     // every material has Ca = Da = 1 and the same Db (lossless, nothing magnetic)
+    float db;       // that Db
+};
+int build_material_index(const float *const coef[4], const Layout &L, unsigned char *mat, float *tab, MaterialInfo *info,
                          cudaStream_t s);
 // Encode the tensor maps of `d`'s arrays for the staged kernel with `by` tile rows into host
 // memory (kTmaSetBytes).
@@ -154,6 +159,41 @@ int leftover_depths(int nx, int ny, int nz, int by, int vec, int resident, int *
 // CTAs of the step kernel with `by` rows (and `vec`) that fit on the whole GPU at once.
 int yee_resident_ctas(int by);
 int yee_resident_ctas(int by, int vec);
+
+// ---------------------------------------------------------------------------------------------
+// A whole run in one cooperative launch, for grids whose fields fit on chip (fdtd_resident.cu).
+// ---------------------------------------------------------------------------------------------
+struct ResidentPlan {
+    int by, bz;            // brick: Nx x by x bz cells
+    int nby, nbz;          // bricks in y and z, one CTA each
+    int lw, lwp;           // units (four x cells) per row; float4 slots of a row with its wall node
+    int kz, nzc, threads;  // planes per thread, columns of kz planes per brick, CTA size
+    int items;             // ghost units a thread sends and receives
+    size_t smem, xch_bytes;
+};
+// Coefficients: Ca = Da = 1 and one Db everywhere (Cb per node), or all four per node.
+enum { COEF_SIMPLE = 0, COEF_DENSE = 1 };
+struct ResidentArgs {
+    const float *in[6];
+    float *out[6];             // may be `in`
+    const float *coef[4];      // padded arrays
+    float db;                  // COEF_SIMPLE: the one Db
+    const float *wave;
+    long long src;             // padded index of the Ez source node, -1 = none
+    int nwave, step, steps;    // wave[step] is added after the first step of the run
+    int nx, ny, nz, pitch;
+    long long plane;
+    float cx, cy, cz;
+    ulonglong2 *xch;           // plan.xch_bytes, zeroed when made, then kept from run to run
+    unsigned *seq;             // one counter per brick, likewise
+    int *err;                  // raised when a bounded wait expires
+    // set by the launcher: the plan, and byte offsets and strides in shared memory
+    int lw, lwp, by, bz, nby, nbz, kz, threads, half, base[6], row, plane_e, plane_h, below, fail;
+};
+// The plan for a grid; false when it does not fit on chip.
+bool plan_resident(int nx, int ny, int nz, ResidentPlan *out);
+int launch_yee_resident(const ResidentPlan &p, int coef, ResidentArgs a, cudaStream_t s);
+
 int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s);
 int launch_pack_field(const float *src, int ex, int ey, int ez, const Layout &L, float *dst0,
                       float *dst1, cudaStream_t s);
