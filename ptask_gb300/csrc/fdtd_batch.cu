@@ -321,6 +321,7 @@ InstDesc instance_desc(const ptk_server *s, const Inst *in)
     d.src = in->nwave ? in->src : -1;
     d.nwave = in->nwave;
     d.step = in->done;
+    d.par = in->done & 1;
     d.steps_left = in->steps_total - in->done;
     d.tma = in->tma;
     if (s->stages) {

@@ -114,7 +114,7 @@ k_yee_step(const InstDesc *__restrict__ insts, const int *__restrict__ tile0, in
     if (s_off >= D->steps_left) continue;
     const int lt = t - __ldg(tile0 + lo);
     const int step = D->step + s_off;
-    const int par = step & 1;
+    const int par = (D->par + s_off) & 1;
     const int nmain = D->tiles_x * D->tiles_y * D->tiles_z;
     if (lt >= nmain) {
         yee_faces(D, par, lt - nmain, 32 * (BY + 1) * kFaceCellsPerThread);
@@ -290,7 +290,7 @@ k_yee_step(const InstDesc *__restrict__ insts, const int *__restrict__ tile0, in
     }   // tile loop
 }
 
-__global__ void k_advance(InstDesc *insts, int ninst, int nsteps)
+__global__ void k_advance(InstDesc *insts, int ninst, int nsteps, int flips)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= ninst) return;
@@ -299,6 +299,7 @@ __global__ void k_advance(InstDesc *insts, int ninst, int nsteps)
     if (n > 0) {
         d.step += n;
         d.steps_left -= n;
+        d.par = (d.par + (flips < 0 ? n : flips)) & 1;
     }
 }
 
@@ -418,10 +419,10 @@ int yee_resident_ctas(int by, int vec)
 
 int yee_resident_ctas(int by) { return yee_resident_ctas(by, 4); }
 
-int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s)
+int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s, int flips)
 {
     if (ninst <= 0) return PTK_OK;
-    k_advance<<<(ninst + 127) / 128, 128, 0, s>>>(d_insts, ninst, nsteps);
+    k_advance<<<(ninst + 127) / 128, 128, 0, s>>>(d_insts, ninst, nsteps, flips);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return PTK_OK;

@@ -59,10 +59,10 @@ static void default_tiles(int nx, int ny, int nz, int *by, int *kc, int *vec)
 }
 
 struct GraphKey {
-    int len, by, kc, vec, stages;
+    int len, by, kc, vec, stages, pair;
     bool operator<(const GraphKey &o) const
     {
-        return std::tie(len, by, kc, vec, stages) < std::tie(o.len, o.by, o.kc, o.vec, o.stages);
+        return std::tie(len, by, kc, vec, stages, pair) < std::tie(o.len, o.by, o.kc, o.vec, o.stages, o.pair);
     }
 };
 
@@ -79,6 +79,7 @@ struct ptk_solver {
     int nwave = 0;
     long long src = -1;
     int step = 0;              // host mirror of the device step counter
+    int par = 0;               // buffer that holds the fields
     int by = 0, kc = 0, vec = 4, stages = 0;
     int *d_err = nullptr;      // raised by the staged kernel if a bounded wait expires
     void *d_tma = nullptr;     // tensor maps of the staged kernel (encoded for tma_by rows)
@@ -95,6 +96,11 @@ struct ptk_solver {
     ResidentPlan rplan{};
     ulonglong2 *d_xch = nullptr;    // its ghost rows in flight
     unsigned *d_seq = nullptr;      // and sequence numbers
+    bool pair = false;              // staged shapes take long runs two steps at a time (fdtd_step_pair.cu)
+    PairPlan pplan{};
+    bool pair_maps = false;         // its tensor maps are encoded
+    bool fused_ready = false;       // prepare_fused has run
+    bool plain = false;             // the autotuner compares tile shapes by their own kernels
     InstDesc *d_desc = nullptr;
     int *d_tile0 = nullptr;
     cudaStream_t cap = nullptr;   // capture stream
@@ -129,6 +135,35 @@ static RunShape run_shape(const ptk_solver *s)
     return {s->by >= 8 ? 8 : 4, 4, false};
 }
 
+// What the resident and the two-step kernel need, made when a staged shape is first set: the plan, the
+// exchange buffer (zeroed once) or the tensor maps' place.
+static int prepare_fused(ptk_solver *s)
+{
+    if (s->fused_ready) return PTK_OK;
+    s->fused_ready = true;
+    cudaStream_t st = default_stream();
+    void *maps = nullptr;
+    int rc = PTK_OK;
+    if (plan_resident(s->L.nx, s->L.ny, s->L.nz, &s->rplan)) {
+        const size_t nseq = sizeof(unsigned) * s->rplan.nby * s->rplan.nbz;
+        rc = pool_alloc(s->rplan.xch_bytes, st, (void **)&s->d_xch);
+        if (rc == PTK_OK) rc = pool_alloc(nseq, st, (void **)&s->d_seq);
+        if (rc == PTK_OK) {
+            PTK_CUDA_TRY(cudaMemsetAsync(s->d_xch, 0, s->rplan.xch_bytes, st));
+            PTK_CUDA_TRY(cudaMemsetAsync(s->d_seq, 0, nseq, st));
+            s->resident = true;
+        }
+    } else if (plan_pair(s->L.nx, s->L.ny, s->L.nz, &s->pplan) && (rc = pool_alloc(kTmaSetBytes, st, &maps)) == PTK_OK) {
+        s->pplan.args.tma = maps;
+        for (int b = 0; b < 2; ++b)
+            for (int f = 0; f < 6; ++f) s->pplan.args.buf[b][f] = s->buf[b][f];
+        s->pair = true;
+    }
+    if (rc) clear_error();   // no room for it: the tile shape's own kernel runs
+    PTK_CUDA_TRY(cudaStreamSynchronize(st));   // runs may come on any stream
+    return PTK_OK;
+}
+
 static int rebuild_material(ptk_solver *s, cudaStream_t st)
 {
     s->minfo = MaterialInfo{};
@@ -150,6 +185,7 @@ static InstDesc host_desc(const ptk_solver *s, int steps_left)
     d.src = s->nwave > 0 ? s->src : -1;
     d.nwave = s->nwave;
     d.step = s->step;
+    d.par = s->par;
     d.steps_left = steps_left;
     const RunShape rs = run_shape(s);
     if (rs.mat) {
@@ -197,10 +233,11 @@ static void drop_graphs(ptk_solver *s)
 }
 
 // Graph of `len` fused steps + one advance for this solver's current tile shape.
-static int solver_graph(ptk_solver *s, int len, cudaGraphExec_t *out)
+static int solver_graph(ptk_solver *s, int len, bool pair, cudaGraphExec_t *out)
 {
     const RunShape rs = run_shape(s);
-    GraphKey key{len, rs.by, s->kc, s->vec, rs.stages * 2 + (rs.mat ? 1 : 0)};
+    const int mode = s->minfo.simple ? PAIR_SIMPLE : PAIR_TABLE;
+    GraphKey key{len, rs.by, s->kc, s->vec, rs.stages * 2 + (rs.mat ? 1 : 0), pair ? 1 + mode : 0};
     auto it = s->graphs.find(key);
     if (it != s->graphs.end()) {
         *out = it->second;
@@ -219,13 +256,16 @@ static int solver_graph(ptk_solver *s, int len, cudaGraphExec_t *out)
         else
             count_launches(1);
     }
-    for (int q = 0; q < len && rc == PTK_OK; ++q)
+    const int pairs = pair ? len / 2 : 0, flips = len - pairs;
+    for (int q = 0; q < pairs && rc == PTK_OK; ++q) rc = launch_yee_pair(s->d_desc, s->pplan, mode, q, s->d_err, s->cap);
+    for (int q = 2 * pairs; q < len && rc == PTK_OK; ++q)
         rc = rs.stages > 0
                  ? launch_yee_step_bulk(s->d_desc, s->d_tile0, 1, s->total_tiles, q, rs.by, rs.stages, grid, s->d_err,
-                                        s->cap, s->d_work, rs.mat, /*lazy=*/true)
+                                        s->cap, s->d_work, rs.mat, /*lazy=*/true, q - pairs)
                  : launch_yee_step_v(s->d_desc, s->d_tile0, 1, s->total_tiles, q, s->by, s->vec, 0, s->cap);
-    if (rc == PTK_OK && rs.stages > 0) rc = launch_yee_faces_steps(s->d_desc, s->d_face0, 1, s->faces, 0, len, s->cap);
-    if (rc == PTK_OK) rc = launch_advance(s->d_desc, 1, len, s->cap);
+    if (rc == PTK_OK && rs.stages > 0)
+        rc = launch_yee_faces_steps(s->d_desc, s->d_face0, 1, s->faces, 0, len, s->cap, flips);
+    if (rc == PTK_OK) rc = launch_advance(s->d_desc, 1, len, s->cap, flips);
     set_capturing(false);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->cap, &g);
@@ -248,15 +288,14 @@ static constexpr int kChunk = 32;   // fused steps per replayed graph
 // A run of this many steps or more on a grid that fits on chip is one resident launch
 // (fdtd_resident.cu) instead of a step kernel per time step.
 static constexpr int kResidentSteps = 8;
+// Larger grids with a material index take runs of this many steps or more two steps per launch
+// (fdtd_step_pair.cu); shorter ones run the tile shape that was set.
+static constexpr int kPairSteps = 16;
 
 static int run_resident(ptk_solver *s, int steps, cudaStream_t st)
 {
     ResidentArgs a{};
-    const int p0 = s->step & 1, p1 = (s->step + steps) & 1;
-    for (int f = 0; f < 6; ++f) {
-        a.in[f] = s->buf[p0][f];
-        a.out[f] = s->buf[p1][f];
-    }
+    for (int f = 0; f < 6; ++f) a.in[f] = a.out[f] = s->buf[s->par][f];   // in place (two steps or more)
     for (int c = 0; c < 4; ++c) a.coef[c] = s->coef[c];
     const int coef = s->mat_enabled && s->minfo.simple ? COEF_SIMPLE : COEF_DENSE;
     a.db = s->minfo.db;
@@ -283,18 +322,30 @@ int solver_run(ptk_solver *s, int steps, cudaStream_t st)
     if (steps < 0) return set_error(PTK_ERR_INVALID, "negative step count");
     s->last_launches = 0;
     if (steps == 0) return PTK_OK;
-    if (s->resident && s->stages > 0 && steps >= kResidentSteps) return run_resident(s, steps, st);
+    if (s->resident && s->stages > 0 && steps >= kResidentSteps && !s->plain) return run_resident(s, steps, st);
     int rc = solver_sync_desc(s, steps, st);
     if (rc) return rc;
+    const bool pair = s->pair && run_shape(s).mat && steps >= kPairSteps && !s->plain;
+    if (pair && !s->pair_maps) {   // the arrays never move: encoded once
+        alignas(64) unsigned char maps[kTmaSetBytes];
+        InstDesc e = host_desc(s, steps);
+        e.mat = s->mat;
+        rc = encode_pair_maps(e, s->pplan, maps);
+        if (rc) return rc;
+        PTK_CUDA_TRY(cudaStreamSynchronize(st));
+        PTK_CUDA_TRY(cudaMemcpy(const_cast<void *>(s->pplan.args.tma), maps, kTmaSetBytes, cudaMemcpyHostToDevice));
+        s->pair_maps = true;
+    }
     int left = steps;
     while (left > 0) {
-        const int len = left >= kChunk ? kChunk : left;
+        const int len = left >= kChunk ? kChunk : left, flips = pair ? len - len / 2 : len;
         cudaGraphExec_t ex;
-        rc = solver_graph(s, len, &ex);
+        rc = solver_graph(s, len, pair, &ex);
         if (rc) return rc;
         PTK_CUDA_TRY(cudaGraphLaunch(ex, st));
-        count_graph_launch(len + 1);
-        s->last_launches += len + 1;
+        count_graph_launch(flips + 1);
+        s->last_launches += flips + 1;
+        s->par = (s->par + flips) & 1;
         left -= len;
     }
     s->step += steps;
@@ -349,15 +400,6 @@ try {
     if (rc == PTK_OK) cudaMemsetAsync(s->mat, 0, (size_t)s->L.total, st);
     if (rc == PTK_OK) rc = pool_alloc(2 * sizeof(long long), st, (void **)&s->d_face0);
     if (rc == PTK_OK) rc = pool_alloc(sizeof(int) * kChunk, st, (void **)&s->d_work);
-    if (rc == PTK_OK && plan_resident(p->Nx, p->Ny, p->Nz, &s->rplan)) {
-        const size_t nseq = sizeof(unsigned) * s->rplan.nby * s->rplan.nbz;
-        rc = pool_alloc(s->rplan.xch_bytes, st, (void **)&s->d_xch);
-        if (rc == PTK_OK) rc = pool_alloc(nseq, st, (void **)&s->d_seq);
-        if (rc == PTK_OK && (cudaMemsetAsync(s->d_xch, 0, s->rplan.xch_bytes, st) != cudaSuccess ||
-                             cudaMemsetAsync(s->d_seq, 0, nseq, st) != cudaSuccess))
-            rc = set_error(PTK_ERR_CUDA, "exchange buffer reset failed");
-        s->resident = rc == PTK_OK;
-    }
     if (rc == PTK_OK) {
         s->faces = face_nodes(p->Nx, p->Ny, p->Nz);
         const long long f0[2] = {0, s->faces};   // pageable: staged before the call returns
@@ -408,6 +450,7 @@ int ptk_solver_destroy(ptk_solver *s)
         pool_free(s->d_work, st);
         pool_free(s->d_xch, st);
         pool_free(s->d_seq, st);
+        pool_free(const_cast<void *>(s->pplan.args.tma), st);
         if (s->cap) cudaStreamDestroy(s->cap);
     }
     cudaStreamSynchronize(st);
@@ -446,7 +489,7 @@ int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *str
     PTK_CHECK_ARG(s && f, "NULL argument");
     std::lock_guard<std::mutex> lk(s->mu);
     cudaStream_t st = S(stream);
-    const int par = s->step & 1;
+    const int par = s->par;
     for (int q = 0; q < 6; ++q) {
         PTK_CHECK_ARG(f[q], "field %d is NULL", q);
         int ex, ey, ez;
@@ -546,14 +589,6 @@ int ptk_solver_reset_clock(ptk_solver *s, void *stream)
     PTK_CHECK_ARG(s, "NULL solver");
     (void)stream;
     std::lock_guard<std::mutex> lk(s->mu);
-    // The parity of the current field buffer is tied to the step counter; keep it and only
-    // rebase the waveform index by storing the offset in the host mirror.
-    if (s->step & 1) {
-        // Swap buffer roles so that step 0 reads the buffer that holds the current fields.  The
-        // staged kernel's tensor maps name the buffers by parity: encode them again.
-        for (int f = 0; f < 6; ++f) std::swap(s->buf[0][f], s->buf[1][f]);
-        s->tma_by = 0;
-    }
     s->step = 0;
     return PTK_OK;
 }
@@ -582,7 +617,7 @@ int ptk_solver_set_tiles(ptk_solver *s, const ptk_tile_config *cfg)
     s->kc = kc;
     s->vec = vec;
     s->stages = stages;
-    return PTK_OK;
+    return stages > 0 ? prepare_fused(s) : PTK_OK;
 }
 
 int ptk_solver_use_material_index(ptk_solver *s, int enable, void *stream)
@@ -760,6 +795,7 @@ try {
             if (32 * vec > 2 * std::max(Nx, 32)) continue;   // tiles far wider than the grid
             add(by, vec, 0, yee_resident_ctas(by, vec));
         }
+    rc = prepare_fused(s);
     // Staged shapes: timed on vacuum coefficients, i.e. with the material index where the shape has it.
     const int staged[17][2] = {{4, 2}, {4, 3}, {4, 4}, {4, 5}, {4, 6}, {8, 2}, {8, 3}, {8, 4}, {8, 5}, {8, 6},
                                {10, 4}, {10, 5}, {11, 4}, {23, 3}, {23, 4}, {7, 3}, {7, 4}};
@@ -781,6 +817,7 @@ try {
         cudaEventElapsedTime(&ms, e0, e1);
         return ms / n;
     };
+    s->plain = true;   // shapes are compared by their own kernels
     // First pass: every candidate, briefly.  Second pass: the closest few again over longer runs,
     // twice in alternating order, since shapes within a few per cent of each other trade places
     // in short timings.
@@ -810,6 +847,21 @@ try {
                 best_t = e.first / 2;
                 bc = e.second;
             }
+        // Staged shapes take long runs through the resident or the two-step kernel: the best of them is
+        // compared by such a run.
+        s->plain = false;
+        if ((s->resident || s->pair) && !rc)
+            for (const auto &e : timed)
+                if (e.second.stages > 0) {
+                    const float ms = time_shape(bc.stages > 0 ? bc : e.second, std::max(8 * steps, 128));
+                    if (ms < 0) {
+                        rc = PTK_ERR_CUDA;
+                    } else if (ms < best_t || bc.stages > 0) {
+                        best_t = ms;
+                        if (bc.stages == 0) bc = e.second;
+                    }
+                    break;
+                }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

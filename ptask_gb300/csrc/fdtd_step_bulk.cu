@@ -157,7 +157,7 @@ struct Tile {
 // Tile t of the concatenated main-tile lists; false when its instance has no step left.
 template <int BY>
 __device__ __forceinline__ bool tile_at(int t, const InstDesc *__restrict__ insts, const int *__restrict__ tile0,
-                                        int ninst, int s_off, Tile &T)
+                                        int ninst, int s_off, int p_off, Tile &T)
 {
     int lo = 0, hi = ninst;
     while (hi - lo > 1) {
@@ -177,7 +177,7 @@ __device__ __forceinline__ bool tile_at(int t, const InstDesc *__restrict__ inst
     T.k1 = min(T.k0 + D->kc, D->nz);
     T.D = D;
     T.maps = reinterpret_cast<const CUtensorMap *>(D->tma);
-    T.par = (D->step + s_off) & 1;
+    T.par = (D->par + p_off) & 1;
     T.kstart = T.k0 > 0 ? T.k0 - 1 : T.k0;
     T.nplanes = T.k1 - T.kstart + 1;
     return true;
@@ -197,7 +197,7 @@ __device__ __forceinline__ bool tile_at(int t, const InstDesc *__restrict__ inst
 // last-layer tile at the start and run it after its own layer tile).
 template <int BY, int S, bool MAT, bool LAZY = false>
 __global__ void __launch_bounds__(32 * warps_of<BY>(), ctas_per_sm(BY))
-k_yee_step_bulk(const InstDesc *__restrict__ insts, const int *__restrict__ tile0, int ninst, int s_off,
+k_yee_step_bulk(const InstDesc *__restrict__ insts, const int *__restrict__ tile0, int ninst, int s_off, int p_off,
                 int total_tiles, int *err, int *work)
 {
     constexpr size_t SB = stage_bytes<BY, MAT>();
@@ -238,7 +238,7 @@ k_yee_step_bulk(const InstDesc *__restrict__ insts, const int *__restrict__ tile
     };
     auto fetch = [&](int &t, Tile &T) -> bool {   // first live tile at or after t
         while (t < total_tiles) {
-            if (tile_at<BY>(t, insts, tile0, ninst, s_off, T)) return true;
+            if (tile_at<BY>(t, insts, tile0, ninst, s_off, p_off, T)) return true;
             t = advance(t);
         }
         return false;
@@ -539,9 +539,9 @@ k_yee_step_bulk(const InstDesc *__restrict__ insts, const int *__restrict__ tile
 // and no other node's update reads them, so each evolves alone: H <- Da*H + Db*curl with a fixed
 // curl, the same operations in the same order as one step at a time.  Thread per face node over
 // all instances (face0: prefix of the instances' face-node counts); the result is written to the
-// buffer of the parity the instance's step counter has after its steps in this range.
+// buffer that holds the fields after the range: `flips` buffers on, or (flips < 0) one per step taken.
 __global__ void k_yee_faces_steps(const InstDesc *__restrict__ insts, const long long *__restrict__ face0,
-                                  int ninst, int s_off, int len)
+                                  int ninst, int s_off, int len, int flips)
 {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= __ldg(face0 + ninst)) return;
@@ -555,7 +555,7 @@ __global__ void k_yee_faces_steps(const InstDesc *__restrict__ insts, const long
     if (n <= 0) return;
     const int nx = D->nx, ny = D->ny, nz = D->nz, pitch = D->pitch;
     const long long plane = D->plane;
-    const int p0 = (D->step + s_off) & 1;
+    const int p0 = D->par & 1;
     const float *__restrict__ Ex = D->buf[p0][3];
     const float *__restrict__ Ey = D->buf[p0][4];
     const float *__restrict__ Ez = D->buf[p0][5];
@@ -585,15 +585,15 @@ __global__ void k_yee_faces_steps(const InstDesc *__restrict__ insts, const long
     const float da = D->coef[2][o], db = D->coef[3][o];
     float h = D->buf[p0][f][o];
     for (int s = 0; s < n; ++s) h = yee_b(da, h, db, a1, a0, s1, b1, b0, s2);
-    D->buf[(p0 + n) & 1][f][o] = h;
+    D->buf[(p0 + (flips < 0 ? n : flips)) & 1][f][o] = h;
 }
 
 int launch_yee_faces_steps(const InstDesc *d_insts, const long long *d_face0, int ninst, long long total_faces,
-                           int s_offset, int len, cudaStream_t s)
+                           int s_offset, int len, cudaStream_t s, int flips)
 {
     if (total_faces <= 0 || len <= 0) return PTK_OK;
     const long long blocks = (total_faces + 255) / 256;
-    k_yee_faces_steps<<<(unsigned)blocks, 256, 0, s>>>(d_insts, d_face0, ninst, s_offset, len);
+    k_yee_faces_steps<<<(unsigned)blocks, 256, 0, s>>>(d_insts, d_face0, ninst, s_offset, len, flips);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return PTK_OK;
@@ -630,13 +630,13 @@ static int resident_bulk()
 
 template <int BY, int S, bool MAT, bool LAZY>
 static int launch_bulk(const InstDesc *d_insts, const int *d_tile0, int ninst, int total_tiles, int s_offset,
-                       int grid, int *err, int *work, cudaStream_t s)
+                       int p_offset, int grid, int *err, int *work, cudaStream_t s)
 {
     const size_t smem = smem_bytes<BY, S, MAT, LAZY>();
     int rc = prepare_bulk<BY, S, MAT, LAZY>();
     if (rc) return rc;
     const int g = (grid <= 0 || grid > total_tiles) ? total_tiles : grid;
-    k_yee_step_bulk<BY, S, MAT, LAZY><<<g, dim3(32, warps_of<BY>()), smem, s>>>(d_insts, d_tile0, ninst, s_offset,
+    k_yee_step_bulk<BY, S, MAT, LAZY><<<g, dim3(32, warps_of<BY>()), smem, s>>>(d_insts, d_tile0, ninst, s_offset, p_offset,
                                                                                 total_tiles, err, work);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(1);
@@ -655,19 +655,21 @@ static int launch_bulk(const InstDesc *d_insts, const int *d_tile0, int ninst, i
     X(7, 3, true) X(7, 4, true)
 
 int launch_yee_step_bulk(const InstDesc *d_insts, const int *d_tile0, int ninst, int total_tiles, int s_offset,
-                         int by, int stages, int grid, int *err, cudaStream_t s, int *work, bool mat, bool lazy)
+                         int by, int stages, int grid, int *err, cudaStream_t s, int *work, bool mat, bool lazy,
+                         int p_offset)
 {
+    if (p_offset < 0) p_offset = s_offset;
     if (total_tiles <= 0) return PTK_OK;
     if (lazy && mat) {
 #define PTK_BULK_L(B, S, M)                                                                           \
     if (by == B && stages == S && mat == M)                                                           \
-        return launch_bulk<B, S, M, true>(d_insts, d_tile0, ninst, total_tiles, s_offset, grid, err, work, s);
+        return launch_bulk<B, S, M, true>(d_insts, d_tile0, ninst, total_tiles, s_offset, p_offset, grid, err, work, s);
         PTK_MAT_SHAPES(PTK_BULK_L)
 #undef PTK_BULK_L
     }
 #define PTK_BULK(B, S, M)                                                                               \
     if (by == B && stages == S && mat == M)                                                             \
-        return launch_bulk<B, S, M, false>(d_insts, d_tile0, ninst, total_tiles, s_offset, grid, err, work, s);
+        return launch_bulk<B, S, M, false>(d_insts, d_tile0, ninst, total_tiles, s_offset, p_offset, grid, err, work, s);
     PTK_DENSE_SHAPES(PTK_BULK) PTK_MAT_SHAPES(PTK_BULK)
 #undef PTK_BULK
     return set_error(PTK_ERR_INVALID, "no staged kernel for %d rows x %d stages%s", by, stages,

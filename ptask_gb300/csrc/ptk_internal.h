@@ -78,6 +78,7 @@ struct InstDesc {
     long long src;             // padded index of the Ez source node, -1 = none
     int nwave;
     int step;                  // absolute index of the first step of the current chunk
+    int par;                   // buffer that holds the fields at that step
     int steps_left;            // steps still to run at the start of the current chunk
     int tiles_x, tiles_y, tiles_z, face_tiles;
     int kc;                    // z-planes per main tile
@@ -133,14 +134,15 @@ int launch_yee_step_v(const InstDesc *d_insts, const int *d_tile0, int ninst, in
 // every instance carries a material index (and its map) and the coefficients come from its table.
 // With `lazy` (material-index shapes), each CTA claims its next tile from `work` just before the
 // ring needs it instead of when the current one starts (the single-instance solver's form).
+// p_offset: buffer flips since the chunk's start (-1: one per step, s_offset).
 int launch_yee_step_bulk(const InstDesc *d_insts, const int *d_tile0, int ninst, int total_tiles, int s_offset,
                          int by, int stages, int grid, int *err, cudaStream_t s, int *work = nullptr,
-                         bool mat = false, bool lazy = false);
+                         bool mat = false, bool lazy = false, int p_offset = -1);
 // The face H nodes (Hx at i = Nx, Hy at j = Ny, Hz at k = Nz) of every instance advanced by `len`
 // steps from step offset s_offset in one launch; the staged kernel's tile lists leave them out
 // (descriptors planned with face_tiles = 0).  d_face0: ninst + 1 prefix sums of face_nodes().
 int launch_yee_faces_steps(const InstDesc *d_insts, const long long *d_face0, int ninst, long long total_faces,
-                           int s_offset, int len, cudaStream_t s);
+                           int s_offset, int len, cudaStream_t s, int flips = -1);
 long long face_nodes(int nx, int ny, int nz);
 // Cells per thread of the tile width that goes with `by` staged rows (plan_tiles' vec): 23-row
 // tiles are 64 cells wide (2), all others 128 (4).
@@ -194,7 +196,29 @@ struct ResidentArgs {
 bool plan_resident(int nx, int ny, int nz, ResidentPlan *out);
 int launch_yee_resident(const ResidentPlan &p, int coef, ResidentArgs a, cudaStream_t s);
 
-int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s);
+// ---------------------------------------------------------------------------------------------
+// Two time steps in one pass over memory (fdtd_step_pair.cu), with the material index.
+// ---------------------------------------------------------------------------------------------
+enum { PAIR_SIMPLE = 0, PAIR_TABLE = 1 };   // every material Ca = Da = 1 and one Db, or any
+struct PairArgs {
+    int nxt, nyt, nzt, kc, tiles;   // tiles in x, y, z (kc planes deep)
+    int lw, rf, mw;                 // units per row and rows of a frame; bytes of a row of material ids
+    int tx_bytes;                   // bytes in flight of a ring stage
+    const void *tma;                // 13 tensor maps: Hx..Ez of both buffers, ids
+    float *buf[2][6];               // the fields' two buffers
+};
+struct PairPlan {
+    PairArgs args;
+    int threads, grid;
+    size_t smem;
+};
+bool plan_pair(int nx, int ny, int nz, PairPlan *out);
+int encode_pair_maps(const InstDesc &d, const PairPlan &p, void *host_out);   // 13 x 128 bytes
+// The two steps at pair offset `pair` of the chunk: from buffer (par + pair) & 1 to the other one.
+int launch_yee_pair(const InstDesc *d_inst, const PairPlan &p, int mode, int pair, int *err, cudaStream_t s);
+
+// Step counters on by nsteps (as far as each instance has steps left), buffers on by `flips` (-1: one per step).
+int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s, int flips = -1);
 int launch_pack_field(const float *src, int ex, int ey, int ez, const Layout &L, float *dst0,
                       float *dst1, cudaStream_t s);
 int launch_unpack_field(const float *src, int ex, int ey, int ez, const Layout &L, float *dst,
