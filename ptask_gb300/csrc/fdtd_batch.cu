@@ -579,7 +579,11 @@ int retire_copies(ptk_server *s, Inst *in, double *h_slot)
             float *stage = nullptr;
             int rc = pool_alloc(in->result[f].size() * sizeof(float), s->st, (void **)&stage);
             if (rc) return rc;
-            rc = launch_unpack_field(in->buf[par][f], a.ex[f], a.ey[f], a.ez[f], in->L, stage, s->st);
+            {
+                float *to[6] = {};
+                to[f] = stage;
+                rc = launch_unpack_fields(in->buf[par], in->L, to, f, 1, s->st);
+            }
             if (rc) return rc;
             PTK_CUDA_TRY(cudaMemcpyAsync(in->result[f].data(), stage, in->result[f].size() * sizeof(float),
                                          cudaMemcpyDeviceToHost, s->st));

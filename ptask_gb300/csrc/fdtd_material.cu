@@ -10,7 +10,7 @@
 //      claimed with atomicCAS, filled, then published; readers of a claimed slot wait for the
 //      publication with a bounded poll (on expiry an error word is raised and the index is not
 //      used).
-//   2. k_mat_compact: one thread numbers the occupied slots in slot order and writes the table.
+//   2. k_mat_compact: one block numbers the occupied slots in slot order and writes the table.
 //   3. k_mat_index: every node looks its tuple up and stores the id.
 //
 // More than kMaxMaterials distinct tuples (or a raised error word) leaves the index unused: the
@@ -59,6 +59,9 @@ __device__ uint4 read_key(const MatScratch *S, int h)
 
 __device__ void insert(MatScratch *S, uint4 key)
 {
+    // Too many materials already: the index will not be used, and a full table would cost every node
+    // a walk through all of it (160^3 cells with a permittivity each: 357 ms).
+    if (*reinterpret_cast<volatile int *>(&S->count) > kMaxMaterials) return;
     unsigned h = mix(key) & (kSlots - 1);
     for (int probe = 0; probe < kSlots; ++probe, h = (h + 1) & (kSlots - 1)) {
         // Most nodes repeat a tuple that is already published: check with a plain read first, so
@@ -89,75 +92,92 @@ __device__ void insert(MatScratch *S, uint4 key)
     atomicOr(&S->err, 2);
 }
 
-// Node q of the (nx+1) x (ny+1) x (nz+1) node grid (row padding is not part of the problem).
+// The (nx+1) x (ny+1) x (nz+1) node grid by rows (row padding is not part of the problem): a warp takes
+// a row at a time.
 struct Nodes {
-    int nx, ny, pitch;
-    long long plane, n;
-    __device__ long long offset(long long q) const
-    {
-        const int i = (int)(q % (nx + 1));
-        q /= nx + 1;
-        const int j = (int)(q % (ny + 1));
-        return i + (long long)pitch * j + plane * (q / (ny + 1));
-    }
+    int nx, ny, pitch, rows;
+    long long plane;
+    __device__ long long row(int r) const { return (long long)pitch * (r % (ny + 1)) + plane * (r / (ny + 1)); }
 };
 
-__global__ void k_mat_insert(const float *Ca, const float *Cb, const float *Da, const float *Db, Nodes N,
-                             MatScratch *S)
+__global__ void __launch_bounds__(256) k_mat_insert(const float *Ca, const float *Cb, const float *Da, const float *Db, Nodes N,
+                                                    MatScratch *S)
 {
     const float *c[4] = {Ca, Cb, Da, Db};
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    uint4 last = make_uint4(0, 0, 0, 0);   // the tuple this thread inserted last (already in the table)
+    const int lane = threadIdx.x & 31;
+    uint4 last = make_uint4(0, 0, 0, 0);   // the tuple this lane saw last (in the table already)
     bool have_last = false;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < N.n; q += stride) {
-        const uint4 key = tuple_at(c, N.offset(q));
-        // lanes with the same tuple (all four words equal) let their lowest lane insert it
-        const unsigned act = __activemask();
-        const unsigned m = __match_any_sync(act, key.x) & __match_any_sync(act, key.y) &
-                           __match_any_sync(act, key.z) & __match_any_sync(act, key.w);
-        if ((threadIdx.x & 31) == __ffs(m) - 1 && !(have_last && same(key, last))) {
-            insert(S, key);
-            last = key;
+    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < N.rows; r += gridDim.x * 8) {
+        const long long o = N.row(r);
+        for (int i = lane; i <= N.nx; i += 32) {
+            const uint4 key = tuple_at(c, o + i);
+            const bool fresh = !(have_last && same(key, last));
+            const unsigned act = __activemask();
+            if (!__any_sync(act, fresh)) continue;
+            // lanes with the same tuple (all four words equal) let their lowest lane insert it
+            const unsigned m = __match_any_sync(act, key.x) & __match_any_sync(act, key.y) &
+                               __match_any_sync(act, key.z) & __match_any_sync(act, key.w);
+            if (lane == __ffs(m) - 1 && fresh) insert(S, key);
+            last = key;   // inserted by this lane or by that one
             have_last = true;
         }
     }
 }
 
-__global__ void k_mat_compact(MatScratch *S, float4 *tab)
+// Numbers the occupied slots in slot order, a thread per slot (one thread for all of them: 56 us).
+__global__ void __launch_bounds__(kSlots) k_mat_compact(MatScratch *S, float4 *tab)
 {
-    int n = 0;
-    bool simple = true;
-    unsigned db = 0;
-    for (int h = 0; h < kSlots; ++h) {
-        if (S->state[h] != 2u) continue;
-        if (n == 0) db = S->key[h].w;
-        simple = simple && S->key[h].x == 0x3f800000u && S->key[h].z == 0x3f800000u && S->key[h].w == db;
-        if (n < kMaxMaterials) {
-            const uint4 k = S->key[h];
-            tab[n] = make_float4(__uint_as_float(k.x), __uint_as_float(k.y), __uint_as_float(k.z), __uint_as_float(k.w));
-        }
-        S->id[h] = n++;
+    __shared__ int before[kSlots / 32];
+    __shared__ unsigned db;
+    const int h = threadIdx.x, lane = h & 31, warp = h >> 5;
+    const bool on = S->state[h] == 2u;
+    const unsigned mask = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) before[warp] = __popc(mask);
+    if (h == 0) db = 0;
+    __syncthreads();
+    int id = __popc(mask & ((1u << lane) - 1)), n = 0;
+    for (int w = 0; w < kSlots / 32; ++w) {
+        if (w == warp) id += n;
+        n += before[w];
     }
-    S->info.nmat = (S->err || n > kMaxMaterials || n != S->count) ? 0 : n;
-    S->info.simple = S->info.nmat > 0 && simple;
-    S->info.db = __uint_as_float(db);
+    const uint4 k = on ? S->key[h] : make_uint4(0, 0, 0, 0);
+    if (on) {
+        if (id < kMaxMaterials)
+            tab[id] = make_float4(__uint_as_float(k.x), __uint_as_float(k.y), __uint_as_float(k.z), __uint_as_float(k.w));
+        S->id[h] = id;
+        if (id == 0) db = k.w;
+    }
+    __syncthreads();
+    const bool simple = __syncthreads_and(!on || (k.x == 0x3f800000u && k.z == 0x3f800000u && k.w == db));
+    if (h == 0) {
+        S->info.nmat = (S->err || n > kMaxMaterials || n != S->count) ? 0 : n;
+        S->info.simple = S->info.nmat > 0 && simple;
+        S->info.db = __uint_as_float(db);
+    }
 }
 
-__global__ void k_mat_index(const float *Ca, const float *Cb, const float *Da, const float *Db, Nodes N,
-                            const MatScratch *S, unsigned char *mat)
+__global__ void __launch_bounds__(256) k_mat_index(const float *Ca, const float *Cb, const float *Da, const float *Db, Nodes N,
+                                                   const MatScratch *S, unsigned char *mat)
 {
     if (S->info.nmat == 0) return;
     const float *c[4] = {Ca, Cb, Da, Db};
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < N.n; q += stride) {
-        const long long o = N.offset(q);
-        const uint4 key = tuple_at(c, o);
-        unsigned h = mix(key) & (kSlots - 1);
-        for (int probe = 0; probe < kSlots; ++probe, h = (h + 1) & (kSlots - 1))
-            if (S->state[h] == 2u && same(S->key[h], key)) {
-                mat[o] = (unsigned char)S->id[h];
-                break;
+    uint4 last = make_uint4(0, 0, 0, 0);   // the tuple looked up last
+    int id = -1;
+    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < N.rows; r += gridDim.x * 8) {
+        const long long o = N.row(r);
+        for (int i = threadIdx.x & 31; i <= N.nx; i += 32) {
+            const uint4 key = tuple_at(c, o + i);
+            if (id < 0 || !same(key, last)) {
+                unsigned h = mix(key) & (kSlots - 1);
+                for (int probe = 0; probe < kSlots; ++probe, h = (h + 1) & (kSlots - 1))
+                    if (S->state[h] == 2u && same(S->key[h], key)) {
+                        id = S->id[h];
+                        break;
+                    }
+                last = key;
             }
+            mat[o + i] = (unsigned char)id;
+        }
     }
 }
 
@@ -172,10 +192,10 @@ int build_material_index(const float *const coef[4], const Layout &L, unsigned c
     int rc = pool_alloc(sizeof(MatScratch), s, (void **)&S);
     if (rc) return rc;
     PTK_CUDA_TRY(cudaMemsetAsync(S, 0, sizeof(MatScratch), s));
-    Nodes N{L.nx, L.ny, L.pitch, L.plane, (long long)(L.nx + 1) * (L.ny + 1) * (L.nz + 1)};
-    const int grid = (int)std::min<long long>((N.n + 255) / 256, 8LL * std::max(1, sm_count()));
+    Nodes N{L.nx, L.ny, L.pitch, (L.ny + 1) * (L.nz + 1), L.plane};
+    const int grid = std::min((N.rows + 7) / 8, 8 * std::max(1, sm_count()));
     k_mat_insert<<<grid, 256, 0, s>>>(coef[0], coef[1], coef[2], coef[3], N, S);
-    k_mat_compact<<<1, 1, 0, s>>>(S, reinterpret_cast<float4 *>(tab));
+    k_mat_compact<<<1, kSlots, 0, s>>>(S, reinterpret_cast<float4 *>(tab));
     k_mat_index<<<grid, 256, 0, s>>>(coef[0], coef[1], coef[2], coef[3], N, S, mat);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(3);

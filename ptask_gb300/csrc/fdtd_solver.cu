@@ -359,6 +359,10 @@ static size_t field_bytes(int f, const ptk_fdtd_params &p)
     return (size_t)ex * ey * ez * sizeof(float);
 }
 
+// Device staging of host arrays: a field's slot, and how much is staged in one go.
+static size_t stage_bytes(int f, const ptk_fdtd_params &p) { return (field_bytes(f, p) + 255) / 256 * 256; }
+static constexpr size_t kStageTogether = (size_t)256 << 20;
+
 }  // namespace ptk
 
 static inline cudaStream_t S(void *s) { return s ? (cudaStream_t)s : default_stream(); }
@@ -464,20 +468,28 @@ int ptk_solver_set_fields(ptk_solver *s, const float *const f[6], int where, voi
     PTK_CHECK_ARG(s && f, "NULL argument");
     std::lock_guard<std::mutex> lk(s->mu);
     cudaStream_t st = S(stream);
-    for (int q = 0; q < 6; ++q) {
-        PTK_CHECK_ARG(f[q], "field %d is NULL", q);
-        int ex, ey, ez;
-        field_extents(q, s->p.Nx, s->p.Ny, s->p.Nz, &ex, &ey, &ez);
-        const float *src = f[q];
-        float *stage = nullptr;
-        if (where == PTK_HOST) {
-            int rc = pool_alloc(field_bytes(q, s->p), st, (void **)&stage);
-            if (rc) return rc;
-            PTK_CUDA_TRY(cudaMemcpyAsync(stage, f[q], field_bytes(q, s->p), cudaMemcpyHostToDevice, st));
-            src = stage;
+    for (int q = 0; q < 6; ++q) PTK_CHECK_ARG(f[q], "field %d is NULL", q);
+    float *const *dst = s->buf[s->par], *const *wall = s->buf[s->par ^ 1];
+    if (where != PTK_HOST) return launch_pack_fields(f, s->L, dst, wall, 0, 6, st);
+    // Host fields pass through device staging, all six at once where that is small, else one by one.
+    size_t total = 0;
+    for (int q = 0; q < 6; ++q) total += stage_bytes(q, s->p);
+    const int per = total <= kStageTogether ? 6 : 1;
+    for (int q0 = 0; q0 < 6; q0 += per) {
+        size_t bytes = 0;
+        for (int q = q0; q < q0 + per; ++q) bytes += stage_bytes(q, s->p);
+        char *stage = nullptr;
+        int rc = pool_alloc(bytes, st, (void **)&stage);
+        if (rc) return rc;
+        const float *src[6] = {};
+        char *at = stage;
+        for (int q = q0; q < q0 + per; ++q) {
+            src[q] = (const float *)at;
+            PTK_CUDA_TRY(cudaMemcpyAsync(at, f[q], field_bytes(q, s->p), cudaMemcpyHostToDevice, st));
+            at += stage_bytes(q, s->p);
         }
-        int rc = launch_pack_field(src, ex, ey, ez, s->L, s->buf[0][q], s->buf[1][q], st);
-        if (stage) pool_free(stage, st);
+        rc = launch_pack_fields(src, s->L, dst, wall, q0, per, st);
+        pool_free(stage, st);
         if (rc) return rc;
     }
     return PTK_OK;
@@ -489,24 +501,30 @@ int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *str
     PTK_CHECK_ARG(s && f, "NULL argument");
     std::lock_guard<std::mutex> lk(s->mu);
     cudaStream_t st = S(stream);
-    const int par = s->par;
-    for (int q = 0; q < 6; ++q) {
-        PTK_CHECK_ARG(f[q], "field %d is NULL", q);
-        int ex, ey, ez;
-        field_extents(q, s->p.Nx, s->p.Ny, s->p.Nz, &ex, &ey, &ez);
-        float *dst = f[q];
-        float *stage = nullptr;
-        if (where == PTK_HOST) {
-            int rc = pool_alloc(field_bytes(q, s->p), st, (void **)&stage);
-            if (rc) return rc;
-            dst = stage;
-        }
-        int rc = launch_unpack_field(s->buf[par][q], ex, ey, ez, s->L, dst, st);
+    for (int q = 0; q < 6; ++q) PTK_CHECK_ARG(f[q], "field %d is NULL", q);
+    const float *const *src = s->buf[s->par];
+    if (where != PTK_HOST) return launch_unpack_fields(src, s->L, f, 0, 6, st);
+    size_t total = 0;
+    for (int q = 0; q < 6; ++q) total += stage_bytes(q, s->p);
+    const int per = total <= kStageTogether ? 6 : 1;
+    for (int q0 = 0; q0 < 6; q0 += per) {
+        size_t bytes = 0;
+        for (int q = q0; q < q0 + per; ++q) bytes += stage_bytes(q, s->p);
+        char *stage = nullptr;
+        int rc = pool_alloc(bytes, st, (void **)&stage);
         if (rc) return rc;
-        if (stage) {
-            PTK_CUDA_TRY(cudaMemcpyAsync(f[q], stage, field_bytes(q, s->p), cudaMemcpyDeviceToHost, st));
-            pool_free(stage, st);
+        float *dst[6] = {};
+        char *at = stage;
+        for (int q = q0; q < q0 + per; ++q) {
+            dst[q] = (float *)at;
+            at += stage_bytes(q, s->p);
         }
+        rc = launch_unpack_fields(src, s->L, dst, q0, per, st);
+        for (int q = q0; q < q0 + per && !rc; ++q)
+            if (cudaMemcpyAsync(f[q], dst[q], field_bytes(q, s->p), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+                rc = set_error(PTK_ERR_CUDA, "download failed: %s", cudaGetErrorString(cudaGetLastError()));
+        pool_free(stage, st);
+        if (rc) return rc;
     }
     if (where == PTK_HOST) {
         PTK_CUDA_TRY(cudaStreamSynchronize(st));
@@ -526,17 +544,19 @@ int ptk_solver_set_coefficients(ptk_solver *s, const float *Ca, const float *Cb,
     std::lock_guard<std::mutex> lk(s->mu);
     cudaStream_t st = S(stream);
     const float *src[4] = {Ca, Cb, Da, Db};
-    const size_t bytes = (size_t)s->p.Nx * s->p.Ny * s->p.Nz * sizeof(float);
-    for (int c = 0; c < 4; ++c) {
-        const float *a = src[c];
-        float *stage = nullptr;
-        if (where == PTK_HOST) {
-            int rc = pool_alloc(bytes, st, (void **)&stage);
-            if (rc) return rc;
-            PTK_CUDA_TRY(cudaMemcpyAsync(stage, src[c], bytes, cudaMemcpyHostToDevice, st));
-            a = stage;
+    const size_t bytes = (size_t)s->p.Nx * s->p.Ny * s->p.Nz * sizeof(float), slot = (bytes + 255) / 256 * 256;
+    const int per = where != PTK_HOST || 4 * slot <= kStageTogether ? 4 : 1;
+    for (int c0 = 0; c0 < 4; c0 += per) {
+        const float *from[4] = {};
+        char *stage = nullptr;
+        int rc = where == PTK_HOST ? pool_alloc(per * slot, st, (void **)&stage) : PTK_OK;
+        if (rc) return rc;
+        for (int c = c0; c < c0 + per; ++c) {
+            from[c] = where == PTK_HOST ? (const float *)(stage + (c - c0) * slot) : src[c];
+            if (where == PTK_HOST)
+                PTK_CUDA_TRY(cudaMemcpyAsync(stage + (c - c0) * slot, src[c], bytes, cudaMemcpyHostToDevice, st));
         }
-        int rc = launch_pack_coef(a, s->L, s->coef[c], st);
+        rc = launch_pack_coefs(from, s->L, s->coef, c0, per, st);
         if (stage) pool_free(stage, st);
         if (rc) return rc;
     }

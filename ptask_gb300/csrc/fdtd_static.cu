@@ -140,12 +140,8 @@ int ptk_fdtd_solve_static(const ptk_fdtd_params *p, float *const fields[6], cons
     k_static_desc<<<1, 1, 0, st>>>(d_desc, d, d_tile0, total);
     PTK_CUDA_TRY(cudaGetLastError());
 
-    for (int q = 0; q < 6; ++q) {
-        int ex, ey, ez;
-        field_extents(q, p->Nx, p->Ny, p->Nz, &ex, &ey, &ez);
-        rc = launch_pack_field(fields[q], ex, ey, ez, L, arrays[q], arrays[6 + q], st);
-        if (rc) return rc;
-    }
+    rc = launch_pack_fields(fields, L, arrays, arrays + 6, 0, 6, st);
+    if (rc) return rc;
     if (vacuum) {
         const float v[4] = {1.0f, p->Dt / p->eps0, 1.0f, p->Dt / p->mu0};
         for (int c = 0; c < 4; ++c) {
@@ -154,23 +150,14 @@ int ptk_fdtd_solve_static(const ptk_fdtd_params *p, float *const fields[6], cons
         }
     } else {
         const float *src[4] = {Ca, Cb, Da, Db};
-        for (int c = 0; c < 4; ++c) {
-            rc = launch_pack_coef(src[c], L, arrays[12 + c], st);
-            if (rc) return rc;
-        }
+        rc = launch_pack_coefs(src, L, arrays + 12, 0, 4, st);
+        if (rc) return rc;
     }
     for (int s = 0; s < steps; ++s) {
         rc = launch_yee_step(d_desc, d_tile0, 1, total, s, by, st);
         if (rc) return rc;
     }
-    const int par = steps & 1;
-    for (int q = 0; q < 6; ++q) {
-        int ex, ey, ez;
-        field_extents(q, p->Nx, p->Ny, p->Nz, &ex, &ey, &ez);
-        rc = launch_unpack_field(arrays[par * 6 + q], ex, ey, ez, L, fields[q], st);
-        if (rc) return rc;
-    }
-    return PTK_OK;
+    return launch_unpack_fields(arrays + 6 * (steps & 1), L, fields, 0, 6, st);
 }
 
 }  // extern "C"

@@ -219,11 +219,14 @@ int launch_yee_pair(const InstDesc *d_inst, const PairPlan &p, int mode, int pai
 
 // Step counters on by nsteps (as far as each instance has steps left), buffers on by `flips` (-1: one per step).
 int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s, int flips = -1);
-int launch_pack_field(const float *src, int ex, int ey, int ez, const Layout &L, float *dst0,
-                      float *dst1, cudaStream_t s);
-int launch_unpack_field(const float *src, int ex, int ey, int ez, const Layout &L, float *dst,
-                        cudaStream_t s);
-int launch_pack_coef(const float *src, const Layout &L, float *dst, cudaStream_t s);
+// Fields first .. first + n - 1 (indices into the arrays given) from the reference layout to the padded
+// one and back, in one launch.  `wall` (may be null): the other buffers, which get the wall nodes
+// i = Nx, j = Ny, k = Nz only: a step writes everything else before it is read.
+int launch_pack_fields(const float *const src[], const Layout &L, float *const dst[], float *const wall[], int first, int n,
+                       cudaStream_t s);
+int launch_unpack_fields(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s);
+// Coefficient arrays first .. first + n - 1, (Nx,Ny,Nz) each, to padded nodes.
+int launch_pack_coefs(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s);
 int launch_fill(float *dst, long long n, float v, cudaStream_t s);
 int launch_field_ref(int field, const float *in0, const float *in1, const float *in2,
                      const ptk_fdtd_params &p, float *out, cudaStream_t s);
