@@ -246,7 +246,8 @@ int ptk_fdtd_solve(const ptk_fdtd_params *p, float *const fields[6], const float
  * (cudaGetSymbolAddress) with that device current and keeps it: make that call before any stream
  * capture, and make no call on a device after cudaDeviceReset.  Calls share the array, which keeps
  * the previous call's contents (each call clears what it uses): calls whose GPU work overlaps race
- * and must be serialised by the caller. */
+ * and must be serialised by the caller.  Longer runs are one cooperative launch whose waits are
+ * bounded; if one ran out, the fields would come back as NaN. */
 int ptk_fdtd_solve_static(const ptk_fdtd_params *p, float *const fields[6], const float *Ca,
                           const float *Cb, const float *Da, const float *Db, int si, int sj, int sk,
                           const float *wave, int nwave, int steps, void *stream);

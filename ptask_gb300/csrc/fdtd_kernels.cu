@@ -439,6 +439,7 @@ constexpr int kRowBatch = 4, kRowThreads = 256;
 
 struct RowMove {
     const float *src[6];
+    const int *err;            // UNPACK: where set, the fields become NaN (may be null)
     float *dst[6], *wall[6];   // wall: where nodes of the walls i = Nx, j = Ny, k = Nz go as well, or null
     int ex[6], ey[6], rows[6]; // dense extents
     int nx, ny, nz, pitch;
@@ -457,6 +458,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const RowMove A)
     const float *__restrict__ src = A.src[f];
     float *__restrict__ dst = A.dst[f];
     float *__restrict__ wall = A.wall[f];
+    const bool bad = MODE == ROWS_UNPACK && A.err && *A.err;
     const int step = gridDim.x * (kRowThreads / 32) * kRowBatch;
     for (int r0 = (blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5)) * kRowBatch; r0 < rows; r0 += step) {
         long long so[kRowBatch], to[kRowBatch];
@@ -485,7 +487,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const RowMove A)
                 for (int h = 0; h < 2; ++h) {
                     const int x = i + 32 * h;
                     if (!on[q] || x >= ex) continue;
-                    dst[to[q] + x] = v[q][h];
+                    dst[to[q] + x] = MODE == ROWS_UNPACK && bad ? __int_as_float(0x7fffffff) : v[q][h];
                     if (MODE == ROWS_PACK && wall && (edge[q] || x == A.nx)) wall[to[q] + x] = v[q][h];
                 }
         }
@@ -530,9 +532,11 @@ int launch_pack_fields(const float *const src[], const Layout &L, float *const d
     return PTK_OK;
 }
 
-int launch_unpack_fields(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s)
+int launch_unpack_fields(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s,
+                         const int *err)
 {
     RowMove a = row_move(L);
+    a.err = err;
     int most = 1;
     for (int q = 0; q < n; ++q) {
         int ez;

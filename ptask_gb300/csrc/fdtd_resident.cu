@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kMaxT, 1) k_yee_resident(const ResidentArgs A)
             f = 2;
             a1 = A.in[3][o + pitch]; a0 = A.in[3][o]; s1 = cy; b1 = A.in[4][o + 1]; b0 = A.in[4][o]; s2 = cx;
         }
-        const float d = A.coef[2][o], cc = A.coef[3][o];
+        const float d = A.coef[2] ? A.coef[2][o] : 1.f, cc = A.coef[3] ? A.coef[3][o] : A.db;
         float h = A.in[f][o];
         for (int s = 0; s < A.steps; ++s) h = upd<false>(d, h, cc, a1, a0, s1, b1, b0, s2);
         A.out[f][o] = h;
@@ -560,28 +560,26 @@ bool shape_cta(ResidentPlan &p)
 // The brick shape with the least estimated time per step among those that fit: shared-memory cycles
 // of the passes plus the ghost rows (sent, polled, stored), plus a part that does not shrink with the brick
 // (latency of a pass, longer with more planes per thread).
-bool plan_resident(int nx, int ny, int nz, ResidentPlan *out)
+bool plan_resident(int nx, int ny, int nz, int sms, ResidentPlan *out)
 {
-    const int sms = sm_count();
     double best = 1e30;
     bool found = false;
     for (int bz = 1; bz <= std::min(nz, 64); ++bz) {
-        const int nbz = (nz + bz - 1) / bz;
-        if (nbz > sms) continue;
-        for (int by = 1; by <= std::min(ny, 64); ++by) {
-            const int nby = (ny + by - 1) / by;
-            if ((long long)nby * nbz > sms) continue;
-            ResidentPlan p{};
-            p.by = by; p.bz = bz; p.nby = nby; p.nbz = nbz;
-            p.lw = (nx + 3) / 4; p.lwp = nx / 4 + 1;
-            if (!shape_cta(p)) continue;
-            const double units = (double)p.lw * by * bz, ghosts = (double)p.lw * ghost_rows(by, bz);
-            const double cost = units * 3.0 + ghosts * 1.0 + 250.0 * p.kz + 600.0;
-            if (cost < best) {
-                best = cost;
-                *out = p;
-                found = true;
-            }
+        const int nbz = (nz + bz - 1) / bz, cols = sms / nbz;
+        if (cols < 1) continue;
+        // the narrowest brick that leaves no more of them than SMs: a wider one only costs more
+        ResidentPlan p{};
+        p.bz = bz; p.nbz = nbz;
+        p.by = (ny + cols - 1) / cols;
+        p.nby = (ny + p.by - 1) / p.by;
+        p.lw = (nx + 3) / 4; p.lwp = nx / 4 + 1;
+        if (!shape_cta(p)) continue;
+        const double units = (double)p.lw * p.by * bz, ghosts = (double)p.lw * ghost_rows(p.by, bz);
+        const double cost = units * 3.0 + ghosts * 1.0 + 250.0 * p.kz + 600.0;
+        if (cost < best) {
+            best = cost;
+            *out = p;
+            found = true;
         }
     }
     return found;

@@ -144,7 +144,7 @@ static int prepare_fused(ptk_solver *s)
     cudaStream_t st = default_stream();
     void *maps = nullptr;
     int rc = PTK_OK;
-    if (plan_resident(s->L.nx, s->L.ny, s->L.nz, &s->rplan)) {
+    if (plan_resident(s->L.nx, s->L.ny, s->L.nz, sm_count(), &s->rplan)) {
         const size_t nseq = sizeof(unsigned) * s->rplan.nby * s->rplan.nbz;
         rc = pool_alloc(s->rplan.xch_bytes, st, (void **)&s->d_xch);
         if (rc == PTK_OK) rc = pool_alloc(nseq, st, (void **)&s->d_seq);
@@ -285,9 +285,6 @@ static int solver_graph(ptk_solver *s, int len, bool pair, cudaGraphExec_t *out)
 
 static constexpr int kChunk = 32;   // fused steps per replayed graph
 
-// A run of this many steps or more on a grid that fits on chip is one resident launch
-// (fdtd_resident.cu) instead of a step kernel per time step.
-static constexpr int kResidentSteps = 8;
 // Larger grids with a material index take runs of this many steps or more two steps per launch
 // (fdtd_step_pair.cu); shorter ones run the tile shape that was set.
 static constexpr int kPairSteps = 16;

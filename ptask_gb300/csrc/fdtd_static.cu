@@ -21,6 +21,9 @@
 //   * All calls share the one array and it keeps the previous call's contents: the regions a call
 //     uses are cleared at its start.  Calls whose GPU work overlaps (different streams, no ordering)
 //     race on the array; serialise them.
+//   * Runs of eight steps or more are one cooperative launch where its scratch fits, else a launch per
+//     step.  The launch's waits are bounded; if one ran out (never with calls serialised), the fields
+//     come back as NaN, since the call does not wait for its result.
 #include "ptk_internal.h"
 
 #include <map>
@@ -71,6 +74,60 @@ __global__ void k_static_desc(InstDesc *dst, InstDesc v, int *tile0, int total)
     tile0[1] = total;
 }
 
+// Scratch of a run in one launch (fdtd_resident.cu): error word, sequence numbers and exchange buffer,
+// all cleared, then the fields and the coefficients in padded form.
+struct ResidentScratch {
+    size_t seq, xch, cleared, arrays, total;
+};
+
+ResidentScratch resident_scratch(const ResidentPlan &p, size_t arr)
+{
+    ResidentScratch r;
+    r.seq = kStaticAlign;
+    r.xch = r.seq + align_up(sizeof(unsigned) * p.nby * p.nbz);
+    r.cleared = r.xch + p.xch_bytes;
+    r.arrays = align_up(r.cleared);
+    r.total = r.arrays + 10 * arr;
+    return r;
+}
+
+// A launch whose bounded waits ran out raises the error word, and the unpacking turns the fields into NaN.
+int solve_resident(const ptk_fdtd_params &p, float *const fields[6], const float *const coefs[4], const float *wave, int nwave,
+                   long long src, int steps, const Layout &L, const ResidentPlan &plan, const ResidentScratch &m, unsigned char *b,
+                   size_t arr, cudaStream_t st)
+{
+    PTK_CUDA_TRY(cudaMemsetAsync(b, 0, m.cleared, st));
+    ResidentArgs a{};
+    a.err = reinterpret_cast<int *>(b);
+    a.seq = reinterpret_cast<unsigned *>(b + m.seq);
+    a.xch = reinterpret_cast<ulonglong2 *>(b + m.xch);
+    float *f[6], *c[4];
+    for (int q = 0; q < 6; ++q) f[q] = reinterpret_cast<float *>(b + m.arrays + q * arr);
+    for (int q = 0; q < 4; ++q) c[q] = reinterpret_cast<float *>(b + m.arrays + (6 + q) * arr);
+    for (int q = 0; q < 6; ++q) a.in[q] = a.out[q] = f[q];
+    int rc = launch_pack_fields(fields, L, f, nullptr, 0, 6, st);
+    if (rc) return rc;
+    if (coefs[0]) {
+        rc = launch_pack_coefs(coefs, L, c, 0, 4, st);
+        for (int q = 0; q < 4; ++q) a.coef[q] = c[q];
+    } else {
+        rc = launch_fill(c[1], L.total, p.Dt / p.eps0, st);
+        a.coef[1] = c[1];
+        a.db = p.Dt / p.mu0;
+    }
+    if (rc) return rc;
+    a.wave = wave;
+    a.nwave = nwave;
+    a.src = src;
+    a.steps = steps;
+    a.nx = L.nx; a.ny = L.ny; a.nz = L.nz; a.pitch = L.pitch;
+    a.plane = L.plane;
+    a.cx = p.Cx; a.cy = p.Cy; a.cz = p.Cz;
+    rc = launch_yee_resident(plan, coefs[0] ? COEF_DENSE : COEF_SIMPLE, a, st);
+    if (rc) return rc;
+    return launch_unpack_fields(f, L, fields, 0, 6, st, a.err);
+}
+
 }  // namespace
 }  // namespace ptk
 
@@ -116,6 +173,20 @@ int ptk_fdtd_solve_static(const ptk_fdtd_params *p, float *const fields[6], cons
     int *d_tile0 = (int *)(b + kStaticAlign);
     float *arrays[16];
     for (int q = 0; q < 16; ++q) arrays[q] = (float *)(b + head + (size_t)q * arr);
+
+    // Longer runs are one launch where its scratch fits (64^3: 27 us per step by the step kernel below,
+    // 3 us so); the rest step with the register kernel.
+    int dev = 0, sms = 0;
+    ResidentPlan plan{};
+    if (steps >= kResidentSteps && cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        plan_resident(p->Nx, p->Ny, p->Nz, sms, &plan)) {
+        const ResidentScratch m = resident_scratch(plan, arr);
+        const float *const coefs[4] = {Ca, Cb, Da, Db};
+        if (m.total <= kStaticScratchBytes)
+            return solve_resident(*p, fields, coefs, has_src ? wave : nullptr, has_src ? nwave : 0,
+                                  has_src ? (long long)si + (long long)L.pitch * sj + L.plane * sk : -1, steps, L, plan, m, b, arr, st);
+    }
 
     // The scratch keeps the previous call's contents: clear everything this call uses.
     PTK_CUDA_TRY(cudaMemsetAsync(b, 0, need, st));

@@ -178,7 +178,7 @@ enum { COEF_SIMPLE = 0, COEF_DENSE = 1 };
 struct ResidentArgs {
     const float *in[6];
     float *out[6];             // may be `in`
-    const float *coef[4];      // padded arrays
+    const float *coef[4];      // padded arrays; COEF_SIMPLE needs Cb only (the others 1, 1, db where null)
     float db;                  // COEF_SIMPLE: the one Db
     const float *wave;
     long long src;             // padded index of the Ez source node, -1 = none
@@ -192,8 +192,11 @@ struct ResidentArgs {
     // set by the launcher: the plan, and byte offsets and strides in shared memory
     int lw, lwp, by, bz, nby, nbz, kz, threads, half, base[6], row, plane_e, plane_h, below, fail;
 };
-// The plan for a grid; false when it does not fit on chip.
-bool plan_resident(int nx, int ny, int nz, ResidentPlan *out);
+// A run of this many steps or more on a grid that fits on chip is one resident launch instead of a step
+// kernel per time step.  (Loading and storing the fields costs 12-30 us, two to six launches' worth.)
+constexpr int kResidentSteps = 8;
+// The plan for a grid on a device of `sms` SMs; false when it does not fit on chip.
+bool plan_resident(int nx, int ny, int nz, int sms, ResidentPlan *out);
 int launch_yee_resident(const ResidentPlan &p, int coef, ResidentArgs a, cudaStream_t s);
 
 // ---------------------------------------------------------------------------------------------
@@ -224,7 +227,10 @@ int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s, int
 // i = Nx, j = Ny, k = Nz only: a step writes everything else before it is read.
 int launch_pack_fields(const float *const src[], const Layout &L, float *const dst[], float *const wall[], int first, int n,
                        cudaStream_t s);
-int launch_unpack_fields(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s);
+// `err` (device, may be null): a raised error word turns the unpacked fields into NaN, for callers that
+// do not wait for the result.
+int launch_unpack_fields(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s,
+                         const int *err = nullptr);
 // Coefficient arrays first .. first + n - 1, (Nx,Ny,Nz) each, to padded nodes.
 int launch_pack_coefs(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s);
 int launch_fill(float *dst, long long n, float v, cudaStream_t s);

@@ -108,3 +108,37 @@ def test_two_solvers_run_resident_launches_from_two_threads():
         ref = oracle.step_ext_f32(f, steps, pr.params, pr.Ca, pr.Cb, pr.Da, pr.Db, pr.src, pr.wave)
         for q in range(6):
             np.testing.assert_array_equal(got[q], ref[q], err_msg=P.FIELDS[q])
+
+
+@pytest.mark.parametrize("shape,vacuum", [((89, 89, 89), False), ((64, 64, 64), True), ((33, 71, 50), False), ((400, 20, 21), True),
+                                          ((700, 31, 31), False), ((1, 1, 1), False)])
+def test_static_solve_runs_resident_where_its_scratch_fits(shape, vacuum):
+    """ptk_fdtd_solve_static over the resident launch and, where its scratch does not fit ((700, 31, 31)), the step kernel."""
+    import ctypes as C
+
+    from ptask_gb300 import _lib
+    from ptask_gb300.device import DeviceBuffer
+    steps, V = 13, C.c_void_p
+    pr = P.Problem.generate(*shape, n_boxes=3, eps=(1, 10), box=(2, 20), steps=9, source_mode=0 if vacuum else 2, seed=7)
+    if vacuum:
+        pr = P.Problem.vacuum(pr.params)
+    else:
+        medium(pr, "lossy", None)
+    f = P.random_fields(*shape, seed=94, scale=1e-2)
+    src = pr.src if pr.has_source else (-1, -1, -1)
+    ref = oracle.step_ext_f32(f, steps, pr.params, pr.Ca, pr.Cb, pr.Da, pr.Db, src, pr.wave)
+    bufs = [DeviceBuffer.from_array(a) for a in f]
+    coefs = [] if vacuum else [DeviceBuffer.from_array(a) for a in (pr.Ca, pr.Cb, pr.Da, pr.Db)]
+    wave = DeviceBuffer.from_array(pr.wave) if pr.has_source else None
+    for _ in range(2):   # the second call finds the first one's leftovers in the scratch
+        for b, a in zip(bufs, f):
+            b.upload(a)
+        _lib.call("ptk_fdtd_solve_static", C.byref(pr.params), (V * 6)(*[b.ptr for b in bufs]),
+                  *([c.ptr for c in coefs] if coefs else [None] * 4), *src, wave.ptr if wave else None,
+                  int(pr.wave.size) if wave else 0, steps, None)
+        _lib.call("ptk_device_sync")
+        got = [b.download(a.shape) for b, a in zip(bufs, f)]
+        for q in range(6):
+            np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{shape} {P.FIELDS[q]}")
+    for b in bufs + coefs + ([wave] if wave else []):
+        b.free()
