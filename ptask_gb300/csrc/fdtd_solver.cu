@@ -58,6 +58,25 @@ static void default_tiles(int nx, int ny, int nz, int *by, int *kc, int *vec)
     *kc = k;
 }
 
+// Grids of this many cells or more start with the staged kernel's shape, whose longer runs are one
+// resident launch or take two steps per pass (32^3: 1.8 us per step against 5.5; 256^3: 97 against 215).
+// Smaller ones keep the register kernel and a launch per step, which callers count
+// (ptk_solver_last_launches).
+static constexpr long long kStagedCells = 1 << 14;
+
+// Uniform coefficients v = (Ca, Cb, Da, Db), and the one-entry table that goes with them.
+__global__ void k_uniform_coefs(float *Ca, float *Cb, float *Da, float *Db, long long n, float4 v, float4 *tab)
+{
+    const long long q0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (q0 == 0) *tab = v;
+    for (long long q = q0; q < n; q += (long long)gridDim.x * blockDim.x) {
+        Ca[q] = v.x;
+        Cb[q] = v.y;
+        Da[q] = v.z;
+        Db[q] = v.w;
+    }
+}
+
 struct GraphKey {
     int len, by, kc, vec, stages, pair;
     bool operator<(const GraphKey &o) const
@@ -70,9 +89,12 @@ struct GraphKey {
 
 using namespace ptk;
 
+static constexpr int kChunk = 32;   // fused steps per replayed graph
+
 struct ptk_solver {
     ptk_fdtd_params p;
     Layout L;
+    void *block = nullptr;     // the one device allocation that holds the arrays below but wave and d_xch
     float *buf[2][6] = {};
     float *coef[4] = {};
     float *wave = nullptr;
@@ -99,6 +121,7 @@ struct ptk_solver {
     bool pair = false;              // staged shapes take long runs two steps at a time (fdtd_step_pair.cu)
     PairPlan pplan{};
     bool pair_maps = false;         // its tensor maps are encoded
+    void *d_tma_pair = nullptr;
     bool fused_ready = false;       // prepare_fused has run
     bool plain = false;             // the autotuner compares tile shapes by their own kernels
     InstDesc *d_desc = nullptr;
@@ -136,31 +159,56 @@ static RunShape run_shape(const ptk_solver *s)
 }
 
 // What the resident and the two-step kernel need, made when a staged shape is first set: the plan, the
-// exchange buffer (zeroed once) or the tensor maps' place.
+// exchange buffer (zeroed once) or where the tensor maps go.
 static int prepare_fused(ptk_solver *s)
 {
     if (s->fused_ready) return PTK_OK;
     s->fused_ready = true;
     cudaStream_t st = default_stream();
-    void *maps = nullptr;
-    int rc = PTK_OK;
     if (plan_resident(s->L.nx, s->L.ny, s->L.nz, sm_count(), &s->rplan)) {
-        const size_t nseq = sizeof(unsigned) * s->rplan.nby * s->rplan.nbz;
-        rc = pool_alloc(s->rplan.xch_bytes, st, (void **)&s->d_xch);
-        if (rc == PTK_OK) rc = pool_alloc(nseq, st, (void **)&s->d_seq);
-        if (rc == PTK_OK) {
-            PTK_CUDA_TRY(cudaMemsetAsync(s->d_xch, 0, s->rplan.xch_bytes, st));
-            PTK_CUDA_TRY(cudaMemsetAsync(s->d_seq, 0, nseq, st));
+        // the exchange buffer, and the bricks' counters behind it
+        const size_t seq = (s->rplan.xch_bytes + 255) / 256 * 256, total = seq + sizeof(unsigned) * s->rplan.nby * s->rplan.nbz;
+        if (pool_alloc(total, st, (void **)&s->d_xch) == PTK_OK) {
+            PTK_CUDA_TRY(cudaMemsetAsync(s->d_xch, 0, total, st));
+            PTK_CUDA_TRY(cudaStreamSynchronize(st));   // runs may come on any stream
+            s->d_seq = (unsigned *)((char *)s->d_xch + seq);
             s->resident = true;
+        } else {
+            clear_error();   // no room for it: the tile shape's own kernel runs
         }
-    } else if (plan_pair(s->L.nx, s->L.ny, s->L.nz, &s->pplan) && (rc = pool_alloc(kTmaSetBytes, st, &maps)) == PTK_OK) {
-        s->pplan.args.tma = maps;
+    } else if (plan_pair(s->L.nx, s->L.ny, s->L.nz, &s->pplan)) {
+        s->pplan.args.tma = s->d_tma_pair;
         for (int b = 0; b < 2; ++b)
             for (int f = 0; f < 6; ++f) s->pplan.args.buf[b][f] = s->buf[b][f];
         s->pair = true;
     }
-    if (rc) clear_error();   // no room for it: the tile shape's own kernel runs
-    PTK_CUDA_TRY(cudaStreamSynchronize(st));   // runs may come on any stream
+    return PTK_OK;
+}
+
+// Vacuum coefficients as the material index has them: one entry, every id 0.
+static int uniform_vacuum(ptk_solver *s, cudaStream_t st, bool clear_index)
+{
+    // Scalar coefficients of the reference: (params.Dt/params.eps0), (params.Dt/params.mu0) in FP32.
+    const float4 v = make_float4(1.0f, s->p.Dt / s->p.eps0, 1.0f, s->p.Dt / s->p.mu0);
+    if (clear_index) PTK_CUDA_TRY(cudaMemsetAsync(s->mat, 0, (size_t)s->L.total, st));
+    const int blocks = (int)std::min<long long>((s->L.total + 255) / 256, 16LL * std::max(1, sm_count()));
+    k_uniform_coefs<<<blocks, 256, 0, st>>>(s->coef[0], s->coef[1], s->coef[2], s->coef[3], s->L.total, v,
+                                            reinterpret_cast<float4 *>(s->mat_tab));
+    PTK_CUDA_TRY(cudaGetLastError());
+    count_launches(1);
+    s->minfo = MaterialInfo{};
+    if (s->mat_enabled) s->minfo = MaterialInfo{1, 1, v.w};
+    return PTK_OK;
+}
+
+// The staged kernel's shape without timing: 11 rows, a 4-plane ring and the depth that fills whole waves
+// of resident CTAs best.
+static int staged_default(int nx, int ny, int nz, ptk_tile_config *cfg)
+{
+    const int by = 11, stages = 4, vec = yee_bulk_tile_vec(by);
+    int kc = 0;
+    balanced_depths(nx, ny, nz, by, vec, yee_bulk_resident_ctas(by, stages, true), &kc, 1);
+    *cfg = {by, kc >= nz ? 0 : kc, vec, stages};
     return PTK_OK;
 }
 
@@ -283,8 +331,6 @@ static int solver_graph(ptk_solver *s, int len, bool pair, cudaGraphExec_t *out)
     return PTK_OK;
 }
 
-static constexpr int kChunk = 32;   // fused steps per replayed graph
-
 // Larger grids with a material index take runs of this many steps or more two steps per launch
 // (fdtd_step_pair.cu); shorter ones run the tile shape that was set.
 static constexpr int kPairSteps = 16;
@@ -330,7 +376,7 @@ int solver_run(ptk_solver *s, int steps, cudaStream_t st)
         rc = encode_pair_maps(e, s->pplan, maps);
         if (rc) return rc;
         PTK_CUDA_TRY(cudaStreamSynchronize(st));
-        PTK_CUDA_TRY(cudaMemcpy(const_cast<void *>(s->pplan.args.tma), maps, kTmaSetBytes, cudaMemcpyHostToDevice));
+        PTK_CUDA_TRY(cudaMemcpy(s->d_tma_pair, maps, kTmaSetBytes, cudaMemcpyHostToDevice));
         s->pair_maps = true;
     }
     int left = steps;
@@ -389,39 +435,53 @@ try {
     default_tiles(p->Nx, p->Ny, p->Nz, &s->by, &s->kc, &s->vec);
     cudaStream_t st = default_stream();
     const size_t bytes = (size_t)s->L.total * sizeof(float);
-    for (int b = 0; b < 2 && rc == PTK_OK; ++b)
-        for (int f = 0; f < 6 && rc == PTK_OK; ++f) rc = pool_alloc(bytes, st, (void **)&s->buf[b][f]);
-    for (int c = 0; c < 4 && rc == PTK_OK; ++c) rc = pool_alloc(bytes, st, (void **)&s->coef[c]);
-    if (rc == PTK_OK) rc = pool_alloc(sizeof(InstDesc), st, (void **)&s->d_desc);
-    if (rc == PTK_OK) rc = pool_alloc(2 * sizeof(int), st, (void **)&s->d_tile0);
-    if (rc == PTK_OK) rc = pool_alloc(sizeof(int), st, (void **)&s->d_err);
-    if (rc == PTK_OK) rc = pool_alloc(kTmaSetBytes, st, &s->d_tma);
-    if (rc == PTK_OK) rc = pool_alloc((size_t)s->L.total, st, (void **)&s->mat);
-    if (rc == PTK_OK) rc = pool_alloc(sizeof(float) * 4 * kMaxMaterials, st, (void **)&s->mat_tab);
-    if (rc == PTK_OK) cudaMemsetAsync(s->mat, 0, (size_t)s->L.total, st);
-    if (rc == PTK_OK) rc = pool_alloc(2 * sizeof(long long), st, (void **)&s->d_face0);
-    if (rc == PTK_OK) rc = pool_alloc(sizeof(int) * kChunk, st, (void **)&s->d_work);
-    if (rc == PTK_OK) {
-        s->faces = face_nodes(p->Nx, p->Ny, p->Nz);
-        const long long f0[2] = {0, s->faces};   // pageable: staged before the call returns
-        if (cudaMemcpyAsync(s->d_face0, f0, sizeof f0, cudaMemcpyHostToDevice, st) != cudaSuccess)
-            rc = set_error(PTK_ERR_CUDA, "face prefix upload failed");
-    }
-    if (rc == PTK_OK && ((uintptr_t)s->d_tma & 63))
-        rc = set_error(PTK_ERR_CUDA, "tensor-map buffer is not 64-byte aligned");
-    if (rc == PTK_OK) cudaMemsetAsync(s->d_err, 0, sizeof(int), st);
+    size_t room = 0;
+    auto take = [&room](size_t n) {   // 256-byte aligned places in the block
+        const size_t at = room;
+        room += (n + 255) / 256 * 256;
+        return at;
+    };
+    size_t at_buf[2][6], at_coef[4];
+    for (int b = 0; b < 2; ++b)
+        for (int f = 0; f < 6; ++f) at_buf[b][f] = take(bytes);
+    const size_t at_mat = take((size_t)s->L.total), at_err = take(sizeof(int));
+    const size_t cleared = room;      // fields, index and error word start at zero
+    for (int c = 0; c < 4; ++c) at_coef[c] = take(bytes);
+    const size_t at_tab = take(sizeof(float) * 4 * kMaxMaterials), at_desc = take(sizeof(InstDesc));
+    const size_t at_tile0 = take(2 * sizeof(int)), at_tma = take(kTmaSetBytes), at_pair = take(kTmaSetBytes);
+    const size_t at_face0 = take(2 * sizeof(long long)), at_work = take(sizeof(int) * kChunk);
+    rc = pool_alloc(room, st, &s->block);
     if (rc) {
         ptk_solver_destroy(s);
         return rc;
     }
+    char *base = static_cast<char *>(s->block);
     for (int b = 0; b < 2; ++b)
-        for (int f = 0; f < 6; ++f) cudaMemsetAsync(s->buf[b][f], 0, bytes, st);
-    for (int c = 0; c < 4; ++c) cudaMemsetAsync(s->coef[c], 0, bytes, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-        ptk_solver_destroy(s);
-        return set_error(PTK_ERR_CUDA, "solver initialisation failed");
+        for (int f = 0; f < 6; ++f) s->buf[b][f] = (float *)(base + at_buf[b][f]);
+    for (int c = 0; c < 4; ++c) s->coef[c] = (float *)(base + at_coef[c]);
+    s->mat = (unsigned char *)(base + at_mat);
+    s->mat_tab = (float *)(base + at_tab);
+    s->d_err = (int *)(base + at_err);
+    s->d_desc = (InstDesc *)(base + at_desc);
+    s->d_tile0 = (int *)(base + at_tile0);
+    s->d_tma = base + at_tma;
+    s->d_tma_pair = base + at_pair;
+    s->d_face0 = (long long *)(base + at_face0);
+    s->d_work = (int *)(base + at_work);
+    s->faces = face_nodes(p->Nx, p->Ny, p->Nz);
+    const long long f0[2] = {0, s->faces};   // pageable: staged before the call returns
+    if ((uintptr_t)base & 63) rc = set_error(PTK_ERR_CUDA, "tensor-map buffer is not 64-byte aligned");
+    if (rc == PTK_OK && (cudaMemsetAsync(base, 0, cleared, st) != cudaSuccess ||
+                         cudaMemcpyAsync(s->d_face0, f0, sizeof f0, cudaMemcpyHostToDevice, st) != cudaSuccess))
+        rc = set_error(PTK_ERR_CUDA, "solver initialisation failed");
+    if (rc == PTK_OK) rc = uniform_vacuum(s, st, /*clear_index=*/false);
+    if (rc == PTK_OK && (long long)p->Nx * p->Ny * p->Nz >= kStagedCells) {
+        ptk_tile_config c;
+        rc = staged_default(p->Nx, p->Ny, p->Nz, &c);
+        s->by = c.by; s->kc = c.kc; s->vec = c.vec; s->stages = c.stages;
+        if (rc == PTK_OK) rc = prepare_fused(s);
     }
-    rc = ptk_solver_set_vacuum(s, nullptr);
+    if (rc == PTK_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = set_error(PTK_ERR_CUDA, "solver initialisation failed");
     if (rc) {
         ptk_solver_destroy(s);
         return rc;
@@ -437,21 +497,9 @@ int ptk_solver_destroy(ptk_solver *s)
     {
         std::lock_guard<std::mutex> lk(s->mu);
         drop_graphs(s);
-        for (int b = 0; b < 2; ++b)
-            for (int f = 0; f < 6; ++f) pool_free(s->buf[b][f], st);
-        for (int c = 0; c < 4; ++c) pool_free(s->coef[c], st);
+        pool_free(s->block, st);
         pool_free(s->wave, st);
-        pool_free(s->d_desc, st);
-        pool_free(s->d_tile0, st);
-        pool_free(s->d_err, st);
-        pool_free(s->d_tma, st);
-        pool_free(s->mat, st);
-        pool_free(s->mat_tab, st);
-        pool_free(s->d_face0, st);
-        pool_free(s->d_work, st);
         pool_free(s->d_xch, st);
-        pool_free(s->d_seq, st);
-        pool_free(const_cast<void *>(s->pplan.args.tma), st);
         if (s->cap) cudaStreamDestroy(s->cap);
     }
     cudaStreamSynchronize(st);
@@ -524,9 +572,9 @@ int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *str
         if (rc) return rc;
     }
     if (where == PTK_HOST) {
-        PTK_CUDA_TRY(cudaStreamSynchronize(st));
         int err = 0;
-        PTK_CUDA_TRY(cudaMemcpy(&err, s->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+        PTK_CUDA_TRY(cudaMemcpyAsync(&err, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PTK_CUDA_TRY(cudaStreamSynchronize(st));
         if (err)
             return set_error(PTK_ERR_TIMEOUT, "a bounded wait of the staged step kernel expired; the fields are invalid");
     }
@@ -564,15 +612,10 @@ int ptk_solver_set_vacuum(ptk_solver *s, void *stream)
 {
     PTK_CHECK_ARG(s, "NULL solver");
     cudaStream_t st = S(stream);
-    // Scalar coefficients of the reference: (params.Dt/params.eps0), (params.Dt/params.mu0) in FP32.
-    const float ce = s->p.Dt / s->p.eps0;
-    const float ch = s->p.Dt / s->p.mu0;
-    const float v[4] = {1.0f, ce, 1.0f, ch};
-    for (int c = 0; c < 4; ++c) {
-        int rc = launch_fill(s->coef[c], s->L.total, v[c], st);
-        if (rc) return rc;
-    }
-    return rebuild_material(s, st);
+    const int rc = uniform_vacuum(s, st, /*clear_index=*/true);
+    if (rc) return rc;
+    PTK_CUDA_TRY(cudaStreamSynchronize(st));
+    return PTK_OK;
 }
 
 int ptk_solver_set_source(ptk_solver *s, int i, int j, int k, const float *wave, int nwave, int where,
@@ -908,11 +951,7 @@ try {
     }
     int rc = ensure_init();
     if (rc) return rc;
-    const int by = 11, stages = 4, vec = yee_bulk_tile_vec(by);
-    int kc = 0;
-    balanced_depths(Nx, Ny, Nz, by, vec, yee_bulk_resident_ctas(by, stages, true), &kc, 1);
-    *cfg = {by, kc, vec, stages};
-    return PTK_OK;
+    return staged_default(Nx, Ny, Nz, cfg);
 } PTK_CATCH_ALL
 
 }  // extern "C"
