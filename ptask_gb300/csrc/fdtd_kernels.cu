@@ -13,7 +13,6 @@
 //   k_yee_step<BY>   fused H+E step over a work list of tiles of one or many instances (padded
 //                    layout); the hot kernel.  Bandwidth bound: 64 algorithmic bytes per cell.
 //   k_field_ref      the reference's per-field task kernels (dense layout), one field per launch.
-//   k_h_half/k_e_half  the three H (or E) tasks of one step fused in one launch (dense layout).
 //   k_rows           reference layout <-> padded layout.
 #include "fdtd_device.cuh"
 
@@ -576,64 +575,73 @@ int launch_fill(float *dst, long long n, float v, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------------------------------------
-// The reference's six task kernels over dense arrays, one output field per launch.  Thread (i,j,k)
-// of the output extents computes exactly the expression of fdtd_<F>Computation_cpu.
+// The reference's task kernels over dense arrays.  Bound by memory (L2 where the fields fit it): a warp
+// takes 32 nodes of a row through kTaskPlanes planes with all their loads in flight, and a z neighbour
+// is the next plane's own value.  Fields that would give fewer than two blocks per SM that way take a
+// plane per warp.  Rows start anywhere, so accesses are single floats.  Per launch, against a thread
+// per node in blocks of 128 along x: 64x64x4 1.19 us (1.44), 45x64x50 1.67 (2.70), 200x150x100 8.5
+// (17.0), 256^3 47 (85).
 // ---------------------------------------------------------------------------------------------
-__global__ void k_field_ref(int field, const float *__restrict__ a, const float *__restrict__ b,
-                            const float *__restrict__ c, ptk_fdtd_params p, float *__restrict__ out)
+constexpr int kTaskRows = 8, kTaskPlanes = 4;
+
+static dim3 task_grid(int ex, int ey, int ez, int planes)
 {
-    const int Nx = p.Nx, Ny = p.Ny, Nz = p.Nz;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    const float ch = __fdiv_rn(p.Dt, p.mu0);
-    const float ce = __fdiv_rn(p.Dt, p.eps0);
-#define D3(ii, jj, kk, d1, d2) ((long long)(ii) + (long long)(d1) * (jj) + (long long)(d1) * (d2) * (kk))
-    switch (field) {
-    case PTK_HX: {   // a=Hx(Nx+1,Ny,Nz) b=Ey(Nx+1,Ny,Nz+1) c=Ez(Nx+1,Ny+1,Nz)
-        if (i > Nx) return;
-        const long long o = D3(i, j, k, Nx + 1, Ny);
-        out[o] = yee_ref(a[o], ch, b[D3(i, j, k + 1, Nx + 1, Ny)], b[D3(i, j, k, Nx + 1, Ny)], p.Cz,
-                         c[D3(i, j + 1, k, Nx + 1, Ny + 1)], c[D3(i, j, k, Nx + 1, Ny + 1)], p.Cy);
-        break;
+    return dim3((ex + 31) / 32, (ey + kTaskRows - 1) / kTaskRows, (ez + planes - 1) / planes);
+}
+
+// One field: out = a + c * ((p' - p) s1 - (q' - q) s2), where the differences of p and q run along
+// directions DP and DQ (0 x, 1 y, 2 z): upwards for H (E false), downwards for E, whose wall nodes are
+// copied.
+struct FieldTask {
+    const float *a, *p, *q;
+    float *out;
+    int ex, ey, ez;                  // extents of a and out
+    int prow, qrow;                  // row lengths of p and q
+    long long aplane, pplane, qplane;
+    int nx, ny, nz;
+    float c, s1, s2;
+};
+
+template <bool E, int DP, int DQ, int PL>
+__global__ void __launch_bounds__(32 * kTaskRows) k_field_ref(const FieldTask T)
+{
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kTaskRows + threadIdx.y, k0 = blockIdx.z * PL;
+    if (i >= T.ex || j >= T.ey) return;
+    const int n = min(PL, T.ez - k0);
+    const float *__restrict__ a = T.a + i + (long long)T.ex * j + T.aplane * k0;
+    const float *__restrict__ p = T.p + i + (long long)T.prow * j + T.pplane * k0;
+    const float *__restrict__ q = T.q + i + (long long)T.qrow * j + T.qplane * k0;
+    float *__restrict__ out = T.out + i + (long long)T.ex * j + T.aplane * k0;
+    constexpr int way = E ? -1 : 1;
+    const long long dp = way * (DP == 0 ? 1LL : DP == 1 ? (long long)T.prow : T.pplane);
+    const long long dq = way * (DQ == 0 ? 1LL : DQ == 1 ? (long long)T.qrow : T.qplane);
+    // E: inside the walls in the two directions across the field's own
+    const bool in = !E || (((DP != 0 && DQ != 0) || (i >= 1 && i <= T.nx - 1)) && ((DP != 1 && DQ != 1) || (j >= 1 && j <= T.ny - 1)));
+    float av[PL], pn[PL], pf[PL], qn[PL], qf[PL];
+    bool on[PL];
+#pragma unroll
+    for (int u = 0; u < PL; ++u) {
+        const bool z = !E || (DP != 2 && DQ != 2) || (k0 + u >= 1 && k0 + u <= T.nz - 1);
+        on[u] = u < n && in && z;
+        if (u < n) av[u] = a[u * T.aplane];
+        // the z neighbour of one plane is the node of another: loaded once
+        const bool mine = u < n && in;
+        if (on[u] || (mine && DP == 2 && !E && u > 0)) pn[u] = p[u * T.pplane];
+        if (on[u] || (mine && DQ == 2 && !E && u > 0)) qn[u] = q[u * T.qplane];
+        if (on[u] && (DP != 2 || (E && u == 0) || (E && !on[u > 0 ? u - 1 : 0]) || (!E && u + 1 >= n))) pf[u] = p[u * T.pplane + dp];
+        if (on[u] && (DQ != 2 || (E && u == 0) || (E && !on[u > 0 ? u - 1 : 0]) || (!E && u + 1 >= n))) qf[u] = q[u * T.qplane + dq];
     }
-    case PTK_HY: {   // a=Hy(Nx,Ny+1,Nz) b=Ex(Nx,Ny+1,Nz+1) c=Ez(Nx+1,Ny+1,Nz)
-        if (i >= Nx) return;
-        const long long o = D3(i, j, k, Nx, Ny + 1);
-        out[o] = yee_ref(a[o], ch, c[D3(i + 1, j, k, Nx + 1, Ny + 1)], c[D3(i, j, k, Nx + 1, Ny + 1)], p.Cx,
-                         b[D3(i, j, k + 1, Nx, Ny + 1)], b[D3(i, j, k, Nx, Ny + 1)], p.Cz);
-        break;
-    }
-    case PTK_HZ: {   // a=Hz(Nx,Ny,Nz+1) b=Ex(Nx,Ny+1,Nz+1) c=Ey(Nx+1,Ny,Nz+1)
-        if (i >= Nx) return;
-        const long long o = D3(i, j, k, Nx, Ny);
-        out[o] = yee_ref(a[o], ch, b[D3(i, j + 1, k, Nx, Ny + 1)], b[D3(i, j, k, Nx, Ny + 1)], p.Cy,
-                         c[D3(i + 1, j, k, Nx + 1, Ny)], c[D3(i, j, k, Nx + 1, Ny)], p.Cx);
-        break;
-    }
-    case PTK_EX: {   // a=Ex(Nx,Ny+1,Nz+1) b=Hy(Nx,Ny+1,Nz) c=Hz(Nx,Ny,Nz+1)
-        if (i >= Nx) return;
-        const long long o = D3(i, j, k, Nx, Ny + 1);
-        if (j < 1 || k < 1 || j > Ny - 1 || k > Nz - 1) { out[o] = a[o]; return; }
-        out[o] = yee_ref(a[o], ce, c[D3(i, j, k, Nx, Ny)], c[D3(i, j - 1, k, Nx, Ny)], p.Cy,
-                         b[D3(i, j, k, Nx, Ny + 1)], b[D3(i, j, k - 1, Nx, Ny + 1)], p.Cz);
-        break;
-    }
-    case PTK_EY: {   // a=Ey(Nx+1,Ny,Nz+1) b=Hx(Nx+1,Ny,Nz) c=Hz(Nx,Ny,Nz+1)
-        if (i > Nx) return;
-        const long long o = D3(i, j, k, Nx + 1, Ny);
-        if (i < 1 || k < 1 || i > Nx - 1 || k > Nz - 1) { out[o] = a[o]; return; }
-        out[o] = yee_ref(a[o], ce, b[D3(i, j, k, Nx + 1, Ny)], b[D3(i, j, k - 1, Nx + 1, Ny)], p.Cz,
-                         c[D3(i, j, k, Nx, Ny)], c[D3(i - 1, j, k, Nx, Ny)], p.Cx);
-        break;
-    }
-    default: {       // PTK_EZ: a=Ez(Nx+1,Ny+1,Nz) b=Hx(Nx+1,Ny,Nz) c=Hy(Nx,Ny+1,Nz)
-        if (i > Nx) return;
-        const long long o = D3(i, j, k, Nx + 1, Ny + 1);
-        if (i < 1 || j < 1 || i > Nx - 1 || j > Ny - 1) { out[o] = a[o]; return; }
-        out[o] = yee_ref(a[o], ce, c[D3(i, j, k, Nx, Ny + 1)], c[D3(i - 1, j, k, Nx, Ny + 1)], p.Cx,
-                         b[D3(i, j, k, Nx + 1, Ny)], b[D3(i, j - 1, k, Nx + 1, Ny)], p.Cy);
-        break;
-    }
+#pragma unroll
+    for (int u = 0; u < PL; ++u) {
+        if (u >= n) break;
+        float v = av[u];
+        if (on[u]) {
+            const int w = E ? (u > 0 ? u - 1 : 0) : (u + 1 < PL ? u + 1 : u);
+            const bool other = E ? (u > 0 && on[w]) : u + 1 < n;
+            const float pp = DP == 2 && other ? pn[w] : pf[u], qq = DQ == 2 && other ? qn[w] : qf[u];
+            v = E ? yee_ref(v, T.c, pn[u], pp, T.s1, qn[u], qq, T.s2) : yee_ref(v, T.c, pp, pn[u], T.s1, qq, qn[u], T.s2);
+        }
+        out[u * T.aplane] = v;
     }
 }
 
@@ -644,96 +652,44 @@ void field_extents(int f, int nx, int ny, int nz, int *ex, int *ey, int *ez)
     *ez = nz + ((f == PTK_HZ || f == PTK_EX || f == PTK_EY) ? 1 : 0);
 }
 
+template <int PL>
+static void field_task(int field, const FieldTask &t, cudaStream_t s)
+{
+    const dim3 grid = task_grid(t.ex, t.ey, t.ez, PL), block(32, kTaskRows);
+    switch (field) {
+    case PTK_HX: k_field_ref<false, 2, 1, PL><<<grid, block, 0, s>>>(t); break;
+    case PTK_HY: k_field_ref<false, 0, 2, PL><<<grid, block, 0, s>>>(t); break;
+    case PTK_HZ: k_field_ref<false, 1, 0, PL><<<grid, block, 0, s>>>(t); break;
+    case PTK_EX: k_field_ref<true, 1, 2, PL><<<grid, block, 0, s>>>(t); break;
+    case PTK_EY: k_field_ref<true, 2, 0, PL><<<grid, block, 0, s>>>(t); break;
+    default: k_field_ref<true, 0, 1, PL><<<grid, block, 0, s>>>(t); break;
+    }
+}
+
 int launch_field_ref(int field, const float *in0, const float *in1, const float *in2,
                      const ptk_fdtd_params &p, float *out, cudaStream_t s)
 {
-    int ex, ey, ez;
-    field_extents(field, p.Nx, p.Ny, p.Nz, &ex, &ey, &ez);
-    dim3 grid((ex + 127) / 128, ey, ez);
-    k_field_ref<<<grid, 128, 0, s>>>(field, in0, in1, in2, p, out);
-    PTK_CUDA_TRY(cudaGetLastError());
-    count_launches(1);
-    return PTK_OK;
-}
-
-// Three H (or E) tasks of one step in one launch over the node box (Nx+1,Ny+1,Nz+1).
-__global__ void k_h_half(const float *__restrict__ Hx, const float *__restrict__ Hy,
-                         const float *__restrict__ Hz, const float *__restrict__ Ex,
-                         const float *__restrict__ Ey, const float *__restrict__ Ez,
-                         ptk_fdtd_params p, float *__restrict__ oHx, float *__restrict__ oHy,
-                         float *__restrict__ oHz)
-{
-    const int Nx = p.Nx, Ny = p.Ny, Nz = p.Nz;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    const float ch = __fdiv_rn(p.Dt, p.mu0);
-    if (i <= Nx && j < Ny && k < Nz) {
-        const long long o = D3(i, j, k, Nx + 1, Ny);
-        oHx[o] = yee_ref(Hx[o], ch, Ey[D3(i, j, k + 1, Nx + 1, Ny)], Ey[D3(i, j, k, Nx + 1, Ny)], p.Cz,
-                         Ez[D3(i, j + 1, k, Nx + 1, Ny + 1)], Ez[D3(i, j, k, Nx + 1, Ny + 1)], p.Cy);
-    }
-    if (i < Nx && j <= Ny && k < Nz) {
-        const long long o = D3(i, j, k, Nx, Ny + 1);
-        oHy[o] = yee_ref(Hy[o], ch, Ez[D3(i + 1, j, k, Nx + 1, Ny + 1)], Ez[D3(i, j, k, Nx + 1, Ny + 1)], p.Cx,
-                         Ex[D3(i, j, k + 1, Nx, Ny + 1)], Ex[D3(i, j, k, Nx, Ny + 1)], p.Cz);
-    }
-    if (i < Nx && j < Ny && k <= Nz) {
-        const long long o = D3(i, j, k, Nx, Ny);
-        oHz[o] = yee_ref(Hz[o], ch, Ex[D3(i, j + 1, k, Nx, Ny + 1)], Ex[D3(i, j, k, Nx, Ny + 1)], p.Cy,
-                         Ey[D3(i + 1, j, k, Nx + 1, Ny)], Ey[D3(i, j, k, Nx + 1, Ny)], p.Cx);
-    }
-}
-
-__global__ void k_e_half(const float *__restrict__ Ex, const float *__restrict__ Ey,
-                         const float *__restrict__ Ez, const float *__restrict__ Hx,
-                         const float *__restrict__ Hy, const float *__restrict__ Hz,
-                         ptk_fdtd_params p, float *__restrict__ oEx, float *__restrict__ oEy,
-                         float *__restrict__ oEz)
-{
-    const int Nx = p.Nx, Ny = p.Ny, Nz = p.Nz;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    const float ce = __fdiv_rn(p.Dt, p.eps0);
-    if (i < Nx && j <= Ny && k <= Nz) {
-        const long long o = D3(i, j, k, Nx, Ny + 1);
-        oEx[o] = (j < 1 || k < 1 || j > Ny - 1 || k > Nz - 1)
-            ? Ex[o]
-            : yee_ref(Ex[o], ce, Hz[D3(i, j, k, Nx, Ny)], Hz[D3(i, j - 1, k, Nx, Ny)], p.Cy,
-                      Hy[D3(i, j, k, Nx, Ny + 1)], Hy[D3(i, j, k - 1, Nx, Ny + 1)], p.Cz);
-    }
-    if (i <= Nx && j < Ny && k <= Nz) {
-        const long long o = D3(i, j, k, Nx + 1, Ny);
-        oEy[o] = (i < 1 || k < 1 || i > Nx - 1 || k > Nz - 1)
-            ? Ey[o]
-            : yee_ref(Ey[o], ce, Hx[D3(i, j, k, Nx + 1, Ny)], Hx[D3(i, j, k - 1, Nx + 1, Ny)], p.Cz,
-                      Hz[D3(i, j, k, Nx, Ny)], Hz[D3(i - 1, j, k, Nx, Ny)], p.Cx);
-    }
-    if (i <= Nx && j <= Ny && k < Nz) {
-        const long long o = D3(i, j, k, Nx + 1, Ny + 1);
-        oEz[o] = (i < 1 || j < 1 || i > Nx - 1 || j > Ny - 1)
-            ? Ez[o]
-            : yee_ref(Ez[o], ce, Hy[D3(i, j, k, Nx, Ny + 1)], Hy[D3(i - 1, j, k, Nx, Ny + 1)], p.Cx,
-                      Hx[D3(i, j, k, Nx + 1, Ny)], Hx[D3(i, j - 1, k, Nx + 1, Ny)], p.Cy);
-    }
-}
-#undef D3
-
-int launch_h_half(const float *const in[6], float *const out[3], const ptk_fdtd_params &p,
-                  cudaStream_t s)
-{
-    dim3 grid((p.Nx + 1 + 127) / 128, p.Ny + 1, p.Nz + 1);
-    k_h_half<<<grid, 128, 0, s>>>(in[0], in[1], in[2], in[3], in[4], in[5], p, out[0], out[1], out[2]);
-    PTK_CUDA_TRY(cudaGetLastError());
-    count_launches(1);
-    return PTK_OK;
-}
-
-int launch_e_half(const float *const e_in[3], const float *const h_new[3], float *const out[3],
-                  const ptk_fdtd_params &p, cudaStream_t s)
-{
-    dim3 grid((p.Nx + 1 + 127) / 128, p.Ny + 1, p.Nz + 1);
-    k_e_half<<<grid, 128, 0, s>>>(e_in[0], e_in[1], e_in[2], h_new[0], h_new[1], h_new[2], p,
-                                  out[0], out[1], out[2]);
+    // p and q of each field: which input, and which field's extents it has
+    static const int pin[6] = {1, 2, 1, 2, 1, 2}, pf[6] = {PTK_EY, PTK_EZ, PTK_EX, PTK_HZ, PTK_HX, PTK_HY};
+    static const int qf[6] = {PTK_EZ, PTK_EX, PTK_EY, PTK_HY, PTK_HZ, PTK_HX};
+    const float sc[3] = {p.Cx, p.Cy, p.Cz};
+    static const int dp[6] = {2, 0, 1, 1, 2, 0}, dq[6] = {1, 2, 0, 2, 0, 1};
+    const float *in[3] = {in0, in1, in2};
+    FieldTask t{};
+    t.a = in0; t.p = in[pin[field]]; t.q = in[3 - pin[field]]; t.out = out;
+    int ey, ez;
+    field_extents(field, p.Nx, p.Ny, p.Nz, &t.ex, &t.ey, &t.ez);
+    t.aplane = (long long)t.ex * t.ey;
+    field_extents(pf[field], p.Nx, p.Ny, p.Nz, &t.prow, &ey, &ez);
+    t.pplane = (long long)t.prow * ey;
+    field_extents(qf[field], p.Nx, p.Ny, p.Nz, &t.qrow, &ey, &ez);
+    t.qplane = (long long)t.qrow * ey;
+    t.nx = p.Nx; t.ny = p.Ny; t.nz = p.Nz;
+    t.c = field < 3 ? p.Dt / p.mu0 : p.Dt / p.eps0;
+    t.s1 = sc[dp[field]]; t.s2 = sc[dq[field]];
+    const dim3 grid = task_grid(t.ex, t.ey, t.ez, kTaskPlanes);
+    if ((long long)grid.x * grid.y * grid.z >= 2 * std::max(1, sm_count())) field_task<kTaskPlanes>(field, t, s);
+    else field_task<1>(field, t, s);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return PTK_OK;
