@@ -1,13 +1,16 @@
 // fdtd_batch.cu -- batched and served FDTD: many device-resident instances of uneven size advanced
 // together by the fused step kernel, with continuous admission by HBM budget.
 //
-// One time step of every active instance is ONE launch of the step kernel (the TMA-staged
-// k_yee_step_bulk with a material index by default, the register kernel k_yee_step on request) over
-// the concatenated tile lists of all instances: a persistent grid of resident CTAs takes tiles from
-// a counter.  Chunks of steps are replayed as captured CUDA graphs (at most kMaxGraphs kept).
-// Instances finish at their own step counts: their tiles go idle inside the chunk in which they
-// finish and they leave the batch at the chunk boundary, where newly arrived requests are admitted
-// if they fit the HBM budget.  Request problems are generated on the device (coefficients and the
+// Two time steps of every active instance are ONE launch of the two-step kernel (k_yee_pair, a CTA per
+// tile of the instances' tile lists); a chunk's odd step, and the steps of a batch that holds an instance
+// too thin for it (fewer than 8 planes or 4 rows), are launches of the TMA-staged one-step kernel
+// (k_yee_step_bulk) over the same instances, or of the register kernel k_yee_step on request.  Both take
+// the coefficients from a material index.  Chunks of steps are replayed as captured CUDA graphs (at most
+// kMaxGraphs kept).  Device time of a mix, two steps per pass against one: 64 requests of 32..192 540 ms
+// against 1050, 64 x 32^3 4.0 against 18.0, one 256^3 28 against 40, one 16^3 2.5 against 4.2.
+//
+// Instances finish at their own step counts, with a chunk that ends there, and leave the batch at its
+// end, where newly arrived requests are admitted if they fit the HBM budget.  Request problems are generated on the device (coefficients and the
 // material index from the seeded box list), so admission moves only the waveform and the tensor
 // maps over the host link.
 //
@@ -132,12 +135,16 @@ struct Inst {
     float *coef[4] = {};
     float *wave = nullptr;
     void *tma = nullptr;        // tensor maps of the staged kernel
+    void *tma_pair = nullptr;   // tensor maps of the two-step kernel
+    PairPlan plan{};            // its frame, and its depth in the current work list
+    bool pair = false;          // the frame exists
     unsigned char *mat = nullptr;   // material index (staged kernel)
     float *mat_tab = nullptr;
     int nmat = 0;
     int nwave = 0;
     long long src = -1;
     int steps_total = 0, done = 0;
+    int par = 0;                // buffer that holds the fields
     size_t bytes = 0;
     double t_arrival = 0, t_admit = -1, t_finish = -1;
     double t_arrival_run = 0;   // arrival on the run's clock (scaled trace time)
@@ -152,7 +159,7 @@ struct Inst {
 // usable when thousands of requests of different sizes come and go): byte offsets, each array
 // 256-byte aligned.
 struct InstBlock {
-    size_t field[2][6], coef[4], mat, sum, tma, tab, wave, total;
+    size_t field[2][6], coef[4], mat, sum, tma, tma_pair, tab, wave, total;
 };
 
 InstBlock block_layout(const Layout &L, int nwave)
@@ -171,7 +178,8 @@ InstBlock block_layout(const Layout &L, int nwave)
     b.mat = take((size_t)L.total);
     b.sum = take(6 * sizeof(double));
     b.tma = take(kTmaSetBytes);
-    b.tab = take((size_t)kMaxMaterials * 4 * sizeof(float));
+    b.tma_pair = take(kPairMapBytes);
+    b.tab = take((size_t)(kMaxBoxes + 1) * 4 * sizeof(float));
     b.wave = take((size_t)std::max(nwave, 1) * sizeof(float));
     b.total = o;
     return b;
@@ -198,6 +206,11 @@ struct ptk_server {
     long long *d_face0 = nullptr;   // staged kernel: prefix sums of the instances' face nodes
     long long *h_face0[2] = {};
     long long total_faces = 0;
+    PairArgs *d_pair = nullptr;     // two-step kernel: the instances' arguments, prefix sums of their tiles
+    PairArgs *h_pair[2] = {};
+    int *d_pair0 = nullptr;
+    int *h_pair0[2] = {};
+    int pair_tiles = 0;             // 0: an instance of the batch has no frame, single steps
     int cap = 0;
     int total_tiles = 0;
     int vec = 4;                    // x cells per thread of the current work list
@@ -223,7 +236,7 @@ struct ptk_server {
     } flight[2];
     bool dirty = true;
     bool admit_blocked = false;     // the pool could not place a request: wait for retirements
-    std::map<std::tuple<int, int, int, int, long long>, cudaGraphExec_t> graphs;
+    std::map<std::tuple<int, int, int, int, int, long long>, cudaGraphExec_t> graphs;
     long long chunks = 0, launches = 0, captures = 0, admit_waits = 0;
     double wall_s = 0, cell_updates = 0;
     double chunk_dev_s = 0, admit_s = 0, retire_s = 0, sched_s = 0;   // where wall_s went
@@ -248,10 +261,16 @@ int grow_worklist(ptk_server *s, int n)
         pool_free(s->d_desc, s->st);
         pool_free(s->d_tile0, s->st);
         pool_free(s->d_face0, s->st);
+        pool_free(s->d_pair, s->st);
+        pool_free(s->d_pair0, s->st);
         for (int b = 0; b < 2; ++b) {
             cudaFreeHost(s->h_desc[b]);
             cudaFreeHost(s->h_tile0[b]);
             cudaFreeHost(s->h_face0[b]);
+            cudaFreeHost(s->h_pair[b]);
+            cudaFreeHost(s->h_pair0[b]);
+            s->h_pair[b] = nullptr;
+            s->h_pair0[b] = nullptr;
             s->h_desc[b] = nullptr;
             s->h_tile0[b] = nullptr;
             s->h_face0[b] = nullptr;
@@ -260,8 +279,12 @@ int grow_worklist(ptk_server *s, int n)
     int rc = pool_alloc(sizeof(InstDesc) * cap, s->st, (void **)&s->d_desc);
     if (!rc) rc = pool_alloc(sizeof(int) * (cap + 1), s->st, (void **)&s->d_tile0);
     if (!rc) rc = pool_alloc(sizeof(long long) * (cap + 1), s->st, (void **)&s->d_face0);
+    if (!rc) rc = pool_alloc(sizeof(PairArgs) * cap, s->st, (void **)&s->d_pair);
+    if (!rc) rc = pool_alloc(sizeof(int) * (cap + 1), s->st, (void **)&s->d_pair0);
     if (rc) return rc;
     for (int b = 0; b < 2; ++b) {
+        PTK_CUDA_TRY(cudaMallocHost(&s->h_pair[b], sizeof(PairArgs) * cap));
+        PTK_CUDA_TRY(cudaMallocHost(&s->h_pair0[b], sizeof(int) * (cap + 1)));
         PTK_CUDA_TRY(cudaMallocHost(&s->h_desc[b], sizeof(InstDesc) * cap));
         PTK_CUDA_TRY(cudaMallocHost(&s->h_tile0[b], sizeof(int) * (cap + 1)));
         PTK_CUDA_TRY(cudaMallocHost(&s->h_face0[b], sizeof(long long) * (cap + 1)));
@@ -321,7 +344,7 @@ InstDesc instance_desc(const ptk_server *s, const Inst *in)
     d.src = in->nwave ? in->src : -1;
     d.nwave = in->nwave;
     d.step = in->done;
-    d.par = in->done & 1;
+    d.par = in->par;
     d.steps_left = in->steps_total - in->done;
     d.tma = in->tma;
     if (s->stages) {
@@ -386,6 +409,7 @@ int admit(ptk_server *s, Inst *in)
     in->d_sum = reinterpret_cast<double *>(base + lay.sum);
     if (s->stages) {
         in->tma = base + lay.tma;
+        in->tma_pair = base + lay.tma_pair;
         in->mat = reinterpret_cast<unsigned char *>(base + lay.mat);
         in->mat_tab = reinterpret_cast<float *>(base + lay.tab);
     }
@@ -426,6 +450,16 @@ int admit(ptk_server *s, Inst *in)
         if (rc) return rc;
         rc = stage_upload(s, in->tma, maps, kTmaSetBytes);
         if (rc) return rc;
+        in->pair = plan_pair_member(in->L.nx, in->L.ny, in->L.nz, &in->plan);
+        if (in->pair) {
+            alignas(64) unsigned char pmaps[kPairMapBytes];
+            in->plan.args.tma = in->tma_pair;
+            for (int b = 0; b < 2; ++b)
+                for (int f = 0; f < 6; ++f) in->plan.args.buf[b][f] = in->buf[b][f];
+            rc = encode_pair_maps(instance_desc(s, in), in->plan, pmaps);
+            if (!rc) rc = stage_upload(s, in->tma_pair, pmaps, kPairMapBytes);
+            if (rc) return rc;
+        }
     }
     in->bytes = instance_bytes(in->L, in->nwave);
     s->used += in->bytes;
@@ -446,6 +480,7 @@ void release(ptk_server *s, Inst *in)
     in->wave = nullptr;
     in->d_sum = nullptr;
     in->tma = nullptr;
+    in->tma_pair = nullptr;
     in->mat = nullptr;
     in->mat_tab = nullptr;
     s->used -= in->bytes;
@@ -465,15 +500,27 @@ int rebuild_worklist(ptk_server *s)
     // small grids but hold fewer bytes in flight per thread, and measured slower on the batched
     // workload.  The staged kernel's width goes with its rows (set at creation).
     if (!s->stages) s->vec = 4;
+    bool pair = s->stages > 0;
+    for (const Inst *in : s->active) pair = pair && in->pair;
+    if (pair) {
+        std::vector<PairPlan *> plans;
+        std::vector<int> nz;
+        for (Inst *in : s->active) {
+            plans.push_back(&in->plan);
+            nz.push_back(in->L.nz);
+        }
+        plan_pair_depths(plans.data(), nz.data(), n);
+    }
     if (s->stages) {
         s->depth_cap = choose_depth_cap(s);
         // longest tiles first, so that the dynamic tile queue ends with short ones
-        std::stable_sort(s->active.begin(), s->active.end(), [s](const Inst *a, const Inst *b) {
+        std::stable_sort(s->active.begin(), s->active.end(), [s, pair](const Inst *a, const Inst *b) {
+            if (pair) return a->plan.args.kc > b->plan.args.kc;
             const int da = instance_depth(s, a->L.nz), db = instance_depth(s, b->L.nz);
             return (da ? da : a->L.nz) > (db ? db : b->L.nz);
         });
     }
-    int tiles = 0;
+    int tiles = 0, pair_tiles = 0;
     long long faces = 0;
     for (int q = 0; q < n; ++q) {
         const InstDesc d = instance_desc(s, s->active[q]);
@@ -482,7 +529,13 @@ int rebuild_worklist(ptk_server *s)
         faces += face_nodes(d.nx, d.ny, d.nz);
         h_tile0[q] = tiles;
         tiles += d.tiles_x * d.tiles_y * d.tiles_z + d.face_tiles;
+        if (pair) {
+            s->h_pair[s->par][q] = s->active[q]->plan.args;
+            s->h_pair0[s->par][q] = pair_tiles;
+            pair_tiles += s->active[q]->plan.args.tiles;
+        }
     }
+    s->h_pair0[s->par][n] = s->pair_tiles = pair_tiles;
     h_tile0[n] = tiles;
     s->total_tiles = tiles;
     h_face0[n] = faces;
@@ -492,6 +545,10 @@ int rebuild_worklist(ptk_server *s)
         PTK_CUDA_TRY(cudaMemcpyAsync(s->d_tile0, h_tile0, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s->st));
         PTK_CUDA_TRY(cudaMemcpyAsync(s->d_face0, h_face0, sizeof(long long) * (n + 1), cudaMemcpyHostToDevice,
                                      s->st));
+        if (pair) {
+            PTK_CUDA_TRY(cudaMemcpyAsync(s->d_pair, s->h_pair[s->par], sizeof(PairArgs) * n, cudaMemcpyHostToDevice, s->st));
+            PTK_CUDA_TRY(cudaMemcpyAsync(s->d_pair0, s->h_pair0[s->par], sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s->st));
+        }
     }
     s->dirty = false;
     return PTK_OK;
@@ -499,10 +556,13 @@ int rebuild_worklist(ptk_server *s)
 
 constexpr size_t kMaxGraphs = 256;   // chunk graphs kept for reuse
 
+int chunk_pairs(const ptk_server *s, int len) { return s->pair_tiles ? len / 2 : 0; }
+
 int chunk_graph(ptk_server *s, int len, int grid, cudaGraphExec_t *out)
 {
     const int n = (int)s->active.size();
-    auto key = std::make_tuple(len, n, s->total_tiles, (grid * 8 + s->vec) * 8 + s->stages, s->total_faces);
+    const int pairs = chunk_pairs(s, len), flips = len - pairs;
+    auto key = std::make_tuple(len, n, s->total_tiles, s->pair_tiles, (grid * 8 + s->vec) * 8 + s->stages, s->total_faces);
     auto it = s->graphs.find(key);
     if (it != s->graphs.end()) {
         *out = it->second;
@@ -517,12 +577,14 @@ int chunk_graph(ptk_server *s, int len, int grid, cudaGraphExec_t *out)
         rc = set_error(PTK_ERR_CUDA, "chunk capture: counter reset failed");
     else if (s->stages)
         count_launches(1);
-    if (!rc && s->stages) rc = launch_yee_faces_steps(s->d_desc, s->d_face0, n, s->total_faces, 0, len, cap);
-    for (int q = 0; q < len && !rc; ++q)
+    if (!rc && s->stages) rc = launch_yee_faces_steps(s->d_desc, s->d_face0, n, s->total_faces, 0, len, cap, flips);
+    for (int q = 0; q < pairs && !rc; ++q)
+        rc = launch_yee_pair_batch(s->d_desc, s->d_pair, s->d_pair0, n, s->pair_tiles, q, s->d_err, cap);
+    for (int q = 2 * pairs; q < len && !rc; ++q)
         rc = s->stages ? launch_yee_step_bulk(s->d_desc, s->d_tile0, n, s->total_tiles, q, s->rows, s->stages, grid,
-                                              s->d_err, cap, s->d_work, true)
+                                              s->d_err, cap, s->d_work, true, false, q - pairs)
                        : launch_yee_step_v(s->d_desc, s->d_tile0, n, s->total_tiles, q, s->rows, s->vec, grid, cap);
-    if (!rc) rc = launch_advance(s->d_desc, n, len, cap);
+    if (!rc) rc = launch_advance(s->d_desc, n, len, cap, flips);
     set_capturing(false);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(cap, &g);
@@ -560,7 +622,7 @@ int chunk_graph(ptk_server *s, int len, int grid, cudaGraphExec_t *out)
 // h_slot, valid after the next synchronisation of the server's stream (retire_finish).
 int retire_copies(ptk_server *s, Inst *in, double *h_slot)
 {
-    const int par = in->done & 1;
+    const int par = in->par;
     SumArgs a{};
     for (int f = 0; f < 6; ++f) {
         a.f[f] = in->buf[par][f];
@@ -815,7 +877,7 @@ try {
         }
         s->flight[b].exec = ex;
         // kernels in the chunk graph: the steps, the step-counter advance and (staged) the faces
-        const int kernels = len + 1 + (s->stages && s->total_faces > 0 ? 1 : 0);
+        const int flips = len - chunk_pairs(s, len), kernels = flips + 1 + (s->stages && s->total_faces > 0 ? 1 : 0);
         count_graph_launch(kernels);
         s->launches += kernels;
         ++s->chunks;
@@ -828,7 +890,8 @@ try {
         const double tr = now_s();
         std::vector<Inst *> still, gone;
         for (Inst *in : s->active) {
-            in->done += std::min(len, in->steps_total - in->done);
+            in->done += len;   // no chunk is longer than the shortest remainder
+            in->par = (in->par + flips) & 1;
             (in->done >= in->steps_total ? gone : still).push_back(in);
         }
         s->active.swap(still);
@@ -949,10 +1012,14 @@ int ptk_server_destroy(ptk_server *s)
     if (s->d_desc) pool_free(s->d_desc, s->st);
     if (s->d_tile0) pool_free(s->d_tile0, s->st);
     if (s->d_face0) pool_free(s->d_face0, s->st);
+    if (s->d_pair) pool_free(s->d_pair, s->st);
+    if (s->d_pair0) pool_free(s->d_pair0, s->st);
     for (int b = 0; b < 2; ++b) {
         if (s->h_desc[b]) cudaFreeHost(s->h_desc[b]);
         if (s->h_tile0[b]) cudaFreeHost(s->h_tile0[b]);
         if (s->h_face0[b]) cudaFreeHost(s->h_face0[b]);
+        if (s->h_pair[b]) cudaFreeHost(s->h_pair[b]);
+        if (s->h_pair0[b]) cudaFreeHost(s->h_pair0[b]);
         if (s->h_sums[b]) cudaFreeHost(s->h_sums[b]);
         if (s->h_up[b]) cudaFreeHost(s->h_up[b]);
     }

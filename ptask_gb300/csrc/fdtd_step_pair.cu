@@ -20,6 +20,10 @@
 // mbarriers with a quarter of a plane's work between a warp's arrival and its wait, so warps rarely
 // stand still; the rows are double buffered to allow that.
 //
+// A batch of instances (MANY) is a CTA per tile, scheduled by the hardware, deepest first: the start of a CTA
+// (3 us) is paid per tile, but a list of uneven tiles balances itself.  85 % of the persistent
+// form's rate on one 256^3, 160 G updates/s on mixes of 32..192 (the one-step kernel: 82).
+//
 // The ring, its bounded waits and the continuous issue across a CTA's tiles are those of the
 // one-step kernel (fdtd_step_bulk.cu).  Arithmetic is the same, operation for operation; with
 // Ca = Da = 1 (PAIR_SIMPLE) the products with them are left out, which changes no bit.
@@ -56,7 +60,8 @@ constexpr int kStage = 6 * kField + kIds;
 constexpr int kRowsAt = kPairStages * kStage, kRowBuf = kRowArrays * kField;
 constexpr int kEdge = 8 * (kPairWarps + 2), kEdgeBuf = kEdgeArrays * kEdge, kEdgesAt = kRowsAt + 2 * kRowBuf;
 constexpr int kTabAt = (kEdgesAt + 2 * kEdgeBuf + 15) / 16 * 16, kBarsAt = kTabAt + 16 * kMaxMaterials;
-constexpr int kPairBytes = kBarsAt + 8 * (kPairStages + 2);
+constexpr int kArgsAt = (kBarsAt + 8 * (kPairStages + 2) + 15) / 16 * 16;
+constexpr int kPairBytes = kArgsAt + (int)sizeof(PairArgs);
 static_assert(kPairBytes <= (int)kPairSmem, "the frame, its rows and the ring fit one CTA");
 
 __device__ __forceinline__ float4 lds4(const char *sm, int o) { return *reinterpret_cast<const float4 *>(sm + o); }
@@ -209,13 +214,33 @@ __device__ __forceinline__ void lookup(const float *tab, unsigned ids, int half,
 
 }  // namespace
 
-template <int MODE>
-__global__ void __launch_bounds__(kPairThreads, 1) k_yee_pair(const InstDesc *__restrict__ D, const PairArgs P, int q, int *err)
+// MANY: a CTA per tile of the batch's instances, in list order; a warp finds its block's instance among the
+// tile counts' prefix sums, and the instance's arguments move to shared memory.  Otherwise: one instance, whose
+// tiles a CTA takes with the grid's stride.
+template <int MODE, bool MANY>
+__global__ void __launch_bounds__(kPairThreads, 1)
+    k_yee_pair(const InstDesc *__restrict__ D, const PairArgs P1, const PairArgs *__restrict__ PN, const int *__restrict__ tile0, int ninst,
+               int q, int *err)
 {
     constexpr bool D1 = MODE == PAIR_SIMPLE;
     constexpr int S = kPairStages;
     extern __shared__ __align__(128) char sm[];
-    const int lw = P.lw, RF = P.rf;
+    const PairArgs &P = MANY ? *reinterpret_cast<const PairArgs *>(sm + kArgsAt) : P1;
+    int t = blockIdx.x;
+    if constexpr (MANY) {
+        // 32 probes a round: the last instance whose first tile is not after this block's
+        int lo = 0, n = ninst;
+        while (n > 1) {
+            const int lane = threadIdx.x & 31, step = (n + 31) / 32;
+            const int c = __popc(__ballot_sync(0xffffffffu, lane * step < n && __ldg(tile0 + lo + min(lane * step, n - 1)) <= t)) - 1;
+            lo += c * step;
+            n = min(step, n - c * step);
+        }
+        t -= __ldg(tile0 + lo);
+        D += lo;
+        const int *from = reinterpret_cast<const int *>(PN + lo);
+        for (int w = threadIdx.x; w < (int)(sizeof(PairArgs) / 4); w += blockDim.x) reinterpret_cast<int *>(sm + kArgsAt)[w] = __ldg(from + w);
+    }
     float *tab = reinterpret_cast<float *>(sm + kTabAt);
     uint64_t *bars = reinterpret_cast<uint64_t *>(sm + kBarsAt), *bar1 = bars + S, *bar2 = bars + S + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -238,6 +263,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_yee_pair(const InstDesc *__
     const float dbu = MODE == PAIR_SIMPLE ? __ldg(gtab).w : 0.f;
     __syncthreads();
 
+    const int lw = P.lw, RF = P.rf;
     const int par = (D->par + q) & 1, step = D->step + 2 * q;
     const CUtensorMap *maps = static_cast<const CUtensorMap *>(P.tma);
     const int nx = D->nx, ny = D->ny, nz = D->nz;
@@ -245,8 +271,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_yee_pair(const InstDesc *__
     const long long src = D->src;
     const float w1 = src >= 0 && step < D->nwave ? __ldg(D->wave + step) : 0.f;
     const float w2 = src >= 0 && step + 1 < D->nwave ? __ldg(D->wave + step + 1) : 0.f;
-    float *const oHx = P.buf[par ^ 1][0], *const oHy = P.buf[par ^ 1][1], *const oHz = P.buf[par ^ 1][2];
-    float *const oEx = P.buf[par ^ 1][3], *const oEy = P.buf[par ^ 1][4], *const oEz = P.buf[par ^ 1][5];
+    // One instance: the six pointers are launch constants.  MANY: one, and the distance of the fields.
+    float *const o0 = P.buf[par ^ 1][0];
+    const long long apart = MANY ? P.buf[par ^ 1][1] - o0 : 0;
+    float *const oHx = o0, *const oHy = MANY ? o0 + apart : P.buf[par ^ 1][1], *const oHz = MANY ? o0 + 2 * apart : P.buf[par ^ 1][2];
+    float *const oEx = MANY ? o0 + 3 * apart : P.buf[par ^ 1][3], *const oEy = MANY ? o0 + 4 * apart : P.buf[par ^ 1][4];
+    float *const oEz = MANY ? o0 + 5 * apart : P.buf[par ^ 1][5];
     const unsigned pitch = D->pitch, plane = (unsigned)D->plane;
 
     // A tile's frame and planes: the planes kstart .. k1 + 1 are loaded, the last one as "next" only.
@@ -267,9 +297,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_yee_pair(const InstDesc *__
                         lane < 6 ? px : px & ~15, py, k, &bars[s]);
     };
     if (lane < 7) tma_acquire(lane < 6 ? maps + par * 6 + lane : maps + 12);
-    if ((int)blockIdx.x < P.tiles) {
+    if (t < P.tiles) {
         int xt, yt, k0, k1, kstart;
-        tile_at(blockIdx.x, xt, yt, k0, k1, kstart);
+        tile_at(t, xt, yt, k0, k1, kstart);
         if (warp == 0)   // a tile has more planes than the ring
             for (int s = 0; s < S; ++s) issue(xt * (4 * lw - 4), yt * (RF - 3), kstart + s, s);
     }
@@ -294,7 +324,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_yee_pair(const InstDesc *__
         }
     };
 
-    for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
+    for (; t < P.tiles; t += gridDim.x) {
         int xt, yt, k0, k1, kstart;
         tile_at(t, xt, yt, k0, k1, kstart);
         const int xs = xt * (4 * lw - 4), js = yt * (RF - 3);
@@ -479,6 +509,20 @@ bool lay_out(PairPlan &p)
 
 }  // namespace
 
+// The frame of `nxt` tiles in x: as many rows as a CTA's threads allow.  False when no such frame exists.
+static bool pair_frame(int nx, int ny, int nxt, PairArgs *a)
+{
+    a->nxt = nxt;
+    a->lw = (nx + 1 + 4 * (nxt - 1) + 4 * nxt - 1) / (4 * nxt);
+    if (a->lw > kMaxLw || (a->lw < 8 && nxt > 1)) return false;
+    a->rf = std::min(std::min(kPairThreads / a->lw, 255), ny + 1);
+    if (a->rf < 5) return false;
+    a->nyt = ny <= a->rf - 1 ? 1 : 1 + (ny - (a->rf - 1) + a->rf - 4) / (a->rf - 3);
+    return true;
+}
+
+static bool pair_fits(int nx, int ny, int nz) { return make_layout(nx, ny, nz).total * 4 < 1LL << 32 && nz >= 8; }
+
 // The tile shape with the least estimated time for two steps: rounds of resident CTAs times the planes each
 // streams (its depth, the planes recomputed at its start, the ring's turn at its end).
 bool plan_pair(int nx, int ny, int nz, PairPlan *out)
@@ -486,24 +530,17 @@ bool plan_pair(int nx, int ny, int nz, PairPlan *out)
     const int sms = sm_count();
     double best = 1e30;
     bool found = false;
-    const Layout L = make_layout(nx, ny, nz);
-    if (sms <= 0 || L.total * 4 >= 1LL << 32 || nz < 8) return false;
+    if (sms <= 0 || !pair_fits(nx, ny, nz)) return false;
     for (int nxt = 1; nxt <= 64; ++nxt) {
-        const int lw = (nx + 1 + 4 * (nxt - 1) + 4 * nxt - 1) / (4 * nxt);
-        if (lw > kMaxLw) continue;
-        if (lw < 8 && nxt > 1) break;
-        const int rf = std::min(std::min(kPairThreads / lw, 255), ny + 1);
-        if (rf < 5) continue;
-        const int nyt = ny <= rf - 1 ? 1 : 1 + (ny - (rf - 1) + rf - 4) / (rf - 3);
+        PairPlan p{};
+        if (!pair_frame(nx, ny, nxt, &p.args)) continue;
         for (int nzt = 1; nzt <= nz / 8; ++nzt) {
             const int kc = (nz + nzt - 1) / nzt;
             if ((nz + kc - 1) / kc != nzt) continue;
-            const long long tiles = (long long)nxt * nyt * nzt, waves = (tiles + sms - 1) / sms;
+            const long long tiles = (long long)nxt * p.args.nyt * nzt, waves = (tiles + sms - 1) / sms;
             const double cost = (double)waves * (kc + 3.5);
-            PairPlan p{};
-            p.args.nxt = nxt; p.args.nyt = nyt; p.args.nzt = nzt; p.args.kc = kc; p.args.lw = lw; p.args.rf = rf;
-            p.args.tiles = (int)tiles;
-            p.threads = (lw * rf + 31) / 32 * 32;
+            p.args.nzt = nzt; p.args.kc = kc; p.args.tiles = (int)tiles;
+            p.threads = (p.args.lw * p.args.rf + 31) / 32 * 32;
             p.grid = (int)std::min<long long>(tiles, sms);
             const double c = cost * (0.35 + 0.65 * p.threads / kPairThreads);
             if (c < best && lay_out(p)) {
@@ -514,6 +551,64 @@ bool plan_pair(int nx, int ny, int nz, PairPlan *out)
         }
     }
     return found;
+}
+
+// In a batch every CTA has all its threads, so the frame is the one with the fewest tiles per plane.  It does
+// not depend on the rest of the batch; the depth does (plan_pair_depths).
+bool plan_pair_member(int nx, int ny, int nz, PairPlan *out)
+{
+    bool found = false;
+    if (!pair_fits(nx, ny, nz)) return false;
+    for (int nxt = 1; nxt <= 64; ++nxt) {
+        PairPlan p{};
+        if (!pair_frame(nx, ny, nxt, &p.args)) continue;
+        const int nyt = p.args.nyt;
+        p.args.rf = std::max(5, std::min(p.args.rf, (ny + 1 + 3 * (nyt - 1) + nyt - 1) / nyt));   // no more rows than these tiles need
+        if (lay_out(p) && (!found || nxt * nyt < out->args.nxt * out->args.nyt)) {
+            *out = p;
+            found = true;
+        }
+    }
+    return found;
+}
+
+static int pair_depth(int nz, int cap)   // near-equal tiles of at most cap planes, if that leaves 8 in each
+{
+    const int parts = std::max(1, std::min((nz + cap - 1) / cap, nz / 8));
+    return (nz + parts - 1) / parts;
+}
+
+// The depths of a batch's tiles: the cap whose list has the least bound on its time, which is the smaller of
+// whole rounds of the deepest tile and (a free SM takes the next tile, deepest first) the mean load plus one
+// tile.  A tile costs its planes, those recomputed, and its CTA's start (about five planes' time).
+void plan_pair_depths(PairPlan *const plans[], const int nz[], int n)
+{
+    constexpr double kStart = 8.5;
+    const int sms = std::max(1, sm_count());
+    int deepest = 8, cap = 8;
+    for (int q = 0; q < n; ++q) deepest = std::max(deepest, nz[q]);
+    double best = 1e30;
+    for (int c = 8; c <= deepest; c += 1 + c / 16) {
+        double tiles = 0, load = 0;
+        int top = 0;
+        for (int q = 0; q < n; ++q) {
+            const int kc = pair_depth(nz[q], c), t = plans[q]->args.nxt * plans[q]->args.nyt * ((nz[q] + kc - 1) / kc);
+            tiles += t;
+            load += t * (kc + kStart);
+            top = std::max(top, kc);
+        }
+        const double rounds = std::ceil(tiles / sms) * (top + kStart), mean = load / sms + top + kStart;
+        if (std::min(rounds, mean) < best) {
+            best = std::min(rounds, mean);
+            cap = c;
+        }
+    }
+    for (int q = 0; q < n; ++q) {
+        PairArgs &a = plans[q]->args;
+        a.kc = pair_depth(nz[q], cap);
+        a.nzt = (nz[q] + a.kc - 1) / a.kc;
+        a.tiles = a.nxt * a.nyt * a.nzt;
+    }
 }
 
 int encode_pair_maps(const InstDesc &d, const PairPlan &p, void *host_out)
@@ -538,14 +633,27 @@ int encode_pair_maps(const InstDesc &d, const PairPlan &p, void *host_out)
     return PTK_OK;
 }
 
-int launch_yee_pair(const InstDesc *d_inst, const PairPlan &p, int mode, int pair, int *err, cudaStream_t s)
+template <int MODE, bool MANY>
+static int launch_pair(const InstDesc *d_inst, const PairArgs &one, const PairArgs *many, const int *tile0, int ninst, int grid, int threads,
+                       int pair, int *err, cudaStream_t s)
 {
-    auto *k = mode == PAIR_SIMPLE ? k_yee_pair<PAIR_SIMPLE> : k_yee_pair<PAIR_TABLE>;
-    PTK_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
-    k<<<p.grid, p.threads, p.smem, s>>>(d_inst, p.args, pair, err);
+    PTK_CUDA_TRY(cudaFuncSetAttribute(k_yee_pair<MODE, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairBytes));
+    k_yee_pair<MODE, MANY><<<grid, threads, kPairBytes, s>>>(d_inst, one, many, tile0, ninst, pair, err);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return PTK_OK;
+}
+
+int launch_yee_pair(const InstDesc *d_inst, const PairPlan &p, int mode, int pair, int *err, cudaStream_t s)
+{
+    return mode == PAIR_SIMPLE ? launch_pair<PAIR_SIMPLE, false>(d_inst, p.args, nullptr, nullptr, 1, p.grid, p.threads, pair, err, s)
+                               : launch_pair<PAIR_TABLE, false>(d_inst, p.args, nullptr, nullptr, 1, p.grid, p.threads, pair, err, s);
+}
+
+int launch_yee_pair_batch(const InstDesc *d_insts, const PairArgs *d_args, const int *d_tile0, int ninst, int tiles, int pair, int *err,
+                          cudaStream_t s)
+{
+    return launch_pair<PAIR_SIMPLE, true>(d_insts, PairArgs{}, d_args, d_tile0, ninst, tiles, kPairThreads, pair, err, s);
 }
 
 }  // namespace ptk

@@ -216,9 +216,17 @@ struct PairPlan {
     size_t smem;
 };
 bool plan_pair(int nx, int ny, int nz, PairPlan *out);
-int encode_pair_maps(const InstDesc &d, const PairPlan &p, void *host_out);   // 13 x 128 bytes
+constexpr size_t kPairMapBytes = 13 * 128;
+int encode_pair_maps(const InstDesc &d, const PairPlan &p, void *host_out);   // kPairMapBytes
 // The two steps at pair offset `pair` of the chunk: from buffer (par + pair) & 1 to the other one.
 int launch_yee_pair(const InstDesc *d_inst, const PairPlan &p, int mode, int pair, int *err, cudaStream_t s);
+// The same for every instance of a batch in one launch (all of them PAIR_SIMPLE, each instance's six fields
+// of a buffer equally far apart): plans by plan_pair_member, depths for the batch by plan_pair_depths; d_tile0:
+// ninst + 1 prefix sums of the instances' tiles, `tiles` in total.
+bool plan_pair_member(int nx, int ny, int nz, PairPlan *out);
+void plan_pair_depths(PairPlan *const plans[], const int nz[], int n);
+int launch_yee_pair_batch(const InstDesc *d_insts, const PairArgs *d_args, const int *d_tile0, int ninst, int tiles, int pair, int *err,
+                          cudaStream_t s);
 
 // Step counters on by nsteps (as far as each instance has steps left), buffers on by `flips` (-1: one per step).
 int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s, int flips = -1);

@@ -201,3 +201,25 @@ def test_served_trace_matches_oracle():
             assert oracle.normwise_error(fetched[q][f], ref[f]) <= 1e-5
             np.testing.assert_array_equal(fetched[q][f], ref[f], err_msg=f"request {q} ({r.nx}^3 x {r.steps}) "
                                                                          f"field {P.FIELDS[f]}")
+
+
+@pytest.mark.parametrize("chunk", [1, 2, 7, 32])
+@pytest.mark.parametrize("shapes", [
+    [(1, 4, 8), (27, 13, 8), (28, 12, 9), (29, 11, 17), (239, 5, 8), (240, 4, 10), (64, 64, 24)],   # ends of frames
+    [(20, 16, 12), (18, 3, 12), (33, 20, 9)],              # one too thin for two steps per pass: it leaves first
+    [(9 + q % 23, 4 + q % 17, 8 + q % 5) for q in range(70)],   # more instances than a warp has lanes, twice over
+])
+def test_two_steps_per_pass_in_a_batch(shapes, chunk):
+    """Batches advanced two steps at a time, at odd and even chunk lengths and remainders, against the oracle."""
+    reqs = [Request(*n, 5 + (3 * q) % 11 if n[1] > 3 else 4, 1 + q % 3, 60 + q, box=(1, 6)) for q, n in enumerate(shapes)]
+    with Server(keep_results=True, chunk_steps=chunk) as s:
+        tickets = [s.submit(r) for r in reqs]
+        s.run(time_scale=0)
+        for t, r in zip(tickets, reqs):
+            got = s.fetch(t)
+            pr = P.Problem.generate(r.nx, r.ny, r.nz, n_boxes=r.n_boxes, eps=r.eps, box=r.box, steps=r.steps,
+                                    source_mode=r.source_mode, seed=r.seed)
+            ref = oracle.step_ext_f32(P.zero_fields(r.nx, r.ny, r.nz), r.steps, pr.params, pr.Ca, pr.Cb, pr.Da,
+                                      pr.Db, pr.src, pr.wave)
+            for q in range(6):
+                np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{r} {P.FIELDS[q]}")
