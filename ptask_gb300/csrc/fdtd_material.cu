@@ -31,6 +31,7 @@ struct MatScratch {
     int id[kSlots];
     int count;                // distinct tuples inserted
     int err;                  // 1: a poll expired, 2: the table filled up
+    int varied;               // a node with Ca or Da other than 1, or another Db than the first node's
     MaterialInfo info;        // result
 };
 
@@ -105,12 +106,16 @@ __global__ void __launch_bounds__(256) k_mat_insert(const float *Ca, const float
 {
     const float *c[4] = {Ca, Cb, Da, Db};
     const int lane = threadIdx.x & 31;
+    const unsigned db = __float_as_uint(__ldg(Db));
     uint4 last = make_uint4(0, 0, 0, 0);   // the tuple this lane saw last (in the table already)
-    bool have_last = false;
+    bool have_last = false, varied = false;
     for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < N.rows; r += gridDim.x * 8) {
         const long long o = N.row(r);
+        const bool full = *reinterpret_cast<volatile int *>(&S->count) > kMaxMaterials;   // no index: only `varied` is left to see
         for (int i = lane; i <= N.nx; i += 32) {
             const uint4 key = tuple_at(c, o + i);
+            varied |= key.x != 0x3f800000u || key.z != 0x3f800000u || key.w != db;
+            if (full) continue;
             const bool fresh = !(have_last && same(key, last));
             const unsigned act = __activemask();
             if (!__any_sync(act, fresh)) continue;
@@ -122,37 +127,33 @@ __global__ void __launch_bounds__(256) k_mat_insert(const float *Ca, const float
             have_last = true;
         }
     }
+    if (varied) S->varied = 1;
 }
 
 // Numbers the occupied slots in slot order, a thread per slot (one thread for all of them: 56 us).
-__global__ void __launch_bounds__(kSlots) k_mat_compact(MatScratch *S, float4 *tab)
+__global__ void __launch_bounds__(kSlots) k_mat_compact(MatScratch *S, float4 *tab, const float *Db)
 {
     __shared__ int before[kSlots / 32];
-    __shared__ unsigned db;
     const int h = threadIdx.x, lane = h & 31, warp = h >> 5;
     const bool on = S->state[h] == 2u;
     const unsigned mask = __ballot_sync(0xffffffffu, on);
     if (lane == 0) before[warp] = __popc(mask);
-    if (h == 0) db = 0;
     __syncthreads();
     int id = __popc(mask & ((1u << lane) - 1)), n = 0;
     for (int w = 0; w < kSlots / 32; ++w) {
         if (w == warp) id += n;
         n += before[w];
     }
-    const uint4 k = on ? S->key[h] : make_uint4(0, 0, 0, 0);
     if (on) {
+        const uint4 k = S->key[h];
         if (id < kMaxMaterials)
             tab[id] = make_float4(__uint_as_float(k.x), __uint_as_float(k.y), __uint_as_float(k.z), __uint_as_float(k.w));
         S->id[h] = id;
-        if (id == 0) db = k.w;
     }
-    __syncthreads();
-    const bool simple = __syncthreads_and(!on || (k.x == 0x3f800000u && k.z == 0x3f800000u && k.w == db));
     if (h == 0) {
         S->info.nmat = (S->err || n > kMaxMaterials || n != S->count) ? 0 : n;
-        S->info.simple = S->info.nmat > 0 && simple;
-        S->info.db = __uint_as_float(db);
+        S->info.simple = !S->varied;
+        S->info.db = *Db;
     }
 }
 
@@ -195,7 +196,7 @@ int build_material_index(const float *const coef[4], const Layout &L, unsigned c
     Nodes N{L.nx, L.ny, L.pitch, (L.ny + 1) * (L.nz + 1), L.plane};
     const int grid = std::min((N.rows + 7) / 8, 8 * std::max(1, sm_count()));
     k_mat_insert<<<grid, 256, 0, s>>>(coef[0], coef[1], coef[2], coef[3], N, S);
-    k_mat_compact<<<1, kSlots, 0, s>>>(S, reinterpret_cast<float4 *>(tab));
+    k_mat_compact<<<1, kSlots, 0, s>>>(S, reinterpret_cast<float4 *>(tab), coef[3]);
     k_mat_index<<<grid, 256, 0, s>>>(coef[0], coef[1], coef[2], coef[3], N, S, mat);
     PTK_CUDA_TRY(cudaGetLastError());
     count_launches(3);

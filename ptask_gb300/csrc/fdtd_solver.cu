@@ -148,6 +148,14 @@ struct RunShape {
     bool mat;
 };
 
+// How the two-step kernel would get the coefficients, or -1: four arrays that all vary are not for it.
+static int pair_mode(const ptk_solver *s)
+{
+    if (!s->mat_enabled || s->stages <= 0) return -1;
+    if (use_mat(s)) return s->minfo.simple ? PAIR_SIMPLE : PAIR_TABLE;
+    return s->minfo.simple ? PAIR_CELLS : -1;
+}
+
 static RunShape run_shape(const ptk_solver *s)
 {
     if (s->stages <= 0) return {s->by, 0, false};
@@ -284,7 +292,7 @@ static void drop_graphs(ptk_solver *s)
 static int solver_graph(ptk_solver *s, int len, bool pair, cudaGraphExec_t *out)
 {
     const RunShape rs = run_shape(s);
-    const int mode = s->minfo.simple ? PAIR_SIMPLE : PAIR_TABLE;
+    const int mode = pair_mode(s);
     GraphKey key{len, rs.by, s->kc, s->vec, rs.stages * 2 + (rs.mat ? 1 : 0), pair ? 1 + mode : 0};
     auto it = s->graphs.find(key);
     if (it != s->graphs.end()) {
@@ -331,8 +339,9 @@ static int solver_graph(ptk_solver *s, int len, bool pair, cudaGraphExec_t *out)
     return PTK_OK;
 }
 
-// Larger grids with a material index take runs of this many steps or more two steps per launch
-// (fdtd_step_pair.cu); shorter ones run the tile shape that was set.
+// Larger grids with a material index, or with a Cb per cell and nothing else that varies (160^3: 30.3 us per
+// step against 83 by the one-step kernel with four arrays), take runs of this many steps or more two steps per
+// launch (fdtd_step_pair.cu); shorter ones run the tile shape that was set.
 static constexpr int kPairSteps = 16;
 
 static int run_resident(ptk_solver *s, int steps, cudaStream_t st)
@@ -368,7 +377,7 @@ int solver_run(ptk_solver *s, int steps, cudaStream_t st)
     if (s->resident && s->stages > 0 && steps >= kResidentSteps && !s->plain) return run_resident(s, steps, st);
     int rc = solver_sync_desc(s, steps, st);
     if (rc) return rc;
-    const bool pair = s->pair && run_shape(s).mat && steps >= kPairSteps && !s->plain;
+    const bool pair = s->pair && pair_mode(s) >= 0 && steps >= kPairSteps && !s->plain;
     if (pair && !s->pair_maps) {   // the arrays never move: encoded once
         alignas(64) unsigned char maps[kTmaSetBytes];
         InstDesc e = host_desc(s, steps);

@@ -26,7 +26,9 @@
 //
 // The ring, its bounded waits and the continuous issue across a CTA's tiles are those of the
 // one-step kernel (fdtd_step_bulk.cu).  Arithmetic is the same, operation for operation; with
-// Ca = Da = 1 (PAIR_SIMPLE) the products with them are left out, which changes no bit.
+// Ca = Da = 1 (PAIR_SIMPLE) the products with them are left out, which changes no bit.  PAIR_CELLS takes Cb
+// from its array, 26 bytes per update: the ring has no room for a seventh field, but a thread needs only its
+// own unit, loaded into registers a plane ahead.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     k_yee_pair(const InstDesc *__restrict__ D, const PairArgs P1, const PairArgs *__restrict__ PN, const int *__restrict__ tile0, int ninst,
                int q, int *err)
 {
-    constexpr bool D1 = MODE == PAIR_SIMPLE;
+    constexpr bool D1 = MODE != PAIR_TABLE, CELLS = MODE == PAIR_CELLS;
     constexpr int S = kPairStages;
     extern __shared__ __align__(128) char sm[];
     const PairArgs &P = MANY ? *reinterpret_cast<const PairArgs *>(sm + kArgsAt) : P1;
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         if (MODE == PAIR_SIMPLE) tab[m] = v.y;
         else reinterpret_cast<float4 *>(tab)[m] = v;
     }
-    const float dbu = MODE == PAIR_SIMPLE ? __ldg(gtab).w : 0.f;
+    const float dbu = MODE == PAIR_SIMPLE ? __ldg(gtab).w : CELLS ? __ldg(D->coef[3]) : 0.f;
     __syncthreads();
 
     const int lw = P.lw, RF = P.rf;
@@ -290,13 +292,13 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     };
     // Copies of plane k of the frame at (px, py) into ring slot s, by one warp.
     auto issue = [&](int px, int py, int k, int s) {
-        if (lane == 0) mbar_expect_tx(&bars[s], (uint32_t)P.tx_bytes);
+        if (lane == 0) mbar_expect_tx(&bars[s], (uint32_t)(CELLS ? P.tx_bytes - P.mw * P.rf : P.tx_bytes));
         __syncwarp();
-        if (lane < 7)
+        if (lane < (CELLS ? 6 : 7))
             tma_load_3d(sm + s * kStage + lane * kField, lane < 6 ? maps + par * 6 + lane : maps + 12,
                         lane < 6 ? px : px & ~15, py, k, &bars[s]);
     };
-    if (lane < 7) tma_acquire(lane < 6 ? maps + par * 6 + lane : maps + 12);
+    if (lane < (CELLS ? 6 : 7)) tma_acquire(lane < 6 ? maps + par * 6 + lane : maps + 12);
     if (t < P.tiles) {
         int xt, yt, k0, k1, kstart;
         tile_at(t, xt, yt, k0, k1, kstart);
@@ -346,7 +348,12 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         const int mo = 6 * kField + r * P.mw + (xs & 15) + 4 * lx;
 
         F3 H1a{}, H1b{}, E1a{}, E1b{}, H2a{}, H2b{};
-        float4 cb_m{}, cb_mm{};            // PAIR_SIMPLE: Cb of planes k-1, k-2
+        // PAIR_CELLS: Cb of the node, loaded a plane ahead; units beyond the rows repeat one within
+        const float *const cbp = CELLS ? D->coef[1] + (min((unsigned)i, pitch - 4) + pitch * (unsigned)min(j, ny)) : nullptr;
+        auto cb_at = [&](int k) { return __ldg(reinterpret_cast<const float4 *>(cbp + plane * (unsigned)min(k, nz))); };
+        float4 cb_n{};
+        if constexpr (CELLS) cb_n = cb_at(kstart);
+        float4 cb_m{}, cb_mm{};            // Ca = Da = 1: Cb of planes k-1, k-2
         unsigned id_m = 0, id_mm = 0;      // otherwise their material ids
 
         // E2(kk) from H2(kk) (own, and the rows of buffer b), H2(kk-1); H2 and E2 stored.
@@ -359,7 +366,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             if (edge_lo) { hyp = e.x; hzp = e.y; }
             const float4 hxj = lds4(rd, kRowsAt + R_HX2 * kField), hzj = lds4(rd, kRowsAt + R_HZ2 * kField);
             float4 Dc = make_float4(1.f, 1.f, 1.f, 1.f), Cc = cb;
-            if constexpr (MODE != PAIR_SIMPLE) lookup<MODE>(tab, ids, 0, Dc, Cc);
+            if constexpr (MODE == PAIR_TABLE) lookup<MODE>(tab, ids, 0, Dc, Cc);
             e_update<D1>(E1, Dc, Cc, H2, H2m.x, H2m.y, hxj, hzj, hyp, hzp, in, kk >= 1, cx, cy, cz);
             if (kk == src_k) add_source(E1.z, src_c, w2);
             if (full) {
@@ -403,7 +410,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             e0.x = lds4(co, 3 * kField);
             e0.y = lds4(co, 4 * kField);
             e0.z = lds4(co, 5 * kField);
-            const unsigned ids = *reinterpret_cast<const unsigned *>(cur + mo);
+            unsigned ids = 0;
+            if constexpr (!CELLS) ids = *reinterpret_cast<const unsigned *>(cur + mo);
             float4 Dh = make_float4(1.f, 1.f, 1.f, 1.f), Ch = make_float4(dbu, dbu, dbu, dbu), Dc, Cc;
             {
                 const char *cj = co + rs, *ch = cur + o_hi;
@@ -412,12 +420,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 H1.y = lds4(co, kField);
                 H1.z = lds4(co, 2 * kField);
                 const float eyl = lds1(ch, 4 * kField), ezl = lds1(ch, 5 * kField);
-                lookup<MODE>(tab, ids, 0, Dc, Cc);
+                if constexpr (CELLS) {
+                    Cc = cb_n;
+                    cb_n = cb_at(k + 1);
+                } else {
+                    lookup<MODE>(tab, ids, 0, Dc, Cc);
+                }
                 wait(&bars[ns], nph);
                 const float4 exk = lds4(no, 3 * kField), eyk = lds4(no, 4 * kField);
                 float ezn = __shfl_down_sync(0xffffffffu, e0.z.x, 1), eyn = __shfl_down_sync(0xffffffffu, e0.y.x, 1);
                 if (edge_hi) { eyn = eyl; ezn = ezl; }
-                if constexpr (MODE != PAIR_SIMPLE) lookup<MODE>(tab, ids, 1, Dh, Ch);
+                if constexpr (MODE == PAIR_TABLE) lookup<MODE>(tab, ids, 1, Dh, Ch);
                 h_update<D1>(H1, Dh, Ch, e0, exk, eyk, exj, ezj, eyn, ezn, cx, cy, cz);
             }
             sts4(rw, kRowsAt + R_HX1 * kField, H1.x);
@@ -458,7 +471,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             if (lane == 0) *reinterpret_cast<float2 *>(ew + kEdgesAt + X_E1 * kEdge + e_own) = make_float2(E1.y.x, E1.z.x);
             // ---- H2(k-1) ----
             if (k > kstart) {
-                if constexpr (MODE != PAIR_SIMPLE) lookup<MODE>(tab, id_m, 1, Dh, Ch);
+                if constexpr (MODE == PAIR_TABLE) lookup<MODE>(tab, id_m, 1, Dh, Ch);
                 H2 = H1m;
                 h_update<D1>(H2, Dh, Ch, E1m, E1.x, E1.y, exj, ezj, eyn, ezn, cx, cy, cz);
                 sts4(rw, kRowsAt + R_HX2 * kField, H2.x);
@@ -647,7 +660,8 @@ static int launch_pair(const InstDesc *d_inst, const PairArgs &one, const PairAr
 int launch_yee_pair(const InstDesc *d_inst, const PairPlan &p, int mode, int pair, int *err, cudaStream_t s)
 {
     return mode == PAIR_SIMPLE ? launch_pair<PAIR_SIMPLE, false>(d_inst, p.args, nullptr, nullptr, 1, p.grid, p.threads, pair, err, s)
-                               : launch_pair<PAIR_TABLE, false>(d_inst, p.args, nullptr, nullptr, 1, p.grid, p.threads, pair, err, s);
+           : mode == PAIR_CELLS  ? launch_pair<PAIR_CELLS, false>(d_inst, p.args, nullptr, nullptr, 1, p.grid, p.threads, pair, err, s)
+                                 : launch_pair<PAIR_TABLE, false>(d_inst, p.args, nullptr, nullptr, 1, p.grid, p.threads, pair, err, s);
 }
 
 int launch_yee_pair_batch(const InstDesc *d_insts, const PairArgs *d_args, const int *d_tile0, int ninst, int tiles, int pair, int *err,

@@ -98,10 +98,10 @@ constexpr int kMaxMaterials = 256;
 // distinct tuples of the nodes (i <= Nx, j <= Ny, k <= Nz; row padding excluded) are gathered on
 // the device; if there are at most kMaxMaterials of them, `mat` (L.total bytes, padding left as
 // is) receives each node's id and `tab` (kMaxMaterials x 4 floats) the tuples, and info->nmat their
-// count; otherwise info->nmat = 0 and the index must not be used.  Synchronises `s`.
+// count; otherwise info->nmat = 0 and the index must not be used (`simple` and `db` hold all the same).  Synchronises `s`.
 struct MaterialInfo {
     int nmat;       // materials in the table, 0 = no index
-    int simple;     // every material has Ca = Da = 1 and the same Db (lossless, nothing magnetic)
+    int simple;     // every node has Ca = Da = 1 and the same Db (lossless, nothing magnetic), index or not
     float db;       // that Db
 };
 int build_material_index(const float *const coef[4], const Layout &L, unsigned char *mat, float *tab, MaterialInfo *info,
@@ -202,7 +202,8 @@ int launch_yee_resident(const ResidentPlan &p, int coef, ResidentArgs a, cudaStr
 // ---------------------------------------------------------------------------------------------
 // Two time steps in one pass over memory (fdtd_step_pair.cu), with the material index.
 // ---------------------------------------------------------------------------------------------
-enum { PAIR_SIMPLE = 0, PAIR_TABLE = 1 };   // every material Ca = Da = 1 and one Db, or any
+// Coefficients: the index's table with Ca = Da = 1 and one Db, or any table, or an array of Cb with Ca = Da = 1 and one Db.
+enum { PAIR_SIMPLE = 0, PAIR_TABLE = 1, PAIR_CELLS = 2 };
 struct PairArgs {
     int nxt, nyt, nzt, kc, tiles;   // tiles in x, y, z (kc planes deep)
     int lw, rf, mw;                 // units per row and rows of a frame; bytes of a row of material ids

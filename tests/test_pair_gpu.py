@@ -78,3 +78,30 @@ def test_clock_reset_after_an_odd_number_of_buffer_flips():
     for q in range(6):
         np.testing.assert_array_equal(got[q], ref[q], err_msg=P.FIELDS[q])
         np.testing.assert_array_equal(again[q], ref[q], err_msg=P.FIELDS[q])
+
+
+@pytest.mark.parametrize("vary", ["permittivity", "one_Ca", "one_Db"])
+@pytest.mark.parametrize("shape", SHAPES + [(40, 33, 28)])   # the last fits on chip
+def test_permittivity_of_every_cell(shape, vary):
+    """More materials than the index holds: Cb from its array while Ca = Da = 1 and Db is one value; one cell
+    that breaks that (its last) sends the run to the kernels that read all four arrays."""
+    steps = 17
+    pr = P.Problem.generate(*shape, n_boxes=0, steps=steps, source_mode=2, seed=sum(shape))
+    pr.Cb *= np.random.default_rng(5).uniform(0.2, 1.0, pr.Cb.shape).astype(np.float32)
+    if vary == "one_Ca":
+        pr.Ca.flat[-1] = np.float32(0.98)
+    if vary == "one_Db":
+        pr.Db.flat[-1] *= np.float32(0.5)
+    f = P.random_fields(*shape, seed=92, scale=1e-2)
+    ref = oracle.step_ext_f32(f, steps, pr.params, pr.Ca, pr.Cb, pr.Da, pr.Db, pr.src, pr.wave)
+    with P.Solver(pr.params) as s:
+        s.set_tiles(11, 0, 4, 4)
+        s.set_problem(pr)
+        assert s.material_count() == 0
+        s.set_fields(f)
+        s.run(steps)
+        if shape[0] > 40:
+            assert s.last_launches() == (steps // 2 + 2 if vary == "permittivity" else steps + 1)
+        got = s.get_fields()
+    for q in range(6):
+        np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{shape} {P.FIELDS[q]}")
