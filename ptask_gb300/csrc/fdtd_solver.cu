@@ -59,7 +59,7 @@ static void default_tiles(int nx, int ny, int nz, int *by, int *kc, int *vec)
 }
 
 // Grids of this many cells or more start with the staged kernel's shape, whose longer runs are one
-// resident launch or take two steps per pass (32^3: 1.8 us per step against 5.5; 256^3: 97 against 215).
+// resident launch or take two steps per pass (32^3: 1.8 us per step against 5.5; 256^3: 87 against 215).
 // Smaller ones keep the register kernel and a launch per step, which callers count
 // (ptk_solver_last_launches).
 static constexpr long long kStagedCells = 1 << 14;
@@ -339,7 +339,7 @@ static int solver_graph(ptk_solver *s, int len, bool pair, cudaGraphExec_t *out)
     return PTK_OK;
 }
 
-// Larger grids with a material index, or with a Cb per cell and nothing else that varies (160^3: 30.3 us per
+// Larger grids with a material index, or with a Cb per cell and nothing else that varies (160^3: 25.4 us per
 // step against 83 by the one-step kernel with four arrays), take runs of this many steps or more two steps per
 // launch (fdtd_step_pair.cu); shorter ones run the tile shape that was set.
 static constexpr int kPairSteps = 16;

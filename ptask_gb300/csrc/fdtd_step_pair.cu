@@ -20,8 +20,14 @@
 // mbarriers with a quarter of a plane's work between a warp's arrival and its wait, so warps rarely
 // stand still; the rows are double buffered to allow that.
 //
+// What bounds it: the time a warp takes for a plane, some 3300 cycles for 570 instructions, a fifth of them in
+// the three waits; 48 % of the issue slots and 4.7 of 6.8 TB/s are used at 256^3.  Warps that wait for their
+// neighbours only (counters polled in shared memory, 107 us per step against 93 at the time), a fourth ring
+// stage with fewer warps (100) and two CTAs of half the frame per SM (95) were all slower.  A launch starts while
+// the one before it ends (programmatic dependent launch) and waits only before its first copy: 1.1 us a step.
+//
 // A batch of instances (MANY) is a CTA per tile, scheduled by the hardware, deepest first: the start of a CTA
-// (3 us) is paid per tile, but a list of uneven tiles balances itself.  85 % of the persistent
+// (3 us) is paid per tile, but a list of uneven tiles balances itself.  94 % of the persistent
 // form's rate on one 256^3, 160 G updates/s on mixes of 32..192 (the one-step kernel: 82).
 //
 // The ring, its bounded waits and the continuous issue across a CTA's tiles are those of the
@@ -35,13 +41,18 @@
 #include "fdtd_device.cuh"
 #include "fdtd_tma.cuh"
 
+#include <type_traits>
+
 namespace ptk {
 
 namespace {
 
 using namespace tma;
 
-constexpr int kPairThreads = 384;     // at most: 168 registers each
+// Threads of a CTA at most, with 168 registers each: the code that the compiler makes for 11 warps takes 3-6 %
+// less time per plane than for 12 (256^3: 87 us per step against 90-93), and 8 warps with more registers lose
+// more to the smaller frame's halo (103) than they gain.
+constexpr int kPairThreads = 352;
 constexpr int kPairWarps = kPairThreads / 32;
 constexpr int kPairStages = 3;
 constexpr size_t kPairSmem = 232448;
@@ -58,11 +69,11 @@ enum { X_H1 = 0, X_E1 = 1, X_H2 = 2 };
 constexpr int kMaxLw = 60;            // a TMA box is at most 256 elements wide, the ids 15 more than the row
 constexpr int kField = (16 * (kPairThreads + kMaxLw + 1) + 127) / 128 * 128;
 constexpr int kIds = 3072;
-constexpr int kStage = 6 * kField + kIds;
+constexpr int kFull = 6 * kField + kIds, kStage = kFull + 128;   // its barrier behind them
 constexpr int kRowsAt = kPairStages * kStage, kRowBuf = kRowArrays * kField;
 constexpr int kEdge = 8 * (kPairWarps + 2), kEdgeBuf = kEdgeArrays * kEdge, kEdgesAt = kRowsAt + 2 * kRowBuf;
-constexpr int kTabAt = (kEdgesAt + 2 * kEdgeBuf + 15) / 16 * 16, kBarsAt = kTabAt + 16 * kMaxMaterials;
-constexpr int kArgsAt = (kBarsAt + 8 * (kPairStages + 2) + 15) / 16 * 16;
+constexpr int kTabAt = (kEdgesAt + 2 * kEdgeBuf + 15) / 16 * 16, kBar1 = kTabAt + 16 * kMaxMaterials, kBar2 = kBar1 + 8;
+constexpr int kBaseAt = kBar2 + 8, kArgsAt = kBaseAt + 16;
 constexpr int kPairBytes = kArgsAt + (int)sizeof(PairArgs);
 static_assert(kPairBytes <= (int)kPairSmem, "the frame, its rows and the ring fit one CTA");
 
@@ -72,17 +83,19 @@ __device__ __forceinline__ void sts4(char *sm, int o, float4 v) { *reinterpret_c
 __device__ __forceinline__ float2 lds2(const char *sm, int o) { return *reinterpret_cast<const float2 *>(sm + o); }
 __device__ __forceinline__ float lds1(const char *sm, int o) { return *reinterpret_cast<const float *>(sm + o); }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
+__device__ __forceinline__ uint64_t *bar_at(char *sm, int o) { return reinterpret_cast<uint64_t *>(sm + o); }
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ bool mbar_done(uint64_t *bar, uint32_t parity)
+__device__ __forceinline__ bool mbar_done(uint32_t bar, uint32_t parity)
 {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done)
-                 : "r"(smem_u32(bar)), "r"(parity)
+                 : "r"(bar), "r"(parity)
                  : "memory");
     return done != 0;
 }
@@ -91,9 +104,10 @@ struct F3 {
     float4 x, y, z;
 };
 
-// Packed pairs of FP32 (sm_100 and up): differences and products of two cells in one instruction, each
-// rounded as its scalar form.  Sums of products stay scalar: ptxas fuses a packed product and the
-// packed sum that takes it, .rn or not, which would change the bits.
+// Packed pairs of FP32 (sm_100 and up): two cells in one instruction, each rounded as its scalar form.
+// ptxas fuses a packed product and the packed sum that takes it, .rn or not, which would change the bits;
+// a sum is therefore a packed multiply-add by one (or minus one), exact in its product, whose ones come from the
+// launch arguments so that the compiler cannot see them.
 struct P2 {
     float a, b;
 };
@@ -114,20 +128,34 @@ __device__ __forceinline__ P2 mul2(float a0, float a1, float b0, float b1)
     return r;
 }
 
+// a one + b: the sum a + b, or with one = -1 the difference b - a
+__device__ __forceinline__ P2 sum2(float a0, float a1, float one, P2 b)
+{
+    P2 r;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmov.b64 z, {%5, %6};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(r.a), "=f"(r.b)
+        : "f"(a0), "f"(a1), "f"(one), "f"(b.a), "f"(b.b));
+    return r;
+}
+
+// What every update takes: Cx, Cy, Cz, and 1 and -1.
+struct Scalars {
+    float cx, cy, cz, one, minus;
+};
+
 // Two cells: h <- d h + c (da s1 - db s2) from the differences da, db.
 template <bool D1>
-__device__ __forceinline__ void upd2(float &h0, float &h1, float d0, float d1, float c0, float c1, P2 da, float s1, P2 db, float s2)
+__device__ __forceinline__ void upd2(float &h0, float &h1, float d0, float d1, float c0, float c1, P2 da, float s1, P2 db, float s2,
+                                     const Scalars &S)
 {
-    const P2 p = mul2(da.a, da.b, s1, s1), m = mul2(db.a, db.b, s2, s2);
-    const P2 t = mul2(c0, c1, __fsub_rn(p.a, m.a), __fsub_rn(p.b, m.b));
-    if constexpr (D1) {
-        h0 = __fadd_rn(h0, t.a);
-        h1 = __fadd_rn(h1, t.b);
-    } else {
-        const P2 g = mul2(d0, d1, h0, h1);
-        h0 = __fadd_rn(g.a, t.a);
-        h1 = __fadd_rn(g.b, t.b);
-    }
+    const P2 p = mul2(da.a, da.b, s1, s1), m = mul2(db.a, db.b, s2, s2), curl = sum2(m.a, m.b, S.minus, p);
+    const P2 t = mul2(c0, c1, curl.a, curl.b);
+    P2 g{h0, h1};
+    if constexpr (!D1) g = mul2(d0, d1, h0, h1);
+    g = sum2(g.a, g.b, S.one, t);
+    h0 = g.a;
+    h1 = g.b;
 }
 
 // All four cells of a unit; differences of whole units, or (x) along the unit with its neighbour n.
@@ -147,20 +175,21 @@ __device__ __forceinline__ D4 diff_down(const float4 &a, float n)   // a[i] - a[
     return {{__fsub_rn(a.x, n), __fsub_rn(a.y, a.x)}, {__fsub_rn(a.z, a.y), __fsub_rn(a.w, a.z)}};
 }
 template <bool D1>
-__device__ __forceinline__ void upd4(float4 &h, const float4 &d, const float4 &c, const D4 &da, float s1, const D4 &db, float s2)
+__device__ __forceinline__ void upd4(float4 &h, const float4 &d, const float4 &c, const D4 &da, float s1, const D4 &db, float s2,
+                                     const Scalars &S)
 {
-    upd2<D1>(h.x, h.y, d.x, d.y, c.x, c.y, da.lo, s1, db.lo, s2);
-    upd2<D1>(h.z, h.w, d.z, d.w, c.z, c.w, da.hi, s1, db.hi, s2);
+    upd2<D1>(h.x, h.y, d.x, d.y, c.x, c.y, da.lo, s1, db.lo, s2, S);
+    upd2<D1>(h.z, h.w, d.z, d.w, c.z, c.w, da.hi, s1, db.hi, s2, S);
 }
 
 // H <- D H + C curl(E): E at the node, Ex, Ey one plane up, Ex, Ez one row up, Ey, Ez one cell on.
 template <bool D1>
 __device__ __forceinline__ void h_update(F3 &h, const float4 &D, const float4 &C, const F3 &e, const float4 &exk, const float4 &eyk,
-                                         const float4 &exj, const float4 &ezj, float eyn, float ezn, float cx, float cy, float cz)
+                                         const float4 &exj, const float4 &ezj, float eyn, float ezn, const Scalars &S)
 {
-    upd4<D1>(h.x, D, C, diff(eyk, e.y), cz, diff(ezj, e.z), cy);
-    upd4<D1>(h.y, D, C, diff_up(e.z, ezn), cx, diff(exk, e.x), cz);
-    upd4<D1>(h.z, D, C, diff(exj, e.x), cy, diff_up(e.y, eyn), cx);
+    upd4<D1>(h.x, D, C, diff(eyk, e.y), S.cz, diff(ezj, e.z), S.cy, S);
+    upd4<D1>(h.y, D, C, diff_up(e.z, ezn), S.cx, diff(exk, e.x), S.cz, S);
+    upd4<D1>(h.z, D, C, diff(exj, e.x), S.cy, diff_up(e.y, eyn), S.cx, S);
 }
 
 // Where a node's E is updated (not on a wall): by row, by plane, by cell of the unit.
@@ -172,19 +201,19 @@ struct Inside {
 template <bool D1>
 __device__ __forceinline__ void e_update(F3 &e, const float4 &D, const float4 &C, const F3 &h, const float4 &hxk, const float4 &hyk,
                                          const float4 &hxj, const float4 &hzj, float hyp, float hzp, const Inside &in, bool k,
-                                         float cx, float cy, float cz)
+                                         const Scalars &S)
 {
     float4 n = e.x;
-    upd4<D1>(n, D, C, diff(h.z, hzj), cy, diff(h.y, hyk), cz);
+    upd4<D1>(n, D, C, diff(h.z, hzj), S.cy, diff(h.y, hyk), S.cz, S);
     if (in.j && k) e.x = n;
     n = e.y;
-    upd4<D1>(n, D, C, diff(h.x, hxk), cz, diff_down(h.z, hzp), cx);
+    upd4<D1>(n, D, C, diff(h.x, hxk), S.cz, diff_down(h.z, hzp), S.cx, S);
     if (k && in.x0) e.y.x = n.x;
     if (k && in.x1) e.y.y = n.y;
     if (k && in.x2) e.y.z = n.z;
     if (k && in.x3) e.y.w = n.w;
     n = e.z;
-    upd4<D1>(n, D, C, diff_down(h.y, hyp), cx, diff(h.x, hxj), cy);
+    upd4<D1>(n, D, C, diff_down(h.y, hyp), S.cx, diff(h.x, hxj), S.cy, S);
     if (in.j && in.x0) e.z.x = n.x;
     if (in.j && in.x1) e.z.y = n.y;
     if (in.j && in.x2) e.z.z = n.z;
@@ -244,16 +273,16 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         for (int w = threadIdx.x; w < (int)(sizeof(PairArgs) / 4); w += blockDim.x) reinterpret_cast<int *>(sm + kArgsAt)[w] = __ldg(from + w);
     }
     float *tab = reinterpret_cast<float *>(sm + kTabAt);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + kBarsAt), *bar1 = bars + S, *bar2 = bars + S + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (smem_u32(sm) & 127u) {   // TMA destinations need 128-byte alignment: refuse, do not fault
         if (tid == 0) atomicOr(err, 2);
         return;
     }
     if (tid == 0) {
-        for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
-        mbar_init(bar1, blockDim.x / 32);
-        mbar_init(bar2, blockDim.x / 32);
+        for (int s = 0; s < S; ++s) mbar_init(bar_at(sm, s * kStage + kFull), 1);
+        mbar_init(bar_at(sm, kBar1), blockDim.x / 32);
+        mbar_init(bar_at(sm, kBar2), blockDim.x / 32);
+        *reinterpret_cast<uint32_t *>(sm + kBaseAt) = smem_u32(sm);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     const float4 *gtab = reinterpret_cast<const float4 *>(D->mat_tab);
@@ -265,11 +294,14 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     const float dbu = MODE == PAIR_SIMPLE ? __ldg(gtab).w : CELLS ? __ldg(D->coef[3]) : 0.f;
     __syncthreads();
 
+    // The window's base for the barriers' addresses, read back so that it stays in a register: the compiler
+    // would rather work it out again at every barrier.
+    const uint32_t base = *reinterpret_cast<volatile uint32_t *>(sm + kBaseAt);
     const int lw = P.lw, RF = P.rf;
     const int par = (D->par + q) & 1, step = D->step + 2 * q;
     const CUtensorMap *maps = static_cast<const CUtensorMap *>(P.tma);
     const int nx = D->nx, ny = D->ny, nz = D->nz;
-    const float cx = D->cx, cy = D->cy, cz = D->cz;
+    const Scalars sc{D->cx, D->cy, D->cz, P.one, -P.one};
     const long long src = D->src;
     const float w1 = src >= 0 && step < D->nwave ? __ldg(D->wave + step) : 0.f;
     const float w2 = src >= 0 && step + 1 < D->nwave ? __ldg(D->wave + step + 1) : 0.f;
@@ -290,20 +322,23 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         k1 = min(k0 + P.kc, nz);
         kstart = max(k0 - 2, 0);
     };
-    // Copies of plane k of the frame at (px, py) into ring slot s, by one warp.
-    auto issue = [&](int px, int py, int k, int s) {
-        if (lane == 0) mbar_expect_tx(&bars[s], (uint32_t)(CELLS ? P.tx_bytes - P.mw * P.rf : P.tx_bytes));
+    // Copies of plane k of the frame at (px, py) into the ring slot at byte c, by one warp.
+    auto issue = [&](int px, int py, int k, int c) {
+        if (lane == 0) mbar_expect_tx(bar_at(sm, c + kFull), (uint32_t)(CELLS ? P.tx_bytes - P.mw * P.rf : P.tx_bytes));
         __syncwarp();
         if (lane < (CELLS ? 6 : 7))
-            tma_load_3d(sm + s * kStage + lane * kField, lane < 6 ? maps + par * 6 + lane : maps + 12,
-                        lane < 6 ? px : px & ~15, py, k, &bars[s]);
+            tma_load_3d(sm + c + lane * kField, lane < 6 ? maps + par * 6 + lane : maps + 12,
+                        lane < 6 ? px : px & ~15, py, k, bar_at(sm, c + kFull));
     };
     if (lane < (CELLS ? 6 : 7)) tma_acquire(lane < 6 ? maps + par * 6 + lane : maps + 12);
+    // Everything above is constant over a chunk; the fields are the launch's before this one.
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (t < P.tiles) {
         int xt, yt, k0, k1, kstart;
         tile_at(t, xt, yt, k0, k1, kstart);
         if (warp == 0)   // a tile has more planes than the ring
-            for (int s = 0; s < S; ++s) issue(xt * (4 * lw - 4), yt * (RF - 3), kstart + s, s);
+            for (int s = 0; s < S; ++s) issue(xt * (4 * lw - 4), yt * (RF - 3), kstart + s, s * kStage);
     }
 
     // this thread's unit of the frame; threads beyond it repeat the last one without storing
@@ -313,14 +348,14 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     // Pairs from the next warp and the one before; lanes that need none read a pair nobody uses.
     const int e_own = 8 * warp + 8, e_hi = edge_hi ? e_own + 8 : 0, e_lo = edge_lo ? e_own - 8 : 0;
     const int o_hi = edge_hi ? o + 16 : 0;   // in a ring stage: the float beyond the unit
-    // The ring: slot of the current plane, and the parity of its barrier's next phase; a plane computed
-    // per phase of bar1 and bar2.  The warps take turns at refilling the ring.
+    // The ring: byte of the current plane's slot, and the parity of its barrier's next phase; a plane computed
+    // per phase of the barriers 1 and 2.  The warps take turns at refilling the ring.
     int cs = 0, turn = 0;
     unsigned cph = 0, n = 0;
     const int nwarps = blockDim.x / 32;
     bool failed = false;
-    auto wait = [&](uint64_t *bar, unsigned phase) {
-        if (!mbar_done(bar, phase & 1) && !failed && !mbar_wait(bar, phase & 1)) {
+    auto wait = [&](int bar, unsigned phase) {
+        if (!mbar_done(base + bar, phase & 1) && !failed && !mbar_wait(bar_at(sm, bar), phase & 1)) {
             failed = true;
             atomicOr(err, 1);
         }
@@ -336,8 +371,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         const bool row_out = tid < lw * RF && j < ny && r <= RF - 2 && (yt == 0 || r >= 2);
         const int left = nx - i;
         const bool upper = xt > 0 && lx == 0, lower = xt + 1 < P.nxt && lx == lw - 1;
-        const bool full = row_out && !upper && !lower && left >= 4, half = row_out && (upper || lower) && left >= 4;
-        const bool few = row_out && left > 0 && left < 4;
+        const bool full = row_out && !upper && !lower && left >= 4, part = row_out && left > 0 && !full;
         unsigned off = (unsigned)i + pitch * (unsigned)j + plane * (unsigned)kstart;   // of plane k
         // the source's plane and cell in this unit
         int src_k = -1, src_c = 0;
@@ -347,27 +381,34 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         }
         const int mo = 6 * kField + r * P.mw + (xs & 15) + 4 * lx;
 
-        F3 H1a{}, H1b{}, E1a{}, E1b{}, H2a{}, H2b{};
         // PAIR_CELLS: Cb of the node, loaded a plane ahead; units beyond the rows repeat one within
         const float *const cbp = CELLS ? D->coef[1] + (min((unsigned)i, pitch - 4) + pitch * (unsigned)min(j, ny)) : nullptr;
-        auto cb_at = [&](int k) { return __ldg(reinterpret_cast<const float4 *>(cbp + plane * (unsigned)min(k, nz))); };
+        auto cb_at = [&](int k) {   // volatile: stays where it is written, a plane before its use
+            float4 v;
+            asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "l"(cbp + plane * (unsigned)min(k, nz)));
+            return v;
+        };
         float4 cb_n{};
         if constexpr (CELLS) cb_n = cb_at(kstart);
-        float4 cb_m{}, cb_mm{};            // Ca = Da = 1: Cb of planes k-1, k-2
-        unsigned id_m = 0, id_mm = 0;      // otherwise their material ids
 
-        // E2(kk) from H2(kk) (own, and the rows of buffer b), H2(kk-1); H2 and E2 stored.
-        auto seg_c = [&](int kk, unsigned offc, unsigned ph, F3 &E1, const F3 &H2, const F3 &H2m, const float4 &cb, unsigned ids) {
-            const unsigned b = ph & 1;
-            const char *rd = sm + od + b * kRowBuf;
+        F3 H1a{}, H1b{}, E1a{}, E1b{}, H2a{}, H2b{};
+        float4 cba{}, cbb{};               // Ca = Da = 1: Cb of two planes
+        unsigned ida = 0, idb = 0;         // otherwise their material ids
+
+        // E2(kk) from H2(kk) (own, and the rows of buffer B), H2(kk-1); H2 and E2 stored.
+        auto seg_c = [&](auto buffer, int kk, unsigned offc, unsigned ph, F3 &E1, const F3 &H2, const F3 &H2m, const float4 &cb, unsigned ids) {
+            constexpr int B = decltype(buffer)::value, rows = kRowsAt + B * kRowBuf;
+            const char *rd = sm + od;
             float hyp = __shfl_up_sync(0xffffffffu, H2.y.w, 1), hzp = __shfl_up_sync(0xffffffffu, H2.z.w, 1);
-            wait(bar2, ph);
-            const float2 e = lds2(sm + kEdgesAt + X_H2 * kEdge, e_lo + b * kEdgeBuf);
+            wait(kBar2, ph);
+            const float2 e = lds2(sm + e_lo, kEdgesAt + B * kEdgeBuf + X_H2 * kEdge);
             if (edge_lo) { hyp = e.x; hzp = e.y; }
-            const float4 hxj = lds4(rd, kRowsAt + R_HX2 * kField), hzj = lds4(rd, kRowsAt + R_HZ2 * kField);
+            const float4 hxj = lds4(rd, rows + R_HX2 * kField), hzj = lds4(rd, rows + R_HZ2 * kField);
             float4 Dc = make_float4(1.f, 1.f, 1.f, 1.f), Cc = cb;
             if constexpr (MODE == PAIR_TABLE) lookup<MODE>(tab, ids, 0, Dc, Cc);
-            e_update<D1>(E1, Dc, Cc, H2, H2m.x, H2m.y, hxj, hzj, hyp, hzp, in, kk >= 1, cx, cy, cz);
+            e_update<D1>(E1, Dc, Cc, H2, H2m.x, H2m.y, hxj, hzj, hyp, hzp, in, kk >= 1, sc);
             if (kk == src_k) add_source(E1.z, src_c, w2);
             if (full) {
                 *reinterpret_cast<float4 *>(oHx + offc) = H2.x;
@@ -376,43 +417,48 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 *reinterpret_cast<float4 *>(oEx + offc) = E1.x;
                 *reinterpret_cast<float4 *>(oEy + offc) = E1.y;
                 *reinterpret_cast<float4 *>(oEz + offc) = E1.z;
-            }
-            if (half) {
-                auto put = [&](float *p, const float4 &v) {
-                    *reinterpret_cast<float2 *>(p + offc + (upper ? 2 : 0)) = upper ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
-                };
-                put(oHx, H2.x); put(oHy, H2.y); put(oHz, H2.z);
-                put(oEx, E1.x); put(oEy, E1.y); put(oEz, E1.z);
-            }
-            if (few) {
-                auto put = [&](float *p, const float4 &v) {
-                    if (!upper) p[offc] = v.x;
-                    if (!upper && left > 1) p[offc + 1] = v.y;
-                    if (!lower && left > 2) p[offc + 2] = v.z;
-                };
-                put(oHx, H2.x); put(oHy, H2.y); put(oHz, H2.z);
-                put(oEx, E1.x); put(oEy, E1.y); put(oEz, E1.z);
+            } else if (part) {
+                if (left >= 4) {
+                    auto put = [&](float *p, const float4 &v) {
+                        *reinterpret_cast<float2 *>(p + offc + (upper ? 2 : 0)) = upper ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+                    };
+                    put(oHx, H2.x); put(oHy, H2.y); put(oHz, H2.z);
+                    put(oEx, E1.x); put(oEy, E1.y); put(oEz, E1.z);
+                } else {
+                    auto put = [&](float *p, const float4 &v) {
+                        if (!upper) p[offc] = v.x;
+                        if (!upper && left > 1) p[offc + 1] = v.y;
+                        if (!lower && left > 2) p[offc + 2] = v.z;
+                    };
+                    put(oHx, H2.x); put(oHy, H2.y); put(oHz, H2.z);
+                    put(oEx, E1.x); put(oEy, E1.y); put(oEz, E1.z);
+                }
             }
         };
 
-        // One plane.  On entry E1 holds E1(k-2), E1m E1(k-1), H1m H1(k-1), H2p H2(k-2), H2 H2(k-3); on
-        // exit H1, E1, H2 hold H1(k), E1(k), H2(k-1).  The caller swaps the names.
-        auto plane_step = [&](int k, F3 &H1, const F3 &H1m, F3 &E1, const F3 &E1m, F3 &H2, const F3 &H2p) {
-            const unsigned b = n & 1;
-            const int ns = cs + 1 == S ? 0 : cs + 1;
-            const unsigned nph = cs + 1 == S ? cph ^ 1 : cph;
-            char *const rw = sm + ot + b * kRowBuf;   // own slot of the rows written on this plane
-            char *const ew = sm + b * kEdgeBuf;
-            if (k == kstart) wait(&bars[cs], cph);
-            const char *cur = sm + cs * kStage, *co = cur + o, *no = sm + ns * kStage + o;
+        // One plane, in buffer B of the rows and pairs (alternating within a tile: what the last plane of a
+        // tile leaves in its buffer has been read when the next tile's first plane writes there).  On entry E1
+        // holds E1(k-2), E1m E1(k-1), H1m H1(k-1), H2p H2(k-2), H2 H2(k-3), cb and id plane k-2's; on exit H1,
+        // E1, H2 hold H1(k), E1(k), H2(k-1), cb and id plane k's.  The caller swaps the names.
+        auto plane_step = [&](auto buffer, int k, F3 &H1, const F3 &H1m, F3 &E1, const F3 &E1m, F3 &H2, const F3 &H2p, float4 &cb,
+                              unsigned &id, unsigned id_m) {
+            constexpr int B = decltype(buffer)::value, rows = kRowsAt + B * kRowBuf, rows_m = kRowsAt + (B ^ 1) * kRowBuf;
+            constexpr int pairs = kEdgesAt + B * kEdgeBuf, pairs_m = kEdgesAt + (B ^ 1) * kEdgeBuf;
+            const int ns = cs == (S - 1) * kStage ? 0 : cs + kStage;
+            const unsigned nph = cs == (S - 1) * kStage ? cph ^ 1 : cph;
+            char *const rw = sm + ot;   // own slot of the rows
+            if (k == kstart) wait(cs + kFull, cph);
+            const char *cur = sm + cs, *co = cur + o, *no = sm + ns + o;
             // ---- H1(k) ----
             F3 e0;
             e0.x = lds4(co, 3 * kField);
             e0.y = lds4(co, 4 * kField);
             e0.z = lds4(co, 5 * kField);
             unsigned ids = 0;
+            [[maybe_unused]] const float4 cb_k = cb_n;
+            if constexpr (CELLS) cb_n = cb_at(k + 1);
             if constexpr (!CELLS) ids = *reinterpret_cast<const unsigned *>(cur + mo);
-            float4 Dh = make_float4(1.f, 1.f, 1.f, 1.f), Ch = make_float4(dbu, dbu, dbu, dbu), Dc, Cc;
+            float4 Dh = make_float4(1.f, 1.f, 1.f, 1.f), Ch = make_float4(dbu, dbu, dbu, dbu);
             {
                 const char *cj = co + rs, *ch = cur + o_hi;
                 const float4 exj = lds4(cj, 3 * kField), ezj = lds4(cj, 5 * kField);
@@ -420,30 +466,28 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 H1.y = lds4(co, kField);
                 H1.z = lds4(co, 2 * kField);
                 const float eyl = lds1(ch, 4 * kField), ezl = lds1(ch, 5 * kField);
-                if constexpr (CELLS) {
-                    Cc = cb_n;
-                    cb_n = cb_at(k + 1);
-                } else {
-                    lookup<MODE>(tab, ids, 0, Dc, Cc);
-                }
-                wait(&bars[ns], nph);
+                wait(ns + kFull, nph);
                 const float4 exk = lds4(no, 3 * kField), eyk = lds4(no, 4 * kField);
                 float ezn = __shfl_down_sync(0xffffffffu, e0.z.x, 1), eyn = __shfl_down_sync(0xffffffffu, e0.y.x, 1);
                 if (edge_hi) { eyn = eyl; ezn = ezl; }
                 if constexpr (MODE == PAIR_TABLE) lookup<MODE>(tab, ids, 1, Dh, Ch);
-                h_update<D1>(H1, Dh, Ch, e0, exk, eyk, exj, ezj, eyn, ezn, cx, cy, cz);
+                h_update<D1>(H1, Dh, Ch, e0, exk, eyk, exj, ezj, eyn, ezn, sc);
             }
-            sts4(rw, kRowsAt + R_HX1 * kField, H1.x);
-            sts4(rw, kRowsAt + R_HZ1 * kField, H1.z);
-            if (edge_hi) *reinterpret_cast<float2 *>(ew + kEdgesAt + X_H1 * kEdge + e_own) = make_float2(H1.y.w, H1.z.w);
+            sts4(rw, rows + R_HX1 * kField, H1.x);
+            sts4(rw, rows + R_HZ1 * kField, H1.z);
+            if (edge_hi) *reinterpret_cast<float2 *>(sm + e_own + pairs + X_H1 * kEdge) = make_float2(H1.y.w, H1.z.w);
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar1);
+            if (lane == 0) mbar_arrive(base + kBar1);
             // ---- E2(k-2) ----
-            if (k - 2 >= k0) seg_c(k - 2, off - 2 * plane, n - 1, E1, H2p, H2, cb_mm, id_mm);
+            if (k - 2 >= k0) seg_c(std::integral_constant<int, (B ^ 1)>(), k - 2, off - 2 * plane, n - 1, E1, H2p, H2, cb, id);
             // ---- E1(k) ----
+            float4 Dc = make_float4(1.f, 1.f, 1.f, 1.f);
+            id = ids;
+            if constexpr (CELLS) cb = cb_k;
+            else lookup<MODE>(tab, ids, 0, Dc, cb);
             float hyp = __shfl_up_sync(0xffffffffu, H1.y.w, 1), hzp = __shfl_up_sync(0xffffffffu, H1.z.w, 1);
             float ezn = __shfl_down_sync(0xffffffffu, E1m.z.x, 1), eyn = __shfl_down_sync(0xffffffffu, E1m.y.x, 1);
-            wait(bar1, n);
+            wait(kBar1, n);
             // Every warp has read plane k's slot (and, on the tile's last plane, k + 1's): refill it with the
             // plane S on, of this tile or the next.
             if (warp == turn) {
@@ -457,55 +501,56 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 }
             }
             turn = turn + 1 == nwarps ? 0 : turn + 1;
-            const char *rd = sm + od + b * kRowBuf, *rj = sm + ot + rs + (b ^ 1) * kRowBuf;
-            const float2 eh = lds2(ew + kEdgesAt + X_H1 * kEdge, e_lo), ee = lds2(sm + kEdgesAt + X_E1 * kEdge, e_hi + (b ^ 1) * kEdgeBuf);
-            const float4 hxj = lds4(rd, kRowsAt + R_HX1 * kField), hzj = lds4(rd, kRowsAt + R_HZ1 * kField);
-            const float4 exj = lds4(rj, kRowsAt + R_EX1 * kField), ezj = lds4(rj, kRowsAt + R_EZ1 * kField);   // for H2 below
+            const char *rd = sm + od, *rj = sm + ot + rs;
+            const float2 eh = lds2(sm + e_lo, pairs + X_H1 * kEdge), ee = lds2(sm + e_hi, pairs_m + X_E1 * kEdge);
+            const float4 hxj = lds4(rd, rows + R_HX1 * kField), hzj = lds4(rd, rows + R_HZ1 * kField);
+            const float4 exj = lds4(rj, rows_m + R_EX1 * kField), ezj = lds4(rj, rows_m + R_EZ1 * kField);   // for H2 below
             if (edge_lo) { hyp = eh.x; hzp = eh.y; }
             if (edge_hi) { eyn = ee.x; ezn = ee.y; }
             E1 = e0;
-            e_update<D1>(E1, Dc, Cc, H1, H1m.x, H1m.y, hxj, hzj, hyp, hzp, in, k >= 1 && k < nz, cx, cy, cz);
+            e_update<D1>(E1, Dc, cb, H1, H1m.x, H1m.y, hxj, hzj, hyp, hzp, in, k >= 1 && k < nz, sc);
             if (k == src_k) add_source(E1.z, src_c, w1);
-            sts4(rw, kRowsAt + R_EX1 * kField, E1.x);
-            sts4(rw, kRowsAt + R_EZ1 * kField, E1.z);
-            if (lane == 0) *reinterpret_cast<float2 *>(ew + kEdgesAt + X_E1 * kEdge + e_own) = make_float2(E1.y.x, E1.z.x);
+            sts4(rw, rows + R_EX1 * kField, E1.x);
+            sts4(rw, rows + R_EZ1 * kField, E1.z);
+            if (lane == 0) *reinterpret_cast<float2 *>(sm + e_own + pairs + X_E1 * kEdge) = make_float2(E1.y.x, E1.z.x);
             // ---- H2(k-1) ----
             if (k > kstart) {
                 if constexpr (MODE == PAIR_TABLE) lookup<MODE>(tab, id_m, 1, Dh, Ch);
                 H2 = H1m;
-                h_update<D1>(H2, Dh, Ch, E1m, E1.x, E1.y, exj, ezj, eyn, ezn, cx, cy, cz);
-                sts4(rw, kRowsAt + R_HX2 * kField, H2.x);
-                sts4(rw, kRowsAt + R_HZ2 * kField, H2.z);
-                if (edge_hi) *reinterpret_cast<float2 *>(ew + kEdgesAt + X_H2 * kEdge + e_own) = make_float2(H2.y.w, H2.z.w);
+                h_update<D1>(H2, Dh, Ch, E1m, E1.x, E1.y, exj, ezj, eyn, ezn, sc);
+                sts4(rw, rows + R_HX2 * kField, H2.x);
+                sts4(rw, rows + R_HZ2 * kField, H2.z);
+                if (edge_hi) *reinterpret_cast<float2 *>(sm + e_own + pairs + X_H2 * kEdge) = make_float2(H2.y.w, H2.z.w);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar2);
-            cb_mm = cb_m;
-            cb_m = Cc;
-            id_mm = id_m;
-            id_m = ids;
+            if (lane == 0) mbar_arrive(base + kBar2);
             off += plane;
             ++n;
             cs = ns;
             cph = nph;
         };
 
+        constexpr std::integral_constant<int, 0> even{};
+        constexpr std::integral_constant<int, 1> uneven{};
         int k = kstart;
         for (; k + 1 <= k1; k += 2) {
-            plane_step(k, H1a, H1b, E1a, E1b, H2a, H2b);
-            plane_step(k + 1, H1b, H1a, E1b, E1a, H2b, H2a);
+            plane_step(even, k, H1a, H1b, E1a, E1b, H2a, H2b, cba, ida, idb);
+            plane_step(uneven, k + 1, H1b, H1a, E1b, E1a, H2b, H2a, cbb, idb, ida);
         }
-        const bool odd = k == k1;
-        if (odd) plane_step(k, H1a, H1b, E1a, E1b, H2a, H2b);
-        if (odd) seg_c(k1 - 1, off - 2 * plane, n - 1, E1b, H2a, H2b, cb_mm, id_mm);
-        else seg_c(k1 - 1, off - 2 * plane, n - 1, E1a, H2b, H2a, cb_mm, id_mm);
+        if (k == k1) {
+            plane_step(even, k, H1a, H1b, E1a, E1b, H2a, H2b, cba, ida, idb);
+            seg_c(even, k1 - 1, off - 2 * plane, n - 1, E1b, H2a, H2b, cbb, idb);
+        } else {
+            seg_c(uneven, k1 - 1, off - 2 * plane, n - 1, E1a, H2b, H2a, cba, ida);
+        }
         // past the tile's last plane, which was read as "next" only
-        if (++cs == S) { cs = 0; cph ^= 1; }
+        cs += kStage;
+        if (cs == S * kStage) { cs = 0; cph ^= 1; }
     }
     // Every issued plane has normally been waited for.  If a wait expired, let the copies still in
     // flight land (bounded) before this CTA's shared memory is released.
     if (tid == 0)
-        for (int s = 0; s < S; ++s) mbar_wait(&bars[s], s < cs ? cph : cph ^ 1);
+        for (int s = 0; s < S; ++s) mbar_wait(bar_at(sm, s * kStage + kFull), s * kStage < cs ? cph : cph ^ 1);
 }
 
 namespace {
@@ -517,54 +562,64 @@ bool lay_out(PairPlan &p)
     a.mw = (4 * a.lw + 12 + 15) / 16 * 16;
     a.tx_bytes = 16 * a.lw * (6 * a.rf + 2) + a.mw * a.rf;   // Ex, Ez: one row more
     p.smem = kPairBytes;
+    a.one = 1.0f;
     return a.mw * a.rf <= kIds;
 }
 
 }  // namespace
 
-// The frame of `nxt` tiles in x: as many rows as a CTA's threads allow.  False when no such frame exists.
-static bool pair_frame(int nx, int ny, int nxt, PairArgs *a)
+// The frame of nxt tiles in x and at least `nyt` in y, with no more rows than that needs.  False when no such
+// frame exists; a->nyt may come out larger, where the threads do not allow the rows.
+static bool pair_frame(int nx, int ny, int nxt, int nyt, int threads, PairArgs *a)
 {
     a->nxt = nxt;
     a->lw = (nx + 1 + 4 * (nxt - 1) + 4 * nxt - 1) / (4 * nxt);
     if (a->lw > kMaxLw || (a->lw < 8 && nxt > 1)) return false;
-    a->rf = std::min(std::min(kPairThreads / a->lw, 255), ny + 1);
-    if (a->rf < 5) return false;
-    a->nyt = ny <= a->rf - 1 ? 1 : 1 + (ny - (a->rf - 1) + a->rf - 4) / (a->rf - 3);
-    return true;
+    const int most = std::min(std::min(threads / a->lw, 255), ny + 1);
+    if (most < 5) return false;
+    const int least = ny <= most - 1 ? 1 : 1 + (ny - (most - 1) + most - 4) / (most - 3);   // tiles with all those rows
+    a->nyt = std::max(nyt, least);
+    a->rf = std::min(most, std::max(5, (ny + 1 + 3 * (a->nyt - 1) + a->nyt - 1) / a->nyt));
+    return a->nyt == 1 || (a->nyt - 1) * (a->rf - 3) < ny - 2;   // the last tile has rows of its own
 }
 
 static bool pair_fits(int nx, int ny, int nz) { return make_layout(nx, ny, nz).total * 4 < 1LL << 32 && nz >= 8; }
 
 // The tile shape with the least estimated time for two steps: rounds of resident CTAs times the planes each
-// streams (its depth, the planes recomputed at its start, the ring's turn at its end).
+// streams (its depth, the planes recomputed at its start, the ring's turn at its end) times a plane's time, which
+// grows with the frame's warps (320 threads of 384: 0.89 of the time)
+// and is 7-14 % longer with rows of 9 to 11 units than of 13 and more.
 bool plan_pair(int nx, int ny, int nz, PairPlan *out)
 {
     const int sms = sm_count();
     double best = 1e30;
     bool found = false;
     if (sms <= 0 || !pair_fits(nx, ny, nz)) return false;
-    for (int nxt = 1; nxt <= 64; ++nxt) {
-        PairPlan p{};
-        if (!pair_frame(nx, ny, nxt, &p.args)) continue;
-        for (int nzt = 1; nzt <= nz / 8; ++nzt) {
-            const int kc = (nz + nzt - 1) / nzt;
-            if ((nz + kc - 1) / kc != nzt) continue;
-            const long long tiles = (long long)nxt * p.args.nyt * nzt, waves = (tiles + sms - 1) / sms;
-            const double cost = (double)waves * (kc + 3.5);
-            p.args.nzt = nzt; p.args.kc = kc; p.args.tiles = (int)tiles;
+    for (int nxt = 1; nxt <= 64; ++nxt)
+        for (int more = 0, nyt = 1; more < 6; ++more, ++nyt) {   // the fewest rows of tiles, and a few more of lower ones
+            PairPlan p{};
+            if (!pair_frame(nx, ny, nxt, nyt, kPairThreads, &p.args)) break;
+            nyt = p.args.nyt;
             p.threads = (p.args.lw * p.args.rf + 31) / 32 * 32;
-            p.grid = (int)std::min<long long>(tiles, sms);
-            const double c = cost * (0.35 + 0.65 * p.threads / kPairThreads);
-            if (c < best && lay_out(p)) {
-                best = c;
-                *out = p;
-                found = true;
+            const double plane = (0.35 + 0.65 * p.threads / kPairThreads) * (1 + 8.0 / (p.args.lw * p.args.lw));
+            for (int nzt = 1; nzt <= nz / 8; ++nzt) {
+                const int kc = (nz + nzt - 1) / nzt;
+                if ((nz + kc - 1) / kc != nzt) continue;
+                const long long tiles = (long long)nxt * nyt * nzt, waves = (tiles + sms - 1) / sms;
+                p.args.nzt = nzt; p.args.kc = kc; p.args.tiles = (int)tiles;
+                p.grid = (int)std::min<long long>(tiles, sms);
+                const double c = (double)waves * (kc + 3.5) * plane;
+                if (c < best && lay_out(p)) {
+                    best = c;
+                    *out = p;
+                    found = true;
+                }
             }
         }
-    }
     return found;
 }
+
+constexpr int kBatchThreads = kPairThreads;
 
 // In a batch every CTA has all its threads, so the frame is the one with the fewest tiles per plane.  It does
 // not depend on the rest of the batch; the depth does (plan_pair_depths).
@@ -574,10 +629,8 @@ bool plan_pair_member(int nx, int ny, int nz, PairPlan *out)
     if (!pair_fits(nx, ny, nz)) return false;
     for (int nxt = 1; nxt <= 64; ++nxt) {
         PairPlan p{};
-        if (!pair_frame(nx, ny, nxt, &p.args)) continue;
-        const int nyt = p.args.nyt;
-        p.args.rf = std::max(5, std::min(p.args.rf, (ny + 1 + 3 * (nyt - 1) + nyt - 1) / nyt));   // no more rows than these tiles need
-        if (lay_out(p) && (!found || nxt * nyt < out->args.nxt * out->args.nyt)) {
+        if (!pair_frame(nx, ny, nxt, 1, kBatchThreads, &p.args)) continue;
+        if (lay_out(p) && (!found || nxt * p.args.nyt < out->args.nxt * out->args.nyt)) {
             *out = p;
             found = true;
         }
@@ -651,8 +704,17 @@ static int launch_pair(const InstDesc *d_inst, const PairArgs &one, const PairAr
                        int pair, int *err, cudaStream_t s)
 {
     PTK_CUDA_TRY(cudaFuncSetAttribute(k_yee_pair<MODE, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairBytes));
-    k_yee_pair<MODE, MANY><<<grid, threads, kPairBytes, s>>>(d_inst, one, many, tile0, ninst, pair, err);
-    PTK_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = kPairBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = pair > 0 ? 1 : 0;
+    PTK_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_yee_pair<MODE, MANY>, d_inst, one, many, tile0, ninst, pair, err));
     count_launches(1);
     return PTK_OK;
 }
@@ -667,7 +729,7 @@ int launch_yee_pair(const InstDesc *d_inst, const PairPlan &p, int mode, int pai
 int launch_yee_pair_batch(const InstDesc *d_insts, const PairArgs *d_args, const int *d_tile0, int ninst, int tiles, int pair, int *err,
                           cudaStream_t s)
 {
-    return launch_pair<PAIR_SIMPLE, true>(d_insts, PairArgs{}, d_args, d_tile0, ninst, tiles, kPairThreads, pair, err, s);
+    return launch_pair<PAIR_SIMPLE, true>(d_insts, PairArgs{}, d_args, d_tile0, ninst, tiles, kBatchThreads, pair, err, s);
 }
 
 }  // namespace ptk

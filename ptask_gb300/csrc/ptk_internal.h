@@ -209,6 +209,7 @@ struct PairArgs {
     int lw, rf, mw;                 // units per row and rows of a frame; bytes of a row of material ids
     int tx_bytes;                   // bytes in flight of a ring stage
     const void *tma;                // 13 tensor maps: Hx..Ez of both buffers, ids
+    float one;                      // 1.0f
     float *buf[2][6];               // the fields' two buffers
 };
 struct PairPlan {
