@@ -14,6 +14,7 @@
 //                    layout); the hot kernel.  Bandwidth bound: 64 algorithmic bytes per cell.
 //   k_field_ref      the reference's per-field task kernels (dense layout), one field per launch.
 //   k_rows           reference layout <-> padded layout.
+#include "fdtd_chain.cuh"
 #include "fdtd_device.cuh"
 
 #include <cstdio>
@@ -579,8 +580,8 @@ int launch_fill(float *dst, long long n, float v, cudaStream_t s)
 // takes 32 nodes of a row through kTaskPlanes planes with all their loads in flight, and a z neighbour
 // is the next plane's own value.  Fields that would give fewer than two blocks per SM that way take a
 // plane per warp.  Rows start anywhere, so accesses are single floats.  Per launch, against a thread
-// per node in blocks of 128 along x: 64x64x4 1.19 us (1.44), 45x64x50 1.67 (2.70), 200x150x100 8.5
-// (17.0), 256^3 47 (85).
+// per node in blocks of 128 along x, in a captured chain: 64x64x4 0.92 us (1.44), 45x64x50 1.35 (2.70),
+// 200x150x100 8.3 (17.0), 256^3 47 (85); called one by one at 200x150x100 8.6 (19.6).
 // ---------------------------------------------------------------------------------------------
 constexpr int kTaskRows = 8, kTaskPlanes = 4;
 
@@ -608,10 +609,10 @@ __global__ void __launch_bounds__(32 * kTaskRows) k_field_ref(const FieldTask T)
     const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kTaskRows + threadIdx.y, k0 = blockIdx.z * PL;
     if (i >= T.ex || j >= T.ey) return;
     const int n = min(PL, T.ez - k0);
-    const float *__restrict__ a = T.a + i + (long long)T.ex * j + T.aplane * k0;
-    const float *__restrict__ p = T.p + i + (long long)T.prow * j + T.pplane * k0;
-    const float *__restrict__ q = T.q + i + (long long)T.qrow * j + T.qplane * k0;
-    float *__restrict__ out = T.out + i + (long long)T.ex * j + T.aplane * k0;
+    const float *a = T.a + i + (long long)T.ex * j + T.aplane * k0;
+    const float *p = T.p + i + (long long)T.prow * j + T.pplane * k0;
+    const float *q = T.q + i + (long long)T.qrow * j + T.qplane * k0;
+    float *out = T.out + i + (long long)T.ex * j + T.aplane * k0;
     constexpr int way = E ? -1 : 1;
     const long long dp = way * (DP == 0 ? 1LL : DP == 1 ? (long long)T.prow : T.pplane);
     const long long dq = way * (DQ == 0 ? 1LL : DQ == 1 ? (long long)T.qrow : T.qplane);
@@ -619,6 +620,7 @@ __global__ void __launch_bounds__(32 * kTaskRows) k_field_ref(const FieldTask T)
     const bool in = !E || (((DP != 0 && DQ != 0) || (i >= 1 && i <= T.nx - 1)) && ((DP != 1 && DQ != 1) || (j >= 1 && j <= T.ny - 1)));
     float av[PL], pn[PL], pf[PL], qn[PL], qf[PL];
     bool on[PL];
+    chain_wait();
 #pragma unroll
     for (int u = 0; u < PL; ++u) {
         const bool z = !E || (DP != 2 && DQ != 2) || (k0 + u >= 1 && k0 + u <= T.nz - 1);
@@ -653,17 +655,11 @@ void field_extents(int f, int nx, int ny, int nz, int *ex, int *ey, int *ez)
 }
 
 template <int PL>
-static void field_task(int field, const FieldTask &t, cudaStream_t s)
+static cudaError_t field_task(int field, const FieldTask &t, cudaStream_t s)
 {
-    const dim3 grid = task_grid(t.ex, t.ey, t.ez, PL), block(32, kTaskRows);
-    switch (field) {
-    case PTK_HX: k_field_ref<false, 2, 1, PL><<<grid, block, 0, s>>>(t); break;
-    case PTK_HY: k_field_ref<false, 0, 2, PL><<<grid, block, 0, s>>>(t); break;
-    case PTK_HZ: k_field_ref<false, 1, 0, PL><<<grid, block, 0, s>>>(t); break;
-    case PTK_EX: k_field_ref<true, 1, 2, PL><<<grid, block, 0, s>>>(t); break;
-    case PTK_EY: k_field_ref<true, 2, 0, PL><<<grid, block, 0, s>>>(t); break;
-    default: k_field_ref<true, 0, 1, PL><<<grid, block, 0, s>>>(t); break;
-    }
+    void (*const k[6])(const FieldTask) = {k_field_ref<false, 2, 1, PL>, k_field_ref<false, 0, 2, PL>, k_field_ref<false, 1, 0, PL>,
+                                           k_field_ref<true, 1, 2, PL>,  k_field_ref<true, 2, 0, PL>,  k_field_ref<true, 0, 1, PL>};
+    return launch_chained(k[field], task_grid(t.ex, t.ey, t.ez, PL), dim3(32, kTaskRows), 0, s, true, t);
 }
 
 int launch_field_ref(int field, const float *in0, const float *in1, const float *in2,
@@ -688,9 +684,8 @@ int launch_field_ref(int field, const float *in0, const float *in1, const float 
     t.c = field < 3 ? p.Dt / p.mu0 : p.Dt / p.eps0;
     t.s1 = sc[dp[field]]; t.s2 = sc[dq[field]];
     const dim3 grid = task_grid(t.ex, t.ey, t.ez, kTaskPlanes);
-    if ((long long)grid.x * grid.y * grid.z >= 2 * std::max(1, sm_count())) field_task<kTaskPlanes>(field, t, s);
-    else field_task<1>(field, t, s);
-    PTK_CUDA_TRY(cudaGetLastError());
+    const bool large = (long long)grid.x * grid.y * grid.z >= 2 * std::max(1, sm_count());
+    PTK_CUDA_TRY(large ? field_task<kTaskPlanes>(field, t, s) : field_task<1>(field, t, s));
     count_launches(1);
     return PTK_OK;
 }

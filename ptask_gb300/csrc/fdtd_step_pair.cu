@@ -38,6 +38,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include "fdtd_chain.cuh"
 #include "fdtd_device.cuh"
 #include "fdtd_tma.cuh"
 
@@ -332,8 +333,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     };
     if (lane < (CELLS ? 6 : 7)) tma_acquire(lane < 6 ? maps + par * 6 + lane : maps + 12);
     // Everything above is constant over a chunk; the fields are the launch's before this one.
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    chain_wait();
     if (t < P.tiles) {
         int xt, yt, k0, k1, kstart;
         tile_at(t, xt, yt, k0, k1, kstart);
@@ -704,17 +704,8 @@ static int launch_pair(const InstDesc *d_inst, const PairArgs &one, const PairAr
                        int pair, int *err, cudaStream_t s)
 {
     PTK_CUDA_TRY(cudaFuncSetAttribute(k_yee_pair<MODE, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairBytes));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = kPairBytes;
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = pair > 0 ? 1 : 0;
-    PTK_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_yee_pair<MODE, MANY>, d_inst, one, many, tile0, ninst, pair, err));
+    PTK_CUDA_TRY(launch_chained(k_yee_pair<MODE, MANY>, dim3(grid), dim3(threads), kPairBytes, s, pair > 0, d_inst, one, many, tile0, ninst,
+                                pair, err));
     count_launches(1);
     return PTK_OK;
 }

@@ -6,6 +6,7 @@
 // node and on E; a new E value only on the old E value of the same node and on H.  The cyclic graph
 // therefore circulates one datablock per field through in-out ports, with no allocation per step
 // (the reference allocates a new output block per task dispatch, OutputPort.cpp:536).
+#include "fdtd_chain.cuh"
 #include "ptk_internal.h"
 
 namespace ptk {
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(32 * kRows) k_h_step(const HalfStep T)
     const long long oHx = i + (long long)(nx + 1) * j + pHx * k0, oHy = i + (long long)nx * j + pHy * k0, oHz = i + (long long)nx * j + pHz * k0;
     const long long oEx = oHy, oEy = oHx, oEz = i + (long long)(nx + 1) * j + pEz * k0;
     const float *Hx = T.h[0], *Hy = T.h[1], *Hz = T.h[2], *Ex = T.e[0], *Ey = T.e[1], *Ez = T.e[2];
+    chain_wait();
     float hx[kPlanes], hy[kPlanes], hz[kPlanes], ex[kPlanes + 1], ey[kPlanes + 1], ez[kPlanes];
     float exj[kPlanes], ezj[kPlanes], eyi[kPlanes], ezi[kPlanes], d[kPlanes], c[kPlanes];
 #pragma unroll
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(32 * kRows) k_e_step(const HalfStep T)
     const long long oHx = i + (long long)(nx + 1) * j + pHx * k0, oHy = i + (long long)nx * j + pHy * k0, oHz = i + (long long)nx * j + pHz * k0;
     const long long oEx = oHy, oEy = oHx, oEz = i + (long long)(nx + 1) * j + pEz * k0;
     const float *Hx = T.h[0], *Hy = T.h[1], *Hz = T.h[2], *Ex = T.e[0], *Ey = T.e[1], *Ez = T.e[2];
+    chain_wait();
     float ex[kPlanes], ey[kPlanes], ez[kPlanes], hx[kPlanes + 1], hy[kPlanes + 1], hz[kPlanes];   // hx[u]: plane k0 + u - 1
     float hxj[kPlanes], hzj[kPlanes], hyi[kPlanes], hzi[kPlanes], d[kPlanes], c[kPlanes];
 #pragma unroll
@@ -189,8 +192,7 @@ int launch_h_half(const float *const in[6], float *const out[3], const ptk_fdtd_
 {
     HalfStep t = half_step(in, in + 3, out, p);
     t.cs = p.Dt / p.mu0;
-    k_h_step<false><<<half_grid(t), dim3(32, kRows), 0, s>>>(t);
-    PTK_CUDA_TRY(cudaGetLastError());
+    PTK_CUDA_TRY(launch_chained(k_h_step<false>, half_grid(t), dim3(32, kRows), 0, s, true, t));
     count_launches(1);
     return PTK_OK;
 }
@@ -200,8 +202,7 @@ int launch_e_half(const float *const e_in[3], const float *const h_new[3], float
 {
     HalfStep t = half_step(h_new, e_in, out, p);
     t.cs = p.Dt / p.eps0;
-    k_e_step<false><<<half_grid(t), dim3(32, kRows), 0, s>>>(t);
-    PTK_CUDA_TRY(cudaGetLastError());
+    PTK_CUDA_TRY(launch_chained(k_e_step<false>, half_grid(t), dim3(32, kRows), 0, s, true, t));
     count_launches(1);
     return PTK_OK;
 }
@@ -224,8 +225,7 @@ int ptk_launch_h_step_coef(float *const h[3], const float *const e[3], const flo
     HalfStep t = half_step(h, e, h, *p);
     t.d = Da;
     t.c = Db;
-    k_h_step<true><<<half_grid(t), dim3(32, kRows), 0, S(stream)>>>(t);
-    PTK_CUDA_TRY(cudaGetLastError());
+    PTK_CUDA_TRY(launch_chained(k_h_step<true>, half_grid(t), dim3(32, kRows), 0, S(stream), true, t));
     count_launches(1);
     return PTK_OK;
 }
@@ -251,8 +251,7 @@ int ptk_launch_e_step_coef(float *const e[3], const float *const h[3], const flo
     t.wave = wave;
     t.nwave = nwave;
     t.counter = src >= 0 ? step_counter : nullptr;
-    k_e_step<true><<<half_grid(t), dim3(32, kRows), 0, S(stream)>>>(t);
-    PTK_CUDA_TRY(cudaGetLastError());
+    PTK_CUDA_TRY(launch_chained(k_e_step<true>, half_grid(t), dim3(32, kRows), 0, S(stream), true, t));
     count_launches(1);
     return PTK_OK;
 }

@@ -42,9 +42,8 @@ def test_scalar_tasks(shape, halves):
         b.free()
 
 
-@pytest.mark.parametrize("shape", SHAPES)
-def test_coefficient_tasks_in_place(shape):
-    steps = 4
+@pytest.mark.parametrize("shape,steps", [(n, 4) for n in SHAPES] + [((97, 41, 70), 60)])   # the last: a long chain of launches
+def test_coefficient_tasks_in_place(shape, steps):
     pr = P.Problem.generate(*shape, n_boxes=2, eps=(1, 9), box=(1, 20), steps=3, source_mode=2, seed=6)
     rng = np.random.default_rng(7)
     for c in (pr.Ca, pr.Cb, pr.Da, pr.Db):
