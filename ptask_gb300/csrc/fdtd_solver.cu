@@ -58,11 +58,11 @@ static void default_tiles(int nx, int ny, int nz, int *by, int *kc, int *vec)
     *kc = k;
 }
 
-// Grids of this many cells or more start with the staged kernel's shape, whose longer runs are one
-// resident launch or take two steps per pass (32^3: 1.8 us per step against 5.5; 256^3: 87 against 215).
-// Smaller ones keep the register kernel and a launch per step, which callers count
+// Grids of more than this many cells start with the staged kernel's shape, whose longer runs are one
+// resident launch or take two steps per pass (24^3: 1.6 us per step against 12.8; 32^3: 1.6 against 5.5; 256^3:
+// 87 against 215).  Smaller ones keep the register kernel and a launch per step, which callers count
 // (ptk_solver_last_launches).
-static constexpr long long kStagedCells = 1 << 14;
+static constexpr long long kStagedCells = 1 << 12;
 
 // Uniform coefficients v = (Ca, Cb, Da, Db), and the one-entry table that goes with them.
 __global__ void k_uniform_coefs(float *Ca, float *Cb, float *Da, float *Db, long long n, float4 v, float4 *tab)
@@ -484,7 +484,7 @@ try {
                          cudaMemcpyAsync(s->d_face0, f0, sizeof f0, cudaMemcpyHostToDevice, st) != cudaSuccess))
         rc = set_error(PTK_ERR_CUDA, "solver initialisation failed");
     if (rc == PTK_OK) rc = uniform_vacuum(s, st, /*clear_index=*/false);
-    if (rc == PTK_OK && (long long)p->Nx * p->Ny * p->Nz >= kStagedCells) {
+    if (rc == PTK_OK && (long long)p->Nx * p->Ny * p->Nz > kStagedCells) {
         ptk_tile_config c;
         rc = staged_default(p->Nx, p->Ny, p->Nz, &c);
         s->by = c.by; s->kc = c.kc; s->vec = c.vec; s->stages = c.stages;
