@@ -10,8 +10,9 @@ Courant 0.5, Gaussian Ez source, 1000 steps).  Prints one JSON line (rank 0):
   value  Mcell-updates/s with the inputs already resident in HBM (device events around the solves)
   e2e    the same metric through the public C-ABI path with pinned host buffers, the H2D upload of the
          inputs and the D2H download of the six result fields inside the timed region
-  roofline  the fused step kernel against measured HBM bandwidth: 49 algorithmic bytes per cell update
-         with the material index (six fields read and written, one id byte), 64 with per-cell arrays
+  roofline  the step kernel against measured HBM bandwidth: 49 algorithmic bytes per cell and pass over memory
+         with the material index (six fields read and written, one id byte), 64 with per-cell arrays; the
+         two-step kernel makes two updates per pass
   cpu_baseline  the CPU oracle (our FP32 port of the reference's fdtd_cpu, OpenMP over all host cores)
                 timed on a bounded sample of the same workload
   served the workload's batched/served half: the 64-instance batched set, a Poisson trace at the
@@ -162,10 +163,20 @@ def hbm_peak():
     return FALLBACK_HBM_GBS, "fallback"
 
 
+def kernel_of(solver, steps: int):
+    """(name, time steps per pass over memory) of the kernel that took the solver's last run of `steps`."""
+    launches = solver.last_launches()
+    if launches == 1 and steps > 1:
+        return "k_yee_resident", steps
+    if launches < 3 * steps // 4:
+        return "k_yee_pair", 2
+    return ("k_yee_step_bulk" if solver.kernel()[0] else "k_yee_step"), 1
+
+
 def traffic_per_cell(kernel: str, mat: bool = False, rows: int = 0):
-    """DRAM bytes per cell update of the given fused step kernel from its committed ncu summary (the
+    """DRAM bytes per cell update of the given step kernel from its committed ncu summary (the
     64-wide 23-row tiles have their own; other staged shapes use the 11-row figure)."""
-    name = {("k_yee_step_bulk", True): "yee_step_bulk_mat_256.md", ("k_yee_step_bulk", False): "yee_step_bulk_256.md"}
+    name = {("k_yee_pair", True): "yee_pair_256.md", ("k_yee_step_bulk", True): "yee_step_bulk_mat_256.md", ("k_yee_step_bulk", False): "yee_step_bulk_256.md"}
     if kernel == "k_yee_step_bulk" and mat and rows == 23:
         name[(kernel, mat)] = "yee_step_bulk_mat23_256.md"
     f = ROOT / "profiles" / name.get((kernel, mat), "yee_step_256.md")
@@ -402,13 +413,13 @@ def run_ours(args, wl, world, rank, local):
     total_cell_updates = cells * T * args.steps * world
     value = total_cell_updates / (dev_ms / 1e3) / 1e6
     e2e_value = total_cell_updates / e2e_s / 1e6
-    per_launch_ms = statistics.median(run_ms) / T
+    per_step_ms = statistics.median(run_ms) / T
     peak, peak_src = hbm_peak()
     run_stages, mat = solver.kernel()
-    bpc = BYTES_PER_CELL_MAT if mat else BYTES_PER_CELL
-    achieved = bpc * cells / (per_launch_ms / 1e3) / 1e9
+    kernel, per_pass = kernel_of(solver, T)
+    bpc = (BYTES_PER_CELL_MAT if mat else BYTES_PER_CELL) / per_pass
+    achieved = bpc * cells / (per_step_ms / 1e3) / 1e9
     by, kc, vec, stages = solver.tiles()
-    kernel = "k_yee_step_bulk" if run_stages else "k_yee_step"
     tpc = traffic_per_cell(kernel, mat, by)
     line = {
         "metric": "FDTD Mcell-updates/s", "value": value, "unit": "Mcell-updates/s", "n_gpus": world,
@@ -424,12 +435,12 @@ def run_ours(args, wl, world, rank, local):
                                     "four per-cell FP32 arrays")},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_src,
-                     "traffic": (tpc * cells) if tpc else None,
-                     "kernel": kernel + " (fused H+E step)",
-                     "algorithmic_bytes_per_launch": bpc * cells,
-                     "algorithmic_bytes_per_cell": bpc,
-                     "frac_of_64B_cell_traffic": BYTES_PER_CELL * cells / (per_launch_ms / 1e3) / 1e9 / peak,
-                     "launch_ms": per_launch_ms},
+                     "traffic": (tpc * cells * per_pass) if tpc else None,
+                     "kernel": f"{kernel} ({per_pass} time step{'s' if per_pass > 1 else ''} per pass)",
+                     "algorithmic_bytes_per_launch": bpc * cells * per_pass,
+                     "algorithmic_bytes_per_cell_update": bpc,
+                     "frac_of_64B_cell_traffic": BYTES_PER_CELL * cells / (per_step_ms / 1e3) / 1e9 / peak,
+                     "launch_ms": per_step_ms * per_pass},
         "e2e_graph": graph_e2e,
         "e2e": {"value": e2e_value, "unit": "Mcell-updates/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": e2e_s * 1e3 / args.steps, "result_ok": result_ok,
@@ -462,7 +473,7 @@ def serve_arms(reqs, scale: float, rows: int, *, cb_runs: int = 1, cb_warmup: in
 
     Arms, all on the same seeded requests and arrival times:
       continuous      ptk_server: requests admitted as they arrive and fit the HBM budget, every active
-                      instance advanced by one persistent step launch per time step
+                      instance advanced by one launch per two time steps
       plain_fused     the same server with one slot (max_active = 1): our best single-instance path
       plain_graph_fused     one PTask FDTD graph per request shape, one request at a time: push the
                       coefficients and fields, Graph::Run of the cyclic graph lowered to the fused loop,
@@ -493,7 +504,7 @@ def serve_arms(reqs, scale: float, rows: int, *, cb_runs: int = 1, cb_warmup: in
         a = {"solves_per_s": len(reqs) / wall, "mcell_updates_per_s": cells / wall / 1e6, "wall_s": wall,
              "p50_latency_s": p50, "p99_latency_s": p99}
         if chunk_dev:
-            a["frac_of_peak_over_device_time"] = BYTES_PER_CELL_MAT * cells / chunk_dev / 1e9 / peak
+            a["frac_of_peak_over_device_time"] = BYTES_PER_CELL_MAT / 2 * cells / chunk_dev / 1e9 / peak
         return a
 
     for _ in range(cb_warmup):
@@ -516,8 +527,8 @@ def serve_arms(reqs, scale: float, rows: int, *, cb_runs: int = 1, cb_warmup: in
            "plain_fused": arm_of(plain["wall_s"], plain["p50_latency_s"], plain["p99_latency_s"],
                                  plain["chunk_device_s"]),
            "gpu_launches": int(best["launches"]), "clocks": clk,
-           "roofline_basis": "49 algorithmic bytes per cell update (material index) over the device time of the "
-                             "replayed chunks (every step launch, faces, advances) of the whole request set; "
+           "roofline_basis": "24.5 algorithmic bytes per cell update (material index, two steps per pass) over the device time "
+                             "of the replayed chunks (every step launch, faces, advances) of the whole request set; "
                              f"peak {peak:.1f} GB/s ({peak_src})"}
     for mode in graph_arms:
         g = graph_dispatch(reqs, scale, mode=mode)
@@ -528,7 +539,7 @@ def serve_arms(reqs, scale: float, rows: int, *, cb_runs: int = 1, cb_warmup: in
 
 
 def batched_desc():
-    return ("batched FDTD: 64 instances in one persistent fused launch per step, edges per axis uniform in "
+    return ("batched FDTD: 64 instances advanced together in fused launches, edges per axis uniform in "
             "[32,192], steps uniform in [100,2000], 1-8 dielectric boxes, seeded sources, FP32")
 
 
@@ -539,10 +550,10 @@ def served_desc(n, rate):
             "cube edge log-uniform in [24,256], steps uniform in [50,1000], FP32, admission by HBM budget")
 
 
-# Staged tile shape per workload, as measured on GB300 (same box, two runs each): the batched mix
-# (x extents 32-192) serves 66.6 solves/s on 23-row, 64-wide tiles (twelve warps, one CTA per SM)
-# against 64.1 on 7-row and 60.2 on 11-row tiles; the served mix (cubes up to 256) 76.3 on the
-# server's default 11-row, 128-wide tiles against 69.2 on 23-row and 67.3 on 7-row tiles.
+# Tile shape of single steps per workload (a chunk's odd step; the rest go two per pass), as measured when all
+# steps were single ones: the batched mix (x extents 32-192) served 66.6 solves/s on 23-row, 64-wide tiles against
+# 64.1 on 7-row and 60.2 on 11-row tiles; the served mix (cubes up to 256) 76.3 on the server's default 11-row,
+# 128-wide tiles against 69.2 on 23-row and 67.3 on 7-row tiles.
 def default_rows(kind: str) -> int:
     return 23 if kind == "batched" else 0
 
@@ -550,7 +561,7 @@ def default_rows(kind: str) -> int:
 def large_subrecord(local: int, solves: int = 3) -> dict:
     """The large workload (512x512x384, 32 boxes, 500 steps) solved from resident zero fields with the
     autotuned tiles: Mcell-updates/s over `solves` complete solves (CUDA events) and the step kernel
-    against the measured HBM bandwidth at 49 (material index) or 64 bytes per cell update."""
+    against the measured HBM bandwidth at 49 (material index) or 64 bytes per cell and pass."""
     import ptask_gb300 as P
     from ptask_gb300.device import DeviceBuffer, Event
     wl = WORKLOADS["large"]
@@ -582,17 +593,18 @@ def large_subrecord(local: int, solves: int = 3) -> dict:
         clk = clocks.stop()
         ms = e0.elapsed_ms(e1) / solves
         stages, mat = s.kernel()
+        kernel, per_pass = kernel_of(s, T)
     for b in dev:
         b.free()
     peak, peak_src = hbm_peak()
-    bpc = BYTES_PER_CELL_MAT if mat else BYTES_PER_CELL
+    bpc = (BYTES_PER_CELL_MAT if mat else BYTES_PER_CELL) / per_pass
     achieved = bpc * cells * T / (ms / 1e3) / 1e9
     return {"workload": wl["desc"], "grid": list(shape), "time_steps": T, "solves": solves,
             "mcell_updates_per_s": cells * T / (ms / 1e3) / 1e6, "ms_per_solve": ms,
             "tiles": {"rows": tiles[0], "z_depth": tiles[1], "cells_per_thread": tiles[2], "staged_planes": stages,
                       "material_index": mat},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "peak_source": peak_src, "algorithmic_bytes_per_cell": bpc,
+                         "peak_source": peak_src, "algorithmic_bytes_per_cell_update": bpc, "kernel": kernel,
                          "basis": "whole solves (step launches, faces, advances) over CUDA-event time"},
             "clocks": clk}
 

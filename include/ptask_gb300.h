@@ -210,8 +210,10 @@ int ptk_solver_set_tiles(ptk_solver *s, const ptk_tile_config *cfg);
 int ptk_solver_use_material_index(ptk_solver *s, int enable, void *stream);
 /* Materials in the current index (0: none, the per-cell arrays are read). */
 int ptk_solver_material_count(const ptk_solver *s, int *nmat);
-/* The step kernel the next run uses: ring stages (0 = register kernel) and whether it reads the
- * material index.  A staged shape with no per-cell-array instantiation falls back to 4 stages. */
+/* The kernel of single steps: ring stages (0 = register kernel) and whether it reads the material
+ * index.  A staged shape with no per-cell-array instantiation falls back to 4 stages.  With a staged
+ * shape, runs of 8 steps or more on grids that fit on chip are one launch, and runs of 16 or more on
+ * larger ones take two steps per launch (ptk_solver_last_launches tells). */
 int ptk_solver_kernel(const ptk_solver *s, int *stages, int *material_index);
 int ptk_solver_get_tiles(const ptk_solver *s, ptk_tile_config *cfg);
 /* Advance `steps` time steps, asynchronously on `stream`. */
@@ -267,7 +269,8 @@ typedef struct ptk_server_config {
     size_t hbm_budget_bytes;   /* device bytes the admitted instances may hold (0: 80% of free HBM) */
     int max_active;            /* instance slots (0: unlimited; 1: plain one-at-a-time dispatch) */
     int chunk_steps;           /* steps per replayed graph between admission points (0: 32) */
-    int tile_rows;             /* fused-kernel tile rows 4, 8 or 16, or 7, 10, 11 or 23 with the
+    int tile_rows;             /* tile rows of single steps (a chunk's odd one; the staged forms take the
+                                  rest two per launch): 4, 8 or 16, or 7, 10, 11 or 23 with the
                                   staged kernel (7- and 23-row tiles are 64 cells wide, the others
                                   128; 0: 11 for the staged kernel, 8 for the register kernel) */
     int keep_results;          /* keep finished fields for ptk_server_fetch */

@@ -173,7 +173,7 @@ class Solver:
         return n.value
 
     def kernel(self) -> tuple[int, bool]:
-        """(ring stages of the next run's step kernel, 0 = register kernel; reads the material index)"""
+        """(ring stages of the kernel of single steps, 0 = register kernel; reads the material index)"""
         st, m = C.c_int(), C.c_int()
         call("ptk_solver_kernel", self._h, C.byref(st), C.byref(m))
         return st.value, bool(m.value)
