@@ -550,7 +550,7 @@ def served_desc(n, rate):
             "cube edge log-uniform in [24,256], steps uniform in [50,1000], FP32, admission by HBM budget")
 
 
-# Tile shape of single steps per workload (a chunk's odd step; the rest go two per pass), as measured when all
+# Tile shape of single steps per workload (one per instance at most; the rest go two per pass), as measured when all
 # steps were single ones: the batched mix (x extents 32-192) served 66.6 solves/s on 23-row, 64-wide tiles against
 # 64.1 on 7-row and 60.2 on 11-row tiles; the served mix (cubes up to 256) 76.3 on the server's default 11-row,
 # 128-wide tiles against 69.2 on 23-row and 67.3 on 7-row tiles.

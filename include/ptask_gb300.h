@@ -269,8 +269,8 @@ typedef struct ptk_server_config {
     size_t hbm_budget_bytes;   /* device bytes the admitted instances may hold (0: 80% of free HBM) */
     int max_active;            /* instance slots (0: unlimited; 1: plain one-at-a-time dispatch) */
     int chunk_steps;           /* steps per replayed graph between admission points (0: 32) */
-    int tile_rows;             /* tile rows of single steps (a chunk's odd one; the staged forms take the
-                                  rest two per launch): 4, 8 or 16, or 7, 10, 11 or 23 with the
+    int tile_rows;             /* tile rows of single steps (one of an instance with an odd number; the
+                                  staged forms take the rest two per launch): 4, 8 or 16, or 7, 10, 11 or 23 with the
                                   staged kernel (7- and 23-row tiles are 64 cells wide, the others
                                   128; 0: 11 for the staged kernel, 8 for the register kernel) */
     int keep_results;          /* keep finished fields for ptk_server_fetch */

@@ -2,17 +2,17 @@
 // together by the fused step kernel, with continuous admission by HBM budget.
 //
 // Two time steps of every active instance are ONE launch of the two-step kernel (k_yee_pair, a CTA per
-// tile of the instances' tile lists); a chunk's odd step, and the steps of a batch that holds an instance
-// too thin for it (fewer than 8 planes or 4 rows), are launches of the TMA-staged one-step kernel
-// (k_yee_step_bulk) over the same instances, or of the register kernel k_yee_step on request.  Both take
-// the coefficients from a material index.  Chunks of steps are replayed as captured CUDA graphs (at most
-// kMaxGraphs kept).  Device time of a mix, two steps per pass against one: 64 requests of 32..192 540 ms
-// against 1050, 64 x 32^3 4.0 against 18.0, one 256^3 28 against 40, one 16^3 2.5 against 4.2.
+// tile of the instances' tile lists).  An instance with an odd number of steps takes one of them by the
+// TMA-staged one-step kernel (k_yee_step_bulk) when it joins; a batch that holds an instance too thin for
+// pairs (fewer than 8 planes or 4 rows) takes all its steps by it, or by the register kernel on request.
+// Both take the coefficients from a material index.  Chunks of steps are replayed as captured CUDA graphs
+// (at most kMaxGraphs kept).  Device time of a mix, two steps per pass against one: 64 requests of 32..192
+// 528 ms against 1050, 64 x 32^3 3.4 against 18.0, one 256^3 23 against 40, one 24^3 2.0 against 4.4.
 //
 // Instances finish at their own step counts, with a chunk that ends there, and leave the batch at its
-// end, where newly arrived requests are admitted if they fit the HBM budget.  Request problems are generated on the device (coefficients and the
-// material index from the seeded box list), so admission moves only the waveform and the tensor
-// maps over the host link.
+// end, where newly arrived requests are admitted if they fit the HBM budget.  Request problems are
+// generated on the device (coefficients and the material index from the seeded box list), so admission
+// moves only the waveform and the tensor maps over the host link.
 //
 // The host keeps one chunk queued ahead: while chunk i runs it admits, rebuilds the work list into
 // the other half of a double-buffered pinned staging area and launches chunk i+1, with chunk i's
@@ -210,7 +210,9 @@ struct ptk_server {
     PairArgs *h_pair[2] = {};
     int *d_pair0 = nullptr;
     int *h_pair0[2] = {};
-    int pair_tiles = 0;             // 0: an instance of the batch has no frame, single steps
+    int pair_tiles = 0;             // 0: single steps (an instance of the batch has no frame, or chunks of one step)
+    int odd = 0, odd_tiles = 0;     // first instances of the list: an odd number of steps left; their one-step tiles
+    long long odd_faces = 0;        // and face nodes
     int cap = 0;
     int total_tiles = 0;
     int vec = 4;                    // x cells per thread of the current work list
@@ -236,7 +238,7 @@ struct ptk_server {
     } flight[2];
     bool dirty = true;
     bool admit_blocked = false;     // the pool could not place a request: wait for retirements
-    std::map<std::tuple<int, int, int, int, int, long long>, cudaGraphExec_t> graphs;
+    std::map<std::tuple<int, int, int, int, int, long long, int, int, long long>, cudaGraphExec_t> graphs;
     long long chunks = 0, launches = 0, captures = 0, admit_waits = 0;
     double wall_s = 0, cell_updates = 0;
     double chunk_dev_s = 0, admit_s = 0, retire_s = 0, sched_s = 0;   // where wall_s went
@@ -500,7 +502,7 @@ int rebuild_worklist(ptk_server *s)
     // small grids but hold fewer bytes in flight per thread, and measured slower on the batched
     // workload.  The staged kernel's width goes with its rows (set at creation).
     if (!s->stages) s->vec = 4;
-    bool pair = s->stages > 0;
+    bool pair = s->stages > 0 && s->cfg.chunk_steps >= 2;
     for (const Inst *in : s->active) pair = pair && in->pair;
     if (pair) {
         std::vector<PairPlan *> plans;
@@ -513,15 +515,19 @@ int rebuild_worklist(ptk_server *s)
     }
     if (s->stages) {
         s->depth_cap = choose_depth_cap(s);
-        // longest tiles first, so that the dynamic tile queue ends with short ones
+        // longest tiles first, so that the dynamic tile queue ends with short ones; pairs: the instances whose
+        // steps are odd in number before the others
         std::stable_sort(s->active.begin(), s->active.end(), [s, pair](const Inst *a, const Inst *b) {
-            if (pair) return a->plan.args.kc > b->plan.args.kc;
+            const int oa = (a->steps_total - a->done) & 1, ob = (b->steps_total - b->done) & 1;
+            if (pair) return oa != ob ? oa > ob : a->plan.args.kc > b->plan.args.kc;
             const int da = instance_depth(s, a->L.nz), db = instance_depth(s, b->L.nz);
             return (da ? da : a->L.nz) > (db ? db : b->L.nz);
         });
     }
     int tiles = 0, pair_tiles = 0;
     long long faces = 0;
+    s->odd = s->odd_tiles = 0;
+    s->odd_faces = 0;
     for (int q = 0; q < n; ++q) {
         const InstDesc d = instance_desc(s, s->active[q]);
         h_desc[q] = d;
@@ -533,6 +539,11 @@ int rebuild_worklist(ptk_server *s)
             s->h_pair[s->par][q] = s->active[q]->plan.args;
             s->h_pair0[s->par][q] = pair_tiles;
             pair_tiles += s->active[q]->plan.args.tiles;
+            if (d.steps_left & 1) {
+                s->odd = q + 1;
+                s->odd_tiles = tiles;
+                s->odd_faces = faces;
+            }
         }
     }
     s->h_pair0[s->par][n] = s->pair_tiles = pair_tiles;
@@ -558,11 +569,16 @@ constexpr size_t kMaxGraphs = 256;   // chunk graphs kept for reuse
 
 int chunk_pairs(const ptk_server *s, int len) { return s->pair_tiles ? len / 2 : 0; }
 
+// Steps of one graph: pairs, for which every instance has an even number left once those with an odd one (the
+// first `odd` of the list) have taken a single step ahead of the others; or single steps of all.  An odd step of
+// the whole batch costs nearly what a pair does (1.56 ms against 1.66 on the served trace), and every instance that
+// finishes on an odd count would ask for one.
 int chunk_graph(ptk_server *s, int len, int grid, cudaGraphExec_t *out)
 {
     const int n = (int)s->active.size();
-    const int pairs = chunk_pairs(s, len), flips = len - pairs;
-    auto key = std::make_tuple(len, n, s->total_tiles, s->pair_tiles, (grid * 8 + s->vec) * 8 + s->stages, s->total_faces);
+    const int pairs = chunk_pairs(s, len), odd = s->pair_tiles ? s->odd : 0;
+    auto key = std::make_tuple(len, n, s->total_tiles, s->pair_tiles, (grid * 8 + s->vec) * 8 + s->stages, s->total_faces, odd,
+                               odd ? s->odd_tiles : 0, odd ? s->odd_faces : 0LL);
     auto it = s->graphs.find(key);
     if (it != s->graphs.end()) {
         *out = it->second;
@@ -573,18 +589,29 @@ int chunk_graph(ptk_server *s, int len, int grid, cudaGraphExec_t *out)
     PTK_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
     set_capturing(true);
     int rc = PTK_OK;
-    if (s->stages && cudaMemsetAsync(s->d_work, 0, sizeof(int) * len, cap) != cudaSuccess)
-        rc = set_error(PTK_ERR_CUDA, "chunk capture: counter reset failed");
-    else if (s->stages)
-        count_launches(1);
-    if (!rc && s->stages) rc = launch_yee_faces_steps(s->d_desc, s->d_face0, n, s->total_faces, 0, len, cap, flips);
+    const int singles = s->pair_tiles ? (odd ? 1 : 0) : len;
+    if (s->stages && singles > 0) {
+        if (cudaMemsetAsync(s->d_work, 0, sizeof(int) * singles, cap) != cudaSuccess)
+            rc = set_error(PTK_ERR_CUDA, "chunk capture: counter reset failed");
+        else
+            count_launches(1);
+    }
+    if (!rc && odd) {
+        rc = launch_yee_faces_steps(s->d_desc, s->d_face0, odd, s->odd_faces, 0, 1, cap);
+        if (!rc)
+            rc = launch_yee_step_bulk(s->d_desc, s->d_tile0, odd, s->odd_tiles, 0, s->rows, s->stages, std::min(grid, s->odd_tiles),
+                                      s->d_err, cap, s->d_work, true);
+        if (!rc) rc = launch_advance(s->d_desc, odd, 1, cap);
+    }
+    if (!rc && s->stages && len > 0)
+        rc = launch_yee_faces_steps(s->d_desc, s->d_face0, n, s->total_faces, 0, len, cap, s->pair_tiles ? pairs : len);
     for (int q = 0; q < pairs && !rc; ++q)
         rc = launch_yee_pair_batch(s->d_desc, s->d_pair, s->d_pair0, n, s->pair_tiles, q, s->d_err, cap);
-    for (int q = 2 * pairs; q < len && !rc; ++q)
+    for (int q = 0; q < len && !rc && !s->pair_tiles; ++q)
         rc = s->stages ? launch_yee_step_bulk(s->d_desc, s->d_tile0, n, s->total_tiles, q, s->rows, s->stages, grid,
-                                              s->d_err, cap, s->d_work, true, false, q - pairs)
+                                              s->d_err, cap, s->d_work, true)
                        : launch_yee_step_v(s->d_desc, s->d_tile0, n, s->total_tiles, q, s->rows, s->vec, grid, cap);
-    if (!rc) rc = launch_advance(s->d_desc, n, len, cap, flips);
+    if (!rc && len > 0) rc = launch_advance(s->d_desc, n, len, cap, s->pair_tiles ? pairs : len);
     set_capturing(false);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(cap, &g);
@@ -860,10 +887,12 @@ try {
         const double ts = now_s();
         if (s->dirty) rc = rebuild_worklist(s);
         if (rc) break;
+        // chunk length: the configured chunk, shortened so that the first finisher leaves promptly; with pairs an
+        // even number, which may be none, after the single step of the instances with an odd number left
         int left_min = 1 << 30;
-        for (Inst *in : s->active) left_min = std::min(left_min, in->steps_total - in->done);
-        // chunk length: the configured chunk, shortened so that the first finisher leaves promptly
-        const int len = std::max(1, std::min(s->cfg.chunk_steps, left_min));
+        const int whole = s->pair_tiles ? ~1 : ~0;
+        for (Inst *in : s->active) left_min = std::min(left_min, (in->steps_total - in->done) & whole);
+        const int len = std::min(s->cfg.chunk_steps & whole, left_min);
         const int grid = s->cfg.persistent ? std::min(grid_cap[s->vec], s->total_tiles) : 0;
         cudaGraphExec_t ex;
         rc = chunk_graph(s, len, grid, &ex);
@@ -877,7 +906,8 @@ try {
         }
         s->flight[b].exec = ex;
         // kernels in the chunk graph: the steps, the step-counter advance and (staged) the faces
-        const int flips = len - chunk_pairs(s, len), kernels = flips + 1 + (s->stages && s->total_faces > 0 ? 1 : 0);
+        const int flips = len - chunk_pairs(s, len), odd = s->pair_tiles ? s->odd : 0;
+        const int kernels = (len > 0 ? flips + 1 + (s->stages && s->total_faces > 0 ? 1 : 0) : 0) + (odd ? 2 + (s->odd_faces > 0 ? 1 : 0) : 0);
         count_graph_launch(kernels);
         s->launches += kernels;
         ++s->chunks;
@@ -889,6 +919,11 @@ try {
         // This chunk's finishers: checksums (and results) and frees queued behind it.
         const double tr = now_s();
         std::vector<Inst *> still, gone;
+        for (int q = 0; q < odd; ++q) {   // the single step; the list's order holds until it is built again
+            ++s->active[q]->done;
+            s->active[q]->par ^= 1;
+        }
+        s->odd = 0;
         for (Inst *in : s->active) {
             in->done += len;   // no chunk is longer than the shortest remainder
             in->par = (in->par + flips) & 1;

@@ -223,3 +223,21 @@ def test_two_steps_per_pass_in_a_batch(shapes, chunk):
                                       pr.Db, pr.src, pr.wave)
             for q in range(6):
                 np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{r} {P.FIELDS[q]}")
+
+
+def test_single_steps_of_odd_counts():
+    """One step in all, odd and even counts that join at once, a thin request that switches the batch to single steps and back."""
+    shapes = [((20, 16, 12), 1), ((20, 16, 12), 2), ((33, 20, 9), 31), ((18, 3, 12), 7), ((24, 24, 24), 64), ((30, 12, 16), 33), ((16, 20, 40), 1)]
+    reqs = [Request(*n, steps, 2, 80 + q, box=(1, 6)) for q, (n, steps) in enumerate(shapes)]
+    for chunk, slots in ((32, 0), (6, 2), (5, 3), (2, 1)):
+        with Server(keep_results=True, chunk_steps=chunk, max_active=slots) as s:
+            tickets = [s.submit(r) for r in reqs]
+            s.run(time_scale=0)
+            for t, r in zip(tickets, reqs):
+                got = s.fetch(t)
+                pr = P.Problem.generate(r.nx, r.ny, r.nz, n_boxes=r.n_boxes, eps=r.eps, box=r.box, steps=r.steps,
+                                        source_mode=r.source_mode, seed=r.seed)
+                ref = oracle.step_ext_f32(P.zero_fields(r.nx, r.ny, r.nz), r.steps, pr.params, pr.Ca, pr.Cb, pr.Da,
+                                          pr.Db, pr.src, pr.wave)
+                for q in range(6):
+                    np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{r} chunk {chunk} {P.FIELDS[q]}")
