@@ -1,9 +1,10 @@
-// fdtd_solver.cu -- device-resident FDTD instance with CUDA-graph replay of the fused step.
+// fdtd_solver.cu -- device-resident FDTD instance: runs on chip, or CUDA-graph replay of the fused step.
 //
 // A solver owns, in HBM: two buffers of each of the six fields (ping-pong), the four coefficient
-// arrays, the source waveform and a one-entry work list (InstDesc + tile prefix).  A run of T steps
-// replays a captured graph of L fused-step launches followed by one "advance" launch that moves the
-// instance's step counter, so the only host work per L steps is one cudaGraphLaunch.  This is the
+// arrays, the source waveform and a one-entry work list (InstDesc + tile prefix).  A run of T steps is
+// one launch where the grid fits on chip (run_resident).  Otherwise it replays a captured graph of
+// launches, of two steps each or of one, followed by one "advance" launch that moves the
+// instance's step counter, so the only host work per graph is one cudaGraphLaunch.  This is the
 // scheduler's execution of an iterated FDTD cycle: the per-task dispatch of the reference
 // (ptask/task.cpp:3822-3900 -> ptask/cutask.cpp:634-705, six launches per step with host-side
 // readiness checks) becomes one replayed graph.
@@ -348,6 +349,10 @@ static constexpr int kPairSteps = 16;
 
 static int run_resident(ptk_solver *s, int steps, cudaStream_t st)
 {
+    // As the replayed graphs of the other runs: not part of a capture.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    PTK_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return set_error(PTK_ERR_CUDA, "a run is not permitted when the stream is capturing");
     ResidentArgs a{};
     for (int f = 0; f < 6; ++f) a.in[f] = a.out[f] = s->buf[s->par][f];   // in place (two steps or more)
     for (int c = 0; c < 4; ++c) a.coef[c] = s->coef[c];

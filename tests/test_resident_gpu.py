@@ -142,3 +142,43 @@ def test_static_solve_runs_resident_where_its_scratch_fits(shape, vacuum):
             np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{shape} {P.FIELDS[q]}")
     for b in bufs + coefs + ([wave] if wave else []):
         b.free()
+
+
+def test_under_capture():
+    """An allocation-free solve is captured and replayed; a solver's run is refused, on chip as by replayed graphs."""
+    import ctypes as C
+
+    from ptask_gb300 import _lib
+    from ptask_gb300.device import DeviceBuffer, Stream
+    V = C.c_void_p
+    shape, steps = (30, 20, 24), 20
+    p = P.reference_params(*shape)
+    f = P.random_fields(*shape, seed=1, scale=1e-2)
+    st = Stream()
+
+    def solve(bufs):
+        _lib.call("ptk_fdtd_solve_static", C.byref(p), (V * 6)(*[b.ptr for b in bufs]), *[None] * 4, -1, -1, -1, None, 0, steps,
+                  st.handle)
+
+    first, second = ([DeviceBuffer.from_array(a) for a in f] for _ in range(2))
+    solve(first)
+    st.sync()
+    graph = V()
+    _lib.call("ptk_capture_begin", st.handle)
+    solve(second)
+    _lib.call("ptk_capture_end", st.handle, C.byref(graph))
+    _lib.call("ptk_graph_exec_launch", graph, st.handle, 1)
+    st.sync()
+    for q in range(6):
+        np.testing.assert_array_equal(second[q].download(P.field_shape(q, *shape)), first[q].download(P.field_shape(q, *shape)))
+    with P.Solver(p) as s:
+        s.set_fields(f)
+        s.run(steps, st.handle)
+        st.sync()
+        before = s.get_fields()
+        _lib.call("ptk_capture_begin", st.handle)
+        with pytest.raises(_lib.PtkError):
+            s.run(steps, st.handle)
+        _lib.call("ptk_capture_end", st.handle, C.byref(graph))
+        for a, b in zip(s.get_fields(), before):
+            np.testing.assert_array_equal(a, b)
