@@ -274,7 +274,7 @@ typedef struct ptk_server_config {
                                   staged kernel (7- and 23-row tiles are 64 cells wide, the others
                                   128; 0: 11 for the staged kernel, 8 for the register kernel) */
     int keep_results;          /* keep finished fields for ptk_server_fetch */
-    int persistent;            /* persistent grid of resident CTAs instead of one CTA per tile */
+    int persistent;            /* single steps: persistent grid of resident CTAs instead of one CTA per tile */
     int stages;                /* step kernel: 0 = TMA-staged with its default ring (3 planes for 4 rows,
                                   else 4; 16 rows become 8), 2..6 = TMA-staged with that many planes where
                                   the rows have that shape, -1 = register kernel */

@@ -11,7 +11,7 @@
 //
 // Kernels here:
 //   k_yee_step<BY>   fused H+E step over a work list of tiles of one or many instances (padded
-//                    layout); the hot kernel.  Bandwidth bound: 64 algorithmic bytes per cell.
+//                    layout), operands in registers.  Bandwidth bound: 64 algorithmic bytes per cell.
 //   k_field_ref      the reference's per-field task kernels (dense layout), one field per launch.
 //   k_rows           reference layout <-> padded layout.
 #include "fdtd_chain.cuh"
