@@ -218,7 +218,8 @@ int ptk_solver_kernel(const ptk_solver *s, int *stages, int *material_index);
 int ptk_solver_get_tiles(const ptk_solver *s, ptk_tile_config *cfg);
 /* Advance `steps` time steps, asynchronously on `stream`. */
 int ptk_solver_run(ptk_solver *s, int steps, void *stream);
-/* Read the six fields back (reference layout). */
+/* Read the six fields back (reference layout).  If a bounded wait of a run has run out, they are invalid:
+ * PTK_HOST, which waits for them, returns PTK_ERR_TIMEOUT; PTK_DEVICE, which does not, delivers NaN. */
 int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *stream);
 /* Device bytes held by the solver. */
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes);
@@ -329,6 +330,9 @@ int ptk_server_destroy(ptk_server *s);
  * bounded wait.  Returns PTK_ERR_TIMEOUT with *error_word = 1 and *elapsed_ms = the launch's device
  * time when the wait ran out as designed; the context stays usable.  No reference counterpart. */
 int ptk_selftest_wait_expiry(int *error_word, float *elapsed_ms);
+/* Raise the solver's error word on `stream`, as a run does whose bounded wait runs out (nothing waits and no
+ * kernel runs): for tests of what the host reports then. */
+int ptk_selftest_solver_expiry(ptk_solver *s, void *stream);
 
 /* ============================== autotuner ===================================================== */
 /* Time candidate tile shapes for a grid of the given size on the current device and return the

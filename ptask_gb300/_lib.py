@@ -144,6 +144,7 @@ _SIGS = {
     "ptk_server_destroy": (C.c_int, [_P]),
     "ptk_autotune_tiles":(C.c_int, [C.c_int, C.c_int, C.c_int, C.POINTER(TileConfig), C.POINTER(C.c_float)]),
     "ptk_default_tiles": (C.c_int, [C.c_int, C.c_int, C.c_int, C.POINTER(TileConfig)]),
+    "ptk_selftest_solver_expiry": (C.c_int, [_P, _P]),
     "ptk_selftest_wait_expiry": (C.c_int, [C.POINTER(C.c_int), C.POINTER(C.c_float)]),
     "ptk_problem_generate": (C.c_int, [C.POINTER(ProblemDesc), C.POINTER(FdtdParams), _P, _P, _P, _P,
                                        C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), _P]),

@@ -564,7 +564,7 @@ int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *str
     cudaStream_t st = S(stream);
     for (int q = 0; q < 6; ++q) PTK_CHECK_ARG(f[q], "field %d is NULL", q);
     const float *const *src = s->buf[s->par];
-    if (where != PTK_HOST) return launch_unpack_fields(src, s->L, f, 0, 6, st);
+    if (where != PTK_HOST) return launch_unpack_fields(src, s->L, f, 0, 6, st, s->d_err);
     size_t total = 0;
     for (int q = 0; q < 6; ++q) total += stage_bytes(q, s->p);
     const int per = total <= kStageTogether ? 6 : 1;
@@ -738,6 +738,15 @@ try {
     std::lock_guard<std::mutex> lk(s->mu);
     return solver_run(s, steps, S(stream));
 } PTK_CATCH_ALL
+
+int ptk_selftest_solver_expiry(ptk_solver *s, void *stream)
+{
+    clear_error();
+    PTK_CHECK_ARG(s, "NULL solver");
+    std::lock_guard<std::mutex> lk(s->mu);
+    PTK_CUDA_TRY(cudaMemsetAsync(s->d_err, 1, 1, S(stream)));
+    return PTK_OK;
+}
 
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes)
 {
