@@ -219,7 +219,8 @@ int ptk_solver_get_tiles(const ptk_solver *s, ptk_tile_config *cfg);
 /* Advance `steps` time steps, asynchronously on `stream`. */
 int ptk_solver_run(ptk_solver *s, int steps, void *stream);
 /* Read the six fields back (reference layout).  If a bounded wait of a run has run out, they are invalid:
- * PTK_HOST, which waits for them, returns PTK_ERR_TIMEOUT; PTK_DEVICE, which does not, delivers NaN. */
+ * PTK_HOST, which waits for them, returns PTK_ERR_TIMEOUT; PTK_DEVICE, which does not, delivers NaN; until
+ * ptk_solver_set_fields gives new ones, from which the solver runs as before. */
 int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *stream);
 /* Device bytes held by the solver. */
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes);

@@ -439,7 +439,7 @@ constexpr int kRowBatch = 4, kRowThreads = 256;
 
 struct RowMove {
     const float *src[6];
-    const int *err;            // UNPACK: where set, the fields become NaN (may be null)
+    int *err;                  // UNPACK: where set, the fields become NaN; PACK: cleared (may be null)
     float *dst[6], *wall[6];   // wall: where nodes of the walls i = Nx, j = Ny, k = Nz go as well, or null
     int ex[6], ey[6], rows[6]; // dense extents
     int nx, ny, nz, pitch;
@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const RowMove A)
     float *__restrict__ dst = A.dst[f];
     float *__restrict__ wall = A.wall[f];
     const bool bad = MODE == ROWS_UNPACK && A.err && *A.err;
+    if (MODE == ROWS_PACK && A.err && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *A.err = 0;
     const int step = gridDim.x * (kRowThreads / 32) * kRowBatch;
     for (int r0 = (blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5)) * kRowBatch; r0 < rows; r0 += step) {
         long long so[kRowBatch], to[kRowBatch];
@@ -515,9 +516,10 @@ static RowMove row_move(const Layout &L)
 }
 
 int launch_pack_fields(const float *const src[], const Layout &L, float *const dst[], float *const wall[], int first, int n,
-                       cudaStream_t s)
+                       cudaStream_t s, int *clear)
 {
     RowMove a = row_move(L);
+    a.err = clear;
     int most = 1;
     for (int q = 0; q < n; ++q) {
         int ez;
@@ -536,7 +538,7 @@ int launch_unpack_fields(const float *const src[], const Layout &L, float *const
                          const int *err)
 {
     RowMove a = row_move(L);
-    a.err = err;
+    a.err = const_cast<int *>(err);   // read only
     int most = 1;
     for (int q = 0; q < n; ++q) {
         int ez;

@@ -13,7 +13,8 @@
 // polls the data itself: no fence, no separate flag, one trip through L2.  Two slots by step parity:
 // a brick writes a slot again two steps later, after its neighbour's rows of the step between have
 // arrived, i.e. after that neighbour has consumed the slot.  Sequence numbers continue from launch
-// to launch (one counter per brick), so the buffer is cleared only when it is made.
+// to launch, counted by the host, so the buffer is cleared only when it is made, and what a launch that gave
+// up has left in it is never taken for a later one's.
 //
 // The bricks wait on one another, so the launch is cooperative (all bricks resident at once) and
 // every wait is bounded: on expiry the error word is raised and the launch ends with invalid fields,
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(kMaxT, 1) k_yee_resident(const ResidentArgs A)
     const float dbu = A.db;   // COEF_SIMPLE: the one Db
     const int qb = min(T - 1 - tid, (by + bz) * lw - 1);
 
-    unsigned seq = A.seq[cta];
+    unsigned seq = A.seq;
     __syncthreads();
 
     for (int step = 0; step < A.steps; ++step) {
@@ -472,7 +473,6 @@ __global__ void __launch_bounds__(kMaxT, 1) k_yee_resident(const ResidentArgs A)
         __syncthreads();
         if (*sfail) break;   // written before this barrier only; all threads leave together
     }
-    if (tid == 0) A.seq[cta] = seq;
 
     // ---- results: the cells of the brick --------------------------------------------------------------
 #pragma unroll 1

@@ -120,7 +120,7 @@ struct ptk_solver {
     bool resident = false;          // the grid fits on chip: staged shapes run whole runs in one launch
     ResidentPlan rplan{};
     ulonglong2 *d_xch = nullptr;    // its ghost rows in flight
-    unsigned *d_seq = nullptr;      // and sequence numbers
+    unsigned seq = 0;               // and the sequence number of the last step
     bool pair = false;              // staged shapes take long runs two steps at a time (fdtd_step_pair.cu)
     PairPlan pplan{};
     bool pair_maps = false;         // its tensor maps are encoded
@@ -177,12 +177,9 @@ static int prepare_fused(ptk_solver *s)
     s->fused_ready = true;
     cudaStream_t st = default_stream();
     if (plan_resident(s->L.nx, s->L.ny, s->L.nz, sm_count(), &s->rplan)) {
-        // the exchange buffer, and the bricks' counters behind it
-        const size_t seq = (s->rplan.xch_bytes + 255) / 256 * 256, total = seq + sizeof(unsigned) * s->rplan.nby * s->rplan.nbz;
-        if (pool_alloc(total, st, (void **)&s->d_xch) == PTK_OK) {
-            PTK_CUDA_TRY(cudaMemsetAsync(s->d_xch, 0, total, st));
+        if (pool_alloc(s->rplan.xch_bytes, st, (void **)&s->d_xch) == PTK_OK) {
+            PTK_CUDA_TRY(cudaMemsetAsync(s->d_xch, 0, s->rplan.xch_bytes, st));
             PTK_CUDA_TRY(cudaStreamSynchronize(st));   // runs may come on any stream
-            s->d_seq = (unsigned *)((char *)s->d_xch + seq);
             s->resident = true;
         } else {
             clear_error();   // no room for it: the tile shape's own kernel runs
@@ -367,10 +364,11 @@ static int run_resident(ptk_solver *s, int steps, cudaStream_t st)
     a.plane = s->L.plane;
     a.cx = s->p.Cx; a.cy = s->p.Cy; a.cz = s->p.Cz;
     a.xch = s->d_xch;
-    a.seq = s->d_seq;
+    a.seq = s->seq;
     a.err = s->d_err;
     int rc = launch_yee_resident(s->rplan, coef, a, st);
     if (rc) return rc;
+    s->seq += (unsigned)steps;
     s->last_launches = 1;
     s->step += steps;
     return PTK_OK;
@@ -531,7 +529,8 @@ int ptk_solver_set_fields(ptk_solver *s, const float *const f[6], int where, voi
     cudaStream_t st = S(stream);
     for (int q = 0; q < 6; ++q) PTK_CHECK_ARG(f[q], "field %d is NULL", q);
     float *const *dst = s->buf[s->par], *const *wall = s->buf[s->par ^ 1];
-    if (where != PTK_HOST) return launch_pack_fields(f, s->L, dst, wall, 0, 6, st);
+    // New fields end the state that an expired wait left behind.
+    if (where != PTK_HOST) return launch_pack_fields(f, s->L, dst, wall, 0, 6, st, s->d_err);
     // Host fields pass through device staging, all six at once where that is small, else one by one.
     size_t total = 0;
     for (int q = 0; q < 6; ++q) total += stage_bytes(q, s->p);
@@ -549,7 +548,7 @@ int ptk_solver_set_fields(ptk_solver *s, const float *const f[6], int where, voi
             PTK_CUDA_TRY(cudaMemcpyAsync(at, f[q], field_bytes(q, s->p), cudaMemcpyHostToDevice, st));
             at += stage_bytes(q, s->p);
         }
-        rc = launch_pack_fields(src, s->L, dst, wall, q0, per, st);
+        rc = launch_pack_fields(src, s->L, dst, wall, q0, per, st, s->d_err);
         pool_free(stage, st);
         if (rc) return rc;
     }

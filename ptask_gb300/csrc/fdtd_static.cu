@@ -74,17 +74,15 @@ __global__ void k_static_desc(InstDesc *dst, InstDesc v, int *tile0, int total)
     tile0[1] = total;
 }
 
-// Scratch of a run in one launch (fdtd_resident.cu): error word, sequence numbers and exchange buffer,
-// all cleared, then the fields and the coefficients in padded form.
+// Scratch of a run in one launch (fdtd_resident.cu): error word and exchange buffer, both cleared, then the fields and the coefficients in padded form.
 struct ResidentScratch {
-    size_t seq, xch, cleared, arrays, total;
+    size_t xch, cleared, arrays, total;
 };
 
 ResidentScratch resident_scratch(const ResidentPlan &p, size_t arr)
 {
     ResidentScratch r;
-    r.seq = kStaticAlign;
-    r.xch = r.seq + align_up(sizeof(unsigned) * p.nby * p.nbz);
+    r.xch = kStaticAlign;
     r.cleared = r.xch + p.xch_bytes;
     r.arrays = align_up(r.cleared);
     r.total = r.arrays + 10 * arr;
@@ -99,7 +97,6 @@ int solve_resident(const ptk_fdtd_params &p, float *const fields[6], const float
     PTK_CUDA_TRY(cudaMemsetAsync(b, 0, m.cleared, st));
     ResidentArgs a{};
     a.err = reinterpret_cast<int *>(b);
-    a.seq = reinterpret_cast<unsigned *>(b + m.seq);
     a.xch = reinterpret_cast<ulonglong2 *>(b + m.xch);
     float *f[6], *c[4];
     for (int q = 0; q < 6; ++q) f[q] = reinterpret_cast<float *>(b + m.arrays + q * arr);

@@ -187,7 +187,7 @@ struct ResidentArgs {
     long long plane;
     float cx, cy, cz;
     ulonglong2 *xch;           // plan.xch_bytes, zeroed when made, then kept from run to run
-    unsigned *seq;             // one counter per brick, likewise
+    unsigned seq;              // steps run on that buffer before: the run's rows carry seq + 1, seq + 2, ...
     int *err;                  // raised when a bounded wait expires
     // set by the launcher: the plan, and byte offsets and strides in shared memory
     int lw, lwp, by, bz, nby, nbz, kz, threads, half, base[6], row, plane_e, plane_h, below, fail;
@@ -235,8 +235,9 @@ int launch_advance(InstDesc *d_insts, int ninst, int nsteps, cudaStream_t s, int
 // Fields first .. first + n - 1 (indices into the arrays given) from the reference layout to the padded
 // one and back, in one launch.  `wall` (may be null): the other buffers, which get the wall nodes
 // i = Nx, j = Ny, k = Nz only: a step writes everything else before it is read.
+// `clear` (device, may be null): an error word that new fields take back.
 int launch_pack_fields(const float *const src[], const Layout &L, float *const dst[], float *const wall[], int first, int n,
-                       cudaStream_t s);
+                       cudaStream_t s, int *clear = nullptr);
 // `err` (device, may be null): a raised error word turns the unpacked fields into NaN, for callers that
 // do not wait for the result.
 int launch_unpack_fields(const float *const src[], const Layout &L, float *const dst[], int first, int n, cudaStream_t s,

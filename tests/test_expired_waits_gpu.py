@@ -49,3 +49,33 @@ def test_device_read_back_is_nan_after_an_expired_wait(shape, tiles):
         assert e.value.code == 5   # PTK_ERR_TIMEOUT
         for q, a in enumerate(fetch_device(s, shape)):
             assert np.isnan(a).all(), P.FIELDS[q]
+
+
+@pytest.mark.parametrize("where", [_lib.PTK_HOST, _lib.PTK_DEVICE])
+@pytest.mark.parametrize("shape,tiles", SOLVERS)
+def test_new_fields_after_an_expired_wait_run_as_before(shape, tiles, where):
+    """A run that finds the word raised gives up, on chip each block at its own step; the solver goes on with new fields."""
+    pr, f = problem(shape, 18)
+    ref = oracle.step_ext_f32(f, 18, pr.params, pr.Ca, pr.Cb, pr.Da, pr.Db, pr.src, pr.wave)
+    with P.Solver(pr.params) as s:
+        s.set_tiles(*tiles)
+        s.set_problem(pr)
+        s.set_fields(f)
+        s.run(18)
+        for _ in range(2):
+            _lib.call("ptk_selftest_solver_expiry", s.handle, None)
+            s.run(17)
+            with pytest.raises(_lib.PtkError):
+                s.get_fields()
+            if where == _lib.PTK_HOST:
+                s.set_fields(f)
+            else:
+                bufs = [DeviceBuffer.from_array(a) for a in f]
+                s.set_fields_device([b.value for b in bufs])
+                _lib.call("ptk_stream_sync", None)
+                for b in bufs:
+                    b.free()
+            s.reset_clock()
+            s.run(18)
+            for q, a in enumerate(s.get_fields()):
+                np.testing.assert_array_equal(a, ref[q], err_msg=P.FIELDS[q])
