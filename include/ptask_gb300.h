@@ -213,7 +213,8 @@ int ptk_solver_material_count(const ptk_solver *s, int *nmat);
 /* The kernel of single steps: ring stages (0 = register kernel) and whether it reads the material
  * index.  A staged shape with no per-cell-array instantiation falls back to 4 stages.  With a staged
  * shape, runs of 8 steps or more on grids that fit on chip are one launch, and runs of 16 or more on
- * larger ones take two steps per launch (ptk_solver_last_launches tells). */
+ * larger ones take two steps per launch (ptk_solver_last_launches tells); with the default shape or the
+ * autotuner's for the grid, shorter runs too take whatever form is fastest. */
 int ptk_solver_kernel(const ptk_solver *s, int *stages, int *material_index);
 int ptk_solver_get_tiles(const ptk_solver *s, ptk_tile_config *cfg);
 /* Advance `steps` time steps, asynchronously on `stream`. */

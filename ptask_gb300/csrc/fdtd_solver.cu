@@ -106,6 +106,9 @@ struct ptk_solver {
     int step = 0;              // host mirror of the device step counter
     int par = 0;               // buffer that holds the fields
     int by = 0, kc = 0, vec = 4, stages = 0;
+    bool ours = true;          // that shape is the default or the autotuner's: short runs may take another form
+    ptk_tile_config alt{};     // runs of up to alt_steps steps in such a form, where no fused one is taken
+    int alt_steps = 0;
     int *d_err = nullptr;      // raised by the staged kernel if a bounded wait expires
     void *d_tma = nullptr;     // tensor maps of the staged kernel (encoded for tma_by rows)
     int tma_by = 0;
@@ -282,6 +285,21 @@ static int solver_sync_desc(ptk_solver *s, int steps_left, cudaStream_t st)
     return PTK_OK;
 }
 
+// The autotuner's choices: a shape, and what its short runs take instead (ptk_solver::alt).
+struct Tuned {
+    ptk_tile_config best;
+    float ms;
+    ptk_tile_config alt;
+    int alt_steps;
+};
+static std::mutex g_tune_mu;
+static std::map<std::tuple<int, int, int>, Tuned> g_tune_cache;
+
+static bool same_tiles(const ptk_tile_config &a, const ptk_tile_config &b)
+{
+    return a.by == b.by && a.kc == b.kc && a.vec == b.vec && a.stages == b.stages;
+}
+
 static void drop_graphs(ptk_solver *s)
 {
     for (auto &kv : s->graphs) cudaGraphExecDestroy(kv.second);
@@ -351,7 +369,12 @@ static int run_resident(ptk_solver *s, int steps, cudaStream_t st)
     PTK_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
     if (capturing != cudaStreamCaptureStatusNone) return set_error(PTK_ERR_CUDA, "a run is not permitted when the stream is capturing");
     ResidentArgs a{};
-    for (int f = 0; f < 6; ++f) a.in[f] = a.out[f] = s->buf[s->par][f];   // in place (two steps or more)
+    // In place, but for a single step: no exchange then tells that a neighbour has read the rows it needs.
+    const int to = steps == 1 ? s->par ^ 1 : s->par;
+    for (int f = 0; f < 6; ++f) {
+        a.in[f] = s->buf[s->par][f];
+        a.out[f] = s->buf[to][f];
+    }
     for (int c = 0; c < 4; ++c) a.coef[c] = s->coef[c];
     const int coef = s->mat_enabled && s->minfo.simple ? COEF_SIMPLE : COEF_DENSE;
     a.db = s->minfo.db;
@@ -370,19 +393,44 @@ static int run_resident(ptk_solver *s, int steps, cudaStream_t st)
     if (rc) return rc;
     s->seq += (unsigned)steps;
     s->last_launches = 1;
+    s->par = to;
     s->step += steps;
     return PTK_OK;
 }
+
+// The solver's tiles for as long as the object lives.
+class TilesAs {
+    ptk_solver *s;
+    ptk_tile_config own;
+
+  public:
+    TilesAs(ptk_solver *s, const ptk_tile_config &c) : s(s), own{s->by, s->kc, s->vec, s->stages} { set(c); }
+    ~TilesAs() { set(own); }
+    void set(const ptk_tile_config &c) { s->by = c.by; s->kc = c.kc; s->vec = c.vec; s->stages = c.stages; }
+};
+
+static int run_steps(ptk_solver *s, int steps, bool pair, cudaStream_t st);
 
 int solver_run(ptk_solver *s, int steps, cudaStream_t st)
 {
     if (steps < 0) return set_error(PTK_ERR_INVALID, "negative step count");
     s->last_launches = 0;
     if (steps == 0) return PTK_OK;
-    if (s->resident && s->stages > 0 && steps >= kResidentSteps && !s->plain) return run_resident(s, steps, st);
+    const bool alt = s->ours && steps <= s->alt_steps;
+    if (s->resident && s->stages > 0 && !s->plain && (s->ours ? !alt : steps >= kResidentSteps)) return run_resident(s, steps, st);
+    const bool pair = s->pair && pair_mode(s) >= 0 && steps >= kPairSteps && !s->plain;
+    if (alt && !pair) {
+        TilesAs other(s, s->alt);
+        return run_steps(s, steps, false, st);
+    }
+    return run_steps(s, steps, pair, st);
+}
+
+// A run by replayed graphs.
+static int run_steps(ptk_solver *s, int steps, bool pair, cudaStream_t st)
+{
     int rc = solver_sync_desc(s, steps, st);
     if (rc) return rc;
-    const bool pair = s->pair && pair_mode(s) >= 0 && steps >= kPairSteps && !s->plain;
     if (pair && !s->pair_maps) {   // the arrays never move: encoded once
         alignas(64) unsigned char maps[kTmaSetBytes];
         InstDesc e = host_desc(s, steps);
@@ -692,6 +740,16 @@ int ptk_solver_set_tiles(ptk_solver *s, const ptk_tile_config *cfg)
     s->kc = kc;
     s->vec = vec;
     s->stages = stages;
+    s->ours = false;
+    {   // the autotuner's shape for this grid leaves the form of short runs to the solver, any other is taken at its word
+        std::lock_guard<std::mutex> tk(g_tune_mu);
+        auto it = g_tune_cache.find({s->p.Nx, s->p.Ny, s->p.Nz});
+        if (it != g_tune_cache.end() && same_tiles(it->second.best, {by, kc, vec, stages})) {
+            s->ours = true;
+            s->alt = it->second.alt;
+            s->alt_steps = it->second.alt_steps;
+        }
+    }
     return stages > 0 ? prepare_fused(s) : PTK_OK;
 }
 
@@ -828,9 +886,6 @@ int ptk_launch_e_half_step(const float *const e_in[3], const float *const h_new[
 // --------------------------------------------------------------------------------------------
 // Autotuner: time candidate (rows, depth) shapes on a scratch solver of the requested size.
 // --------------------------------------------------------------------------------------------
-static std::mutex g_tune_mu;
-static std::map<std::tuple<int, int, int>, std::pair<ptk_tile_config, float>> g_tune_cache;
-
 int ptk_autotune_tiles(int Nx, int Ny, int Nz, ptk_tile_config *best, float *best_ms)
 try {
     clear_error();
@@ -839,8 +894,8 @@ try {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find({Nx, Ny, Nz});
         if (it != g_tune_cache.end()) {
-            *best = it->second.first;
-            if (best_ms) *best_ms = it->second.second;
+            *best = it->second.best;
+            if (best_ms) *best_ms = it->second.ms;
             return PTK_OK;
         }
     }
@@ -859,7 +914,8 @@ try {
     const long long cells = (long long)Nx * Ny * Nz;
     const int steps = (int)std::max(4LL, std::min(64LL, 400000000LL / std::max(1LL, cells)));
     float best_t = 1e30f;
-    ptk_tile_config bc{8, 0, default_vec(Nx), 0};
+    ptk_tile_config bc{8, 0, default_vec(Nx), 0}, single = bc;   // the shape, and what its short runs take
+    int alt_steps = 0;
     std::vector<ptk_tile_config> cands;
     // Fixed depths plus the two that fill whole waves of resident CTAs best for each kernel.
     auto add = [&](int by, int vec, int stages, int resident) {
@@ -901,6 +957,24 @@ try {
         cudaEventElapsedTime(&ms, e0, e1);
         return ms / n;
     };
+    // ms per call of runs of a single step, by the shape's own kernel or as a fused run
+    auto time_single = [&](const ptk_tile_config &c, bool plain) -> float {
+        if (ptk_solver_set_tiles(s, &c)) return -1.f;
+        s->plain = plain;
+        s->ours = !plain;
+        s->alt_steps = 0;
+        const int n = 64;
+        float ms = 0;
+        for (int pass = 0; pass < 2; ++pass) {   // the first warms up
+            cudaEventRecord(e0, st);
+            for (int q = 0; q < n; ++q)
+                if (ptk_solver_run(s, 1, st)) return -1.f;
+            cudaEventRecord(e1, st);
+            cudaEventSynchronize(e1);
+            cudaEventElapsedTime(&ms, e0, e1);
+        }
+        return ms / n;
+    };
     s->plain = true;   // shapes are compared by their own kernels
     // First pass: every candidate, briefly.  Second pass: the closest few again over longer runs,
     // twice in alternating order, since shapes within a few per cent of each other trade places
@@ -932,8 +1006,9 @@ try {
                 bc = e.second;
             }
         // Staged shapes take long runs through the resident or the two-step kernel: the best of them is
-        // compared by such a run.
+        // compared by such a run.  The best shape by its own kernel stays for the runs that are not fused.
         s->plain = false;
+        single = bc;
         if ((s->resident || s->pair) && !rc)
             for (const auto &e : timed)
                 if (e.second.stages > 0) {
@@ -946,6 +1021,15 @@ try {
                     }
                     break;
                 }
+        if (!rc && s->resident && bc.stages > 0) {
+            // On chip every run is fused but, where that is faster, the single step (96^3: 25 us, fused 30; 64^3: 18,
+            // fused 15; two steps 38 and 35).
+            const float own = time_single(single, true), fused = time_single(bc, false);
+            if (own < 0 || fused < 0) rc = PTK_ERR_CUDA;
+            else if (own < fused) alt_steps = 1;
+        } else if (!rc && !same_tiles(single, bc)) {
+            alt_steps = INT_MAX;   // narrow grids: the staged tiles are mostly empty
+        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -953,7 +1037,7 @@ try {
     if (rc) return rc;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tune_cache[{Nx, Ny, Nz}] = {bc, best_t};
+        g_tune_cache[{Nx, Ny, Nz}] = {bc, best_t, single, alt_steps};
     }
     *best = bc;
     if (best_ms) *best_ms = best_t;
@@ -969,7 +1053,7 @@ try {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find({Nx, Ny, Nz});
         if (it != g_tune_cache.end()) {
-            *cfg = it->second.first;
+            *cfg = it->second.best;
             return PTK_OK;
         }
     }

@@ -192,8 +192,11 @@ struct ResidentArgs {
     // set by the launcher: the plan, and byte offsets and strides in shared memory
     int lw, lwp, by, bz, nby, nbz, kz, threads, half, base[6], row, plane_e, plane_h, below, fail;
 };
-// A run of this many steps or more on a grid that fits on chip is one resident launch instead of a step
-// kernel per time step.  (Loading and storing the fields costs 12-30 us, two to six launches' worth.)
+// On a grid that fits on chip a run of a solver whose shape the library chose is one resident launch whatever its
+// length, but for single steps where the autotuner found its best step kernel faster.  us a call for one step and for
+// seven, resident, by the default register tiles and by the tuned shape: 24^3 8.4, 24.7, 14.5 and 18.6, 107, 45; 96^3
+// 30, 39, 25 and 64, 215, 105.  A staged shape that a caller set runs fewer steps than this by its own kernel, as
+// the allocation-free solve does by the register kernel.
 constexpr int kResidentSteps = 8;
 // The plan for a grid on a device of `sms` SMs; false when it does not fit on chip.
 bool plan_resident(int nx, int ny, int nz, int sms, ResidentPlan *out);
