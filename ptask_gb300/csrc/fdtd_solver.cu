@@ -65,6 +65,15 @@ static void default_tiles(int nx, int ny, int nz, int *by, int *kc, int *vec)
 // (ptk_solver_last_launches).
 static constexpr long long kStagedCells = 1 << 12;
 
+// Where the default solver of a larger grid keeps the register kernel for what is not fused: on rows so short that
+// the staged tiles, 128 cells wide, are mostly empty, while one register tile of 32 cells covers them (us per step,
+// register and staged: 8x500x400 161 and 206, 18x330x210 62 and 72, 32x200x190 40 and 41, 33x200x190, two tiles, 66 and 43).
+// And for single steps where little else is in them than the staged graph's start, 5 us longer, and its walls'
+// launch: up to 48 cells (40x160x200 48 and 52, 48x150x150 41 and 43, 64x150x150 46 and 44), and on thin grids (1200x1200x1
+// 52 and 62, 3000x3000x2 342 and 350, 800x800x3 47 and 50; 1000x300x4 29 and 34, 60x3000x6 35 and 39, but 2000x2000x4 253 and 213).
+static constexpr int kNarrow = 32, kNarrowSingle = 48, kThin = 3, kThinSmall = 7;
+static constexpr long long kSmallCells = 2 << 20;
+
 // Uniform coefficients v = (Ca, Cb, Da, Db), and the one-entry table that goes with them.
 __global__ void k_uniform_coefs(float *Ca, float *Cb, float *Da, float *Db, long long n, float4 v, float4 *tab)
 {
@@ -210,6 +219,18 @@ static int uniform_vacuum(ptk_solver *s, cudaStream_t st, bool clear_index)
     s->minfo = MaterialInfo{};
     if (s->mat_enabled) s->minfo = MaterialInfo{1, 1, v.w};
     return PTK_OK;
+}
+
+// What the default shape's short runs take instead (kNarrow).
+static void default_alt(ptk_solver *s)
+{
+    const int nx = s->L.nx, nz = s->L.nz;
+    const bool narrow = nx <= kNarrowSingle && nx <= 32 * default_vec(nx);   // one register tile in x
+    const bool thin = nz <= kThin || (nz <= kThinSmall && (long long)nx * s->L.ny * nz < kSmallCells);
+    if (!narrow && !thin) return;
+    s->alt = ptk_tile_config{};
+    default_tiles(nx, s->L.ny, nz, &s->alt.by, &s->alt.kc, &s->alt.vec);
+    s->alt_steps = nx <= kNarrow ? INT_MAX : 1;
 }
 
 // The staged kernel's shape without timing: 11 rows, a 4-plane ring and the depth that fills whole waves
@@ -542,6 +563,7 @@ try {
         rc = staged_default(p->Nx, p->Ny, p->Nz, &c);
         s->by = c.by; s->kc = c.kc; s->vec = c.vec; s->stages = c.stages;
         if (rc == PTK_OK) rc = prepare_fused(s);
+        if (rc == PTK_OK && !s->resident) default_alt(s);
     }
     if (rc == PTK_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = set_error(PTK_ERR_CUDA, "solver initialisation failed");
     if (rc) {
@@ -772,7 +794,8 @@ int ptk_solver_material_count(const ptk_solver *s, int *nmat)
 int ptk_solver_kernel(const ptk_solver *s, int *stages, int *material_index)
 {
     PTK_CHECK_ARG(s && stages && material_index, "NULL argument");
-    const RunShape rs = run_shape(s);
+    RunShape rs = run_shape(s);
+    if (s->ours && s->alt_steps == INT_MAX) rs = {s->alt.by, s->alt.stages, false};   // a register shape
     *stages = rs.stages;
     *material_index = rs.mat ? 1 : 0;
     return PTK_OK;

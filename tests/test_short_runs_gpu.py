@@ -54,3 +54,25 @@ def test_short_runs_with_the_tuned_shape(shape):
                 assert s.last_launches() == 1
             assert s.tiles() == tiles
         check(s, pr, f, sum(parts), shape)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("shape,register", [((8, 400, 300), (1, 5, 15)), ((32, 200, 190), (1, 5, 15)), ((33, 200, 190), ()),
+                                            ((40, 160, 200), (1,)), ((49, 150, 150), ()), ((700, 700, 3), (1,)), ((60, 3000, 6), (1,))])
+def test_default_shape_of_narrow_and_thin_grids(shape, register, dense):
+    """Rows far shorter than a staged tile, and single steps of thin grids, keep the register kernel; long runs go two
+    steps per launch but for thin grids and media that vary in every coefficient."""
+    parts = (1, 5, 15, 19, 2)
+    pr, f = problem(shape, sum(parts))
+    if dense:
+        rng = np.random.default_rng(3)
+        for c in (pr.Ca, pr.Cb, pr.Da, pr.Db):
+            c *= 1 - np.float32(0.1) * rng.random(c.shape, dtype=np.float32)
+    with P.Solver(pr.params) as s:
+        assert s.kernel()[0] == (0 if 15 in register else 4)
+        s.set_problem(pr)
+        s.set_fields(f)
+        for n in parts:
+            s.run(n)
+            assert s.last_launches() == (n // 2 + 2 if n == 19 and shape[2] >= 8 and not dense else n + 1)
+        check(s, pr, f, sum(parts), shape)
