@@ -18,7 +18,8 @@
 //
 // The bricks wait on one another, so the launch is cooperative (all bricks resident at once) and
 // every wait is bounded: on expiry the error word is raised and the launch ends with invalid fields,
-// which the host reports as PTK_ERR_TIMEOUT.
+// which the host reports as PTK_ERR_TIMEOUT.  Where they cannot all be resident (a stream or context with fewer
+// SMs than the device) the launch is refused and its callers take a launch per step.
 //
 // Arithmetic is that of the step kernels, operation for operation.  With Ca = Da = 1 the products
 // Ca*E and Da*H are the factors themselves, bit for bit, and are left out (COEF_SIMPLE).
@@ -609,7 +610,12 @@ int launch_yee_resident(const ResidentPlan &p, int coef, ResidentArgs a, cudaStr
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     void *args[] = {&a};
-    PTK_CUDA_TRY(cudaLaunchKernelExC(&cfg, k, args));
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, k, args);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return kNotPlaced;
+    }
+    PTK_CUDA_TRY(e);
     count_launches(1);
     return PTK_OK;
 }

@@ -130,6 +130,7 @@ struct ptk_solver {
     int *d_work = nullptr;          // staged path: tile counters, one per step of a chunk
     int total_tiles = 0;
     bool resident = false;          // the grid fits on chip: staged shapes run whole runs in one launch
+    bool refused = false;           // such a launch could not be placed: not tried again
     ResidentPlan rplan{};
     ulonglong2 *d_xch = nullptr;    // its ghost rows in flight
     unsigned seq = 0;               // and the sequence number of the last step
@@ -231,6 +232,14 @@ static void default_alt(ptk_solver *s)
     s->alt = ptk_tile_config{};
     default_tiles(nx, s->L.ny, nz, &s->alt.by, &s->alt.kc, &s->alt.vec);
     s->alt_steps = nx <= kNarrow ? INT_MAX : 1;
+}
+
+// No run is fused after all: with the library's shape all take the best step kernel known.
+static void short_runs_off_chip(ptk_solver *s)
+{
+    if (!s->ours) return;
+    if (s->alt.by > 0) s->alt_steps = INT_MAX;   // the autotuner's
+    else default_alt(s);
 }
 
 // The staged kernel's shape without timing: 11 rows, a 4-plane ring and the depth that fills whole waves
@@ -438,7 +447,14 @@ int solver_run(ptk_solver *s, int steps, cudaStream_t st)
     s->last_launches = 0;
     if (steps == 0) return PTK_OK;
     const bool alt = s->ours && steps <= s->alt_steps;
-    if (s->resident && s->stages > 0 && !s->plain && (s->ours ? !alt : steps >= kResidentSteps)) return run_resident(s, steps, st);
+    if (s->resident && s->stages > 0 && !s->plain && (s->ours ? !alt : steps >= kResidentSteps)) {
+        const int rc = run_resident(s, steps, st);
+        if (rc != kNotPlaced) return rc;
+        s->resident = false;
+        s->refused = true;
+        short_runs_off_chip(s);
+        return solver_run(s, steps, st);
+    }
     const bool pair = s->pair && pair_mode(s) >= 0 && steps >= kPairSteps && !s->plain;
     if (alt && !pair) {
         TilesAs other(s, s->alt);
@@ -763,6 +779,8 @@ int ptk_solver_set_tiles(ptk_solver *s, const ptk_tile_config *cfg)
     s->vec = vec;
     s->stages = stages;
     s->ours = false;
+    s->alt = ptk_tile_config{};
+    s->alt_steps = 0;
     {   // the autotuner's shape for this grid leaves the form of short runs to the solver, any other is taken at its word
         std::lock_guard<std::mutex> tk(g_tune_mu);
         auto it = g_tune_cache.find({s->p.Nx, s->p.Ny, s->p.Nz});
@@ -770,6 +788,7 @@ int ptk_solver_set_tiles(ptk_solver *s, const ptk_tile_config *cfg)
             s->ours = true;
             s->alt = it->second.alt;
             s->alt_steps = it->second.alt_steps;
+            if (s->refused) short_runs_off_chip(s);
         }
     }
     return stages > 0 ? prepare_fused(s) : PTK_OK;

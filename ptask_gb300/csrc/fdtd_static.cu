@@ -180,9 +180,11 @@ int ptk_fdtd_solve_static(const ptk_fdtd_params *p, float *const fields[6], cons
         plan_resident(p->Nx, p->Ny, p->Nz, sms, &plan)) {
         const ResidentScratch m = resident_scratch(plan, arr);
         const float *const coefs[4] = {Ca, Cb, Da, Db};
-        if (m.total <= kStaticScratchBytes)
-            return solve_resident(*p, fields, coefs, has_src ? wave : nullptr, has_src ? nwave : 0,
-                                  has_src ? (long long)si + (long long)L.pitch * sj + L.plane * sk : -1, steps, L, plan, m, b, arr, st);
+        if (m.total <= kStaticScratchBytes) {
+            rc = solve_resident(*p, fields, coefs, has_src ? wave : nullptr, has_src ? nwave : 0,
+                                has_src ? (long long)si + (long long)L.pitch * sj + L.plane * sk : -1, steps, L, plan, m, b, arr, st);
+            if (rc != kNotPlaced) return rc;   // else step by step, from the caller's fields as they still are
+        }
     }
 
     // The scratch keeps the previous call's contents: clear everything this call uses.

@@ -200,6 +200,9 @@ struct ResidentArgs {
 constexpr int kResidentSteps = 8;
 // The plan for a grid on a device of `sms` SMs; false when it does not fit on chip.
 bool plan_resident(int nx, int ny, int nz, int sms, ResidentPlan *out);
+// kNotPlaced: the launch was refused because its bricks cannot all be resident at once (the plan counts the device's
+// SMs; a stream or context may have fewer).  Nothing has run: the step kernels are for such callers.
+constexpr int kNotPlaced = -1;
 int launch_yee_resident(const ResidentPlan &p, int coef, ResidentArgs a, cudaStream_t s);
 
 // ---------------------------------------------------------------------------------------------

@@ -1,0 +1,89 @@
+"""What the library does when a CUDA call that it can do without is refused.
+
+A preloaded library stands in front of the CUDA runtime in a child process and answers chosen calls with
+their error code; nothing reaches the GPU from those.
+"""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <cuda_runtime_api.h>
+#include <dlfcn.h>
+
+int refused;   /* calls answered with an error so far */
+
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args)
+{
+    for (unsigned q = 0; q < c->numAttrs; ++q)
+        if (c->attrs[q].id == cudaLaunchAttributeCooperative && c->attrs[q].val.cooperative) {
+            ++refused;
+            return cudaErrorCooperativeLaunchTooLarge;
+        }
+    cudaError_t (*next)(const cudaLaunchConfig_t *, const void *, void **) = dlsym(RTLD_NEXT, "cudaLaunchKernelExC");
+    return next(c, f, args);
+}
+"""
+
+PRELUDE = r"""
+import ctypes as C, sys
+import numpy as np
+import oracle, ptask_gb300 as P
+from ptask_gb300 import _lib
+from ptask_gb300.device import DeviceBuffer
+refused = C.c_int.in_dll(C.CDLL(sys.argv[1]), "refused")
+V = C.c_void_p
+def problem(shape, steps):
+    pr = P.Problem.generate(*shape, n_boxes=2, eps=(1, 8), box=(3, 9), steps=steps, source_mode=2, seed=sum(shape))
+    f = P.random_fields(*shape, seed=99, scale=1e-2)
+    return pr, f, oracle.step_ext_f32(f, steps, pr.params, pr.Ca, pr.Cb, pr.Da, pr.Db, pr.src, pr.wave)
+def same(got, ref):
+    for q in range(6):
+        np.testing.assert_array_equal(got[q], ref[q], err_msg=P.FIELDS[q])
+"""
+
+
+def child(tmp_path, body):
+    src, so = tmp_path / "shim.c", tmp_path / "shim.so"
+    src.write_text(SHIM)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-I", f"{cuda}/include", str(src), "-o", str(so), "-ldl"], check=True)
+    r = subprocess.run([sys.executable, "-c", PRELUDE + body, str(so)], cwd=ROOT, capture_output=True, text=True, timeout=240,
+                       env=dict(os.environ, LD_PRELOAD=str(so)))
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("shape", [(40, 33, 21), (30, 12, 16)])
+def test_step_kernels_where_an_on_chip_launch_cannot_be_placed(tmp_path, shape):
+    child(tmp_path, f"""
+shape = {shape}
+pr, f, ref = problem(shape, 21)
+for tiles in (None, (11, 0, 4, 4), "tuned"):
+    with P.Solver(pr.params) as s:
+        if tiles:
+            s.set_tiles(*(P.tuned_tiles(*shape) if tiles == "tuned" else tiles))
+        s.set_problem(pr)
+        s.set_fields(f)
+        before = refused.value
+        for n in (1, 9, 2, 9):
+            s.run(n)
+            assert s.last_launches() == n + 1
+        assert refused.value - before <= 1   # asked once
+        same(s.get_fields(), ref)
+assert refused.value >= 2
+before = refused.value
+bufs = [DeviceBuffer.from_array(a) for a in f]
+coefs = [DeviceBuffer.from_array(a) for a in (pr.Ca, pr.Cb, pr.Da, pr.Db, pr.wave)]
+_lib.call("ptk_fdtd_solve_static", C.byref(pr.params), (V * 6)(*[b.ptr for b in bufs]), *[c.ptr for c in coefs[:4]], *pr.src,
+          coefs[4].ptr, int(pr.wave.size), 21, None)
+_lib.call("ptk_device_sync")
+same([b.download(a.shape) for b, a in zip(bufs, f)], ref)
+assert refused.value == before + 1
+""")
