@@ -227,6 +227,8 @@ int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *str
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes);
 /* Number of kernel launches issued by the last ptk_solver_run (graph nodes included). */
 int ptk_solver_last_launches(const ptk_solver *s, long long *launches);
+/* CUDA graphs that it launched (none where the run is one launch). */
+int ptk_solver_last_graphs(const ptk_solver *s, long long *graphs);
 
 /* One-call solve with host buffers: upload fields + coefficients + source, run, download.
  * Ca..Db may be NULL for vacuum coefficients; wave may be NULL for no source.  fields[] are

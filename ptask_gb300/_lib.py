@@ -129,6 +129,7 @@ _SIGS = {
     "ptk_solver_run": (C.c_int, [_P, C.c_int, _P]),
     "ptk_solver_get_fields": (C.c_int, [_P, C.POINTER(_P), C.c_int, _P]),
     "ptk_solver_bytes": (C.c_int, [_P, C.POINTER(C.c_size_t)]),
+    "ptk_solver_last_graphs": (C.c_int, [_P, C.POINTER(C.c_longlong)]),
     "ptk_solver_last_launches": (C.c_int, [_P, C.POINTER(C.c_longlong)]),
     "ptk_fdtd_solve": (C.c_int, [C.POINTER(FdtdParams), C.POINTER(_P), _P, _P, _P, _P, C.c_int, C.c_int,
                                  C.c_int, _P, C.c_int, C.c_int, C.POINTER(C.c_float)]),

@@ -144,7 +144,7 @@ struct ptk_solver {
     int *d_tile0 = nullptr;
     cudaStream_t cap = nullptr;   // capture stream
     std::map<GraphKey, cudaGraphExec_t> graphs;
-    long long last_launches = 0;
+    long long last_launches = 0, last_graphs = 0;
     std::mutex mu;
 };
 
@@ -444,7 +444,7 @@ static int run_steps(ptk_solver *s, int steps, bool pair, cudaStream_t st);
 int solver_run(ptk_solver *s, int steps, cudaStream_t st)
 {
     if (steps < 0) return set_error(PTK_ERR_INVALID, "negative step count");
-    s->last_launches = 0;
+    s->last_launches = s->last_graphs = 0;
     if (steps == 0) return PTK_OK;
     const bool alt = s->ours && steps <= s->alt_steps;
     if (s->resident && s->stages > 0 && !s->plain && (s->ours ? !alt : steps >= kResidentSteps)) {
@@ -487,6 +487,7 @@ static int run_steps(ptk_solver *s, int steps, bool pair, cudaStream_t st)
         PTK_CUDA_TRY(cudaGraphLaunch(ex, st));
         count_graph_launch(flips + 1);
         s->last_launches += flips + 1;
+        ++s->last_graphs;
         s->par = (s->par + flips) & 1;
         left -= len;
     }
@@ -858,6 +859,13 @@ int ptk_solver_last_launches(const ptk_solver *s, long long *launches)
 {
     PTK_CHECK_ARG(s && launches, "NULL argument");
     *launches = s->last_launches;
+    return PTK_OK;
+}
+
+int ptk_solver_last_graphs(const ptk_solver *s, long long *graphs)
+{
+    PTK_CHECK_ARG(s && graphs, "NULL argument");
+    *graphs = s->last_graphs;
     return PTK_OK;
 }
 

@@ -1027,10 +1027,11 @@ bool Graph::try_lower_cycle(Task *top)
             if (rc == PTK_OK) rc = ptk_solver_reset_clock(plan->solver, m_stream);
             if (rc == PTK_OK) rc = ptk_solver_run(plan->solver, (int)N, m_stream);
             if (rc == PTK_OK) rc = ptk_solver_get_fields(plan->solver, dev, PTK_DEVICE, m_stream);
-            long long l = 0;
+            long long l = 0, graphs = 0;
             ptk_solver_last_launches(plan->solver, &l);
+            ptk_solver_last_graphs(plan->solver, &graphs);
             m_stats.kernel_launches += (UINT64)l;
-            m_stats.graph_replays += (UINT64)(N + 31) / 32;
+            m_stats.graph_replays += (UINT64)graphs;
         }
     } else {
         // Generic: capture [top; bottom] once for these blocks, replay N times.

@@ -1,0 +1,23 @@
+"""The public counters against what a run launches."""
+import ctypes as C
+
+import pytest
+
+import ptask_gb300 as P
+from ptask_gb300 import _lib
+from ptask_gb300.graph import FDTDGraph
+
+pytestmark = pytest.mark.gpu
+
+
+# on chip: one launch, no graph; shorter loops and larger grids: 32 steps a graph, two steps per launch 64
+@pytest.mark.parametrize("shape,steps,graphs", [((30, 22, 17), 70, 0), ((30, 22, 17), 5, 1), ((128, 96, 80), 200, 4),
+                                                ((128, 96, 80), 15, 1), ((150, 140, 6), 70, 0), ((700, 700, 3), 70, 3)])
+def test_graph_replays_of_a_lowered_loop(shape, steps, graphs):
+    f = P.zero_fields(*shape)
+    with FDTDGraph(P.reference_params(*shape), "fused") as g:
+        g.set_problem(P.Problem.vacuum(P.reference_params(*shape)))
+        for done in (1, 2):
+            g.solve(f, steps)
+            st = g.stats()
+            assert st["cycles_lowered"] == done and st["graph_replays"] == done * graphs
