@@ -223,7 +223,8 @@ int ptk_solver_run(ptk_solver *s, int steps, void *stream);
  * PTK_HOST, which waits for them, returns PTK_ERR_TIMEOUT; PTK_DEVICE, which does not, delivers NaN; until
  * ptk_solver_set_fields gives new ones, from which the solver runs as before. */
 int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *stream);
-/* Device bytes held by the solver. */
+/* Device bytes held by the solver: fields, coefficients, index and tables, the waveform, and on grids that fit on
+ * chip the exchange buffer of such runs. */
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes);
 /* Number of kernel launches issued by the last ptk_solver_run (graph nodes included). */
 int ptk_solver_last_launches(const ptk_solver *s, long long *launches);

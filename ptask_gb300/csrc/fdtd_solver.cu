@@ -107,6 +107,7 @@ struct ptk_solver {
     ptk_fdtd_params p;
     Layout L;
     void *block = nullptr;     // the one device allocation that holds the arrays below but wave and d_xch
+    size_t block_bytes = 0, wave_bytes = 0;
     float *buf[2][6] = {};
     float *coef[4] = {};
     float *wave = nullptr;
@@ -550,6 +551,7 @@ try {
     const size_t at_tab = take(sizeof(float) * 4 * kMaxMaterials), at_desc = take(sizeof(InstDesc));
     const size_t at_tile0 = take(2 * sizeof(int)), at_tma = take(kTmaSetBytes), at_pair = take(kTmaSetBytes);
     const size_t at_face0 = take(2 * sizeof(long long)), at_work = take(sizeof(int) * kPairChunk);
+    s->block_bytes = room;
     rc = pool_alloc(room, st, &s->block);
     if (rc) {
         ptk_solver_destroy(s);
@@ -737,8 +739,10 @@ int ptk_solver_set_source(ptk_solver *s, int i, int j, int k, const float *wave,
                   s->p.Nx, s->p.Ny, s->p.Nz);
     if (s->wave) pool_free(s->wave, st);
     s->wave = nullptr;
+    s->wave_bytes = 0;
     int rc = pool_alloc((size_t)nwave * sizeof(float), st, (void **)&s->wave);
     if (rc) return rc;
+    s->wave_bytes = (size_t)nwave * sizeof(float);
     PTK_CUDA_TRY(cudaMemcpyAsync(s->wave, wave, (size_t)nwave * sizeof(float),
                                  where == PTK_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
     s->nwave = nwave;
@@ -851,7 +855,7 @@ int ptk_selftest_solver_expiry(ptk_solver *s, void *stream)
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes)
 {
     PTK_CHECK_ARG(s && bytes, "NULL argument");
-    *bytes = (size_t)s->L.total * sizeof(float) * 16 + (size_t)s->nwave * sizeof(float);
+    *bytes = s->block_bytes + s->wave_bytes + (s->d_xch ? s->rplan.xch_bytes : 0);
     return PTK_OK;
 }
 

@@ -1,5 +1,6 @@
 """The public counters against what a run launches."""
 import ctypes as C
+import gc
 
 import pytest
 
@@ -21,3 +22,23 @@ def test_graph_replays_of_a_lowered_loop(shape, steps, graphs):
             g.solve(f, steps)
             st = g.stats()
             assert st["cycles_lowered"] == done and st["graph_replays"] == done * graphs
+
+
+def pool_used():
+    gc.collect()   # objects of earlier tests
+    _lib.call("ptk_device_sync")
+    reserved, used = C.c_size_t(), C.c_size_t()
+    _lib.call("ptk_pool_stats", C.byref(reserved), C.byref(used))
+    return used.value
+
+
+@pytest.mark.parametrize("shape", [(12, 12, 12), (96, 96, 96), (401, 9, 10), (200, 150, 100)])
+def test_solver_bytes_are_what_the_pool_gave(shape):
+    """Three allocations at most, each rounded up by the pool to no more than 2 MiB."""
+    pr = P.Problem.generate(*shape, n_boxes=1, box=(2, 6), steps=50000, seed=4)
+    before = pool_used()
+    with P.Solver(pr.params) as s:
+        s.set_problem(pr)
+        s.run(9)
+        taken = pool_used() - before
+        assert s.nbytes() <= taken <= s.nbytes() + 3 * (2 << 20)
