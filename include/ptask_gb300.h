@@ -226,7 +226,8 @@ int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *str
 /* Device bytes held by the solver: fields, coefficients, index and tables, the waveform, and on grids that fit on
  * chip the exchange buffer of such runs. */
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes);
-/* Number of kernel launches issued by the last ptk_solver_run (graph nodes included). */
+/* Kernel launches of the last ptk_solver_run that advance the cells, and the one of each graph that advances the
+ * clock; the staged kernels' one per graph for the walls is in ptk_launch_count only. */
 int ptk_solver_last_launches(const ptk_solver *s, long long *launches);
 /* CUDA graphs that it launched (none where the run is one launch). */
 int ptk_solver_last_graphs(const ptk_solver *s, long long *graphs);

@@ -486,7 +486,7 @@ static int run_steps(ptk_solver *s, int steps, bool pair, cudaStream_t st)
         rc = solver_graph(s, len, pair, &ex);
         if (rc) return rc;
         PTK_CUDA_TRY(cudaGraphLaunch(ex, st));
-        count_graph_launch(flips + 1);
+        count_graph_launch(flips + 1 + (run_shape(s).stages > 0 && s->faces > 0 ? 1 : 0));   // with the staged kernels' walls
         s->last_launches += flips + 1;
         ++s->last_graphs;
         s->par = (s->par + flips) & 1;

@@ -42,3 +42,19 @@ def test_solver_bytes_are_what_the_pool_gave(shape):
         s.run(9)
         taken = pool_used() - before
         assert s.nbytes() <= taken <= s.nbytes() + 3 * (2 << 20)
+
+
+@pytest.mark.parametrize("tiles,walls", [((8, 0, 4, 0), 0), ((11, 0, 4, 4), 1)])
+@pytest.mark.parametrize("shape,steps", [((40, 33, 21), 5), ((128, 96, 120), 40)])
+def test_launch_count_of_replayed_graphs(shape, steps, tiles, walls):
+    """Steps (two per launch on the larger grid's staged shape), the clock and the staged kernels' walls of each graph,
+    and the two launches that set a run up."""
+    fused = walls and steps == 40
+    graphs, launches = (2, 40) if steps == 40 and not fused else (1, 20 if fused else 5)
+    with P.Solver(P.reference_params(*shape)) as s:
+        s.set_tiles(*tiles)
+        for _ in range(2):
+            before = P.launch_count()
+            s.run(steps)
+            assert s.last_launches() == launches + graphs
+            assert P.launch_count() - before == launches + graphs * (1 + walls) + 2
