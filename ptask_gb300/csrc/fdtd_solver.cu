@@ -507,6 +507,20 @@ static size_t field_bytes(int f, const ptk_fdtd_params &p)
 static size_t stage_bytes(int f, const ptk_fdtd_params &p) { return (field_bytes(f, p) + 255) / 256 * 256; }
 static constexpr size_t kStageTogether = (size_t)256 << 20;
 
+// Staging of `n` arrays from `first` on, bytes(first, n) in all; of the first alone (n becomes 1) where the device
+// has no room for them together.
+template <class Bytes>
+static int stage_alloc(int first, int &n, const Bytes &bytes, cudaStream_t st, char **stage)
+{
+    int rc = pool_alloc(bytes(first, n), st, (void **)stage);
+    if (rc == PTK_ERR_NOMEM && n > 1) {
+        clear_error();
+        n = 1;
+        rc = pool_alloc(bytes(first, n), st, (void **)stage);
+    }
+    return rc;
+}
+
 }  // namespace ptk
 
 static inline cudaStream_t S(void *s) { return s ? (cudaStream_t)s : default_stream(); }
@@ -621,14 +635,15 @@ int ptk_solver_set_fields(ptk_solver *s, const float *const f[6], int where, voi
     // New fields end the state that an expired wait left behind.
     if (where != PTK_HOST) return launch_pack_fields(f, s->L, dst, wall, 0, 6, st, s->d_err);
     // Host fields pass through device staging, all six at once where that is small, else one by one.
-    size_t total = 0;
-    for (int q = 0; q < 6; ++q) total += stage_bytes(q, s->p);
-    const int per = total <= kStageTogether ? 6 : 1;
+    auto bytes = [s](int first, int n) {
+        size_t b = 0;
+        for (int q = first; q < first + n; ++q) b += stage_bytes(q, s->p);
+        return b;
+    };
+    int per = bytes(0, 6) <= kStageTogether ? 6 : 1;
     for (int q0 = 0; q0 < 6; q0 += per) {
-        size_t bytes = 0;
-        for (int q = q0; q < q0 + per; ++q) bytes += stage_bytes(q, s->p);
         char *stage = nullptr;
-        int rc = pool_alloc(bytes, st, (void **)&stage);
+        int rc = stage_alloc(q0, per, bytes, st, &stage);
         if (rc) return rc;
         const float *src[6] = {};
         char *at = stage;
@@ -653,14 +668,15 @@ int ptk_solver_get_fields(ptk_solver *s, float *const f[6], int where, void *str
     for (int q = 0; q < 6; ++q) PTK_CHECK_ARG(f[q], "field %d is NULL", q);
     const float *const *src = s->buf[s->par];
     if (where != PTK_HOST) return launch_unpack_fields(src, s->L, f, 0, 6, st, s->d_err);
-    size_t total = 0;
-    for (int q = 0; q < 6; ++q) total += stage_bytes(q, s->p);
-    const int per = total <= kStageTogether ? 6 : 1;
+    auto bytes = [s](int first, int n) {
+        size_t b = 0;
+        for (int q = first; q < first + n; ++q) b += stage_bytes(q, s->p);
+        return b;
+    };
+    int per = bytes(0, 6) <= kStageTogether ? 6 : 1;
     for (int q0 = 0; q0 < 6; q0 += per) {
-        size_t bytes = 0;
-        for (int q = q0; q < q0 + per; ++q) bytes += stage_bytes(q, s->p);
         char *stage = nullptr;
-        int rc = pool_alloc(bytes, st, (void **)&stage);
+        int rc = stage_alloc(q0, per, bytes, st, &stage);
         if (rc) return rc;
         float *dst[6] = {};
         char *at = stage;
@@ -694,11 +710,11 @@ int ptk_solver_set_coefficients(ptk_solver *s, const float *Ca, const float *Cb,
     cudaStream_t st = S(stream);
     const float *src[4] = {Ca, Cb, Da, Db};
     const size_t bytes = (size_t)s->p.Nx * s->p.Ny * s->p.Nz * sizeof(float), slot = (bytes + 255) / 256 * 256;
-    const int per = where != PTK_HOST || 4 * slot <= kStageTogether ? 4 : 1;
+    int per = where != PTK_HOST || 4 * slot <= kStageTogether ? 4 : 1;
     for (int c0 = 0; c0 < 4; c0 += per) {
         const float *from[4] = {};
         char *stage = nullptr;
-        int rc = where == PTK_HOST ? pool_alloc(per * slot, st, (void **)&stage) : PTK_OK;
+        int rc = where == PTK_HOST ? stage_alloc(c0, per, [slot](int, int n) { return n * slot; }, st, &stage) : PTK_OK;
         if (rc) return rc;
         for (int c = c0; c < c0 + per; ++c) {
             from[c] = where == PTK_HOST ? (const float *)(stage + (c - c0) * slot) : src[c];

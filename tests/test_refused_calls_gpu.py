@@ -18,7 +18,18 @@ SHIM = r"""
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
 
-int refused;   /* calls answered with an error so far */
+int refused, starved; /* launches and allocations answered with an error so far */
+size_t limit = -1;    /* bytes of an allocation at most */
+
+cudaError_t cudaMallocFromPoolAsync(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream)
+{
+    if (bytes > limit) {
+        ++starved;
+        return cudaErrorMemoryAllocation;
+    }
+    cudaError_t (*next)(void **, size_t, cudaMemPool_t, cudaStream_t) = dlsym(RTLD_NEXT, "cudaMallocFromPoolAsync");
+    return next(p, bytes, pool, stream);
+}
 
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args)
 {
@@ -38,7 +49,8 @@ import numpy as np
 import oracle, ptask_gb300 as P
 from ptask_gb300 import _lib
 from ptask_gb300.device import DeviceBuffer
-refused = C.c_int.in_dll(C.CDLL(sys.argv[1]), "refused")
+refused, starved = (C.c_int.in_dll(C.CDLL(sys.argv[1]), n) for n in ("refused", "starved"))
+limit = C.c_size_t.in_dll(C.CDLL(sys.argv[1]), "limit")
 V = C.c_void_p
 def problem(shape, steps):
     pr = P.Problem.generate(*shape, n_boxes=2, eps=(1, 8), box=(3, 9), steps=steps, source_mode=2, seed=sum(shape))
@@ -54,7 +66,8 @@ def child(tmp_path, body):
     src, so = tmp_path / "shim.c", tmp_path / "shim.so"
     src.write_text(SHIM)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-I", f"{cuda}/include", str(src), "-o", str(so), "-ldl"], check=True)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-I", f"{cuda}/include", str(src), "-o", str(so), "-ldl", "-Wl,--no-as-needed",
+                    "-L", f"{cuda}/lib64", "-lcudart", f"-Wl,-rpath,{cuda}/lib64"], check=True)   # the runtime is next to it
     r = subprocess.run([sys.executable, "-c", PRELUDE + body, str(so)], cwd=ROOT, capture_output=True, text=True, timeout=240,
                        env=dict(os.environ, LD_PRELOAD=str(so)))
     assert r.returncode == 0, r.stdout + r.stderr
@@ -86,4 +99,26 @@ _lib.call("ptk_fdtd_solve_static", C.byref(pr.params), (V * 6)(*[b.ptr for b in 
 _lib.call("ptk_device_sync")
 same([b.download(a.shape) for b, a in zip(bufs, f)], ref)
 assert refused.value == before + 1
+""")
+
+
+def test_host_arrays_are_staged_one_by_one_where_there_is_no_room_for_all(tmp_path):
+    child(tmp_path, """
+shape, steps = (40, 33, 21), 9
+pr, f, ref = problem(shape, steps)
+with P.Solver(pr.params) as s:
+    limit.value = max(a.nbytes for a in f) + 256   # the largest field's slot, and no more
+    s.set_problem(pr)
+    s.set_fields(f)
+    s.run(steps)
+    got = s.get_fields()
+    assert starved.value == 6, starved.value   # coefficients, fields, fields back: each tried twice
+    same(got, ref)
+    limit.value = 1000
+    for call in (lambda: s.set_fields(f), s.get_fields, lambda: s.set_problem(pr)):
+        try:
+            call()
+            raise SystemExit("no error")
+        except _lib.PtkError as e:
+            assert e.code == 3, e.code   # PTK_ERR_NOMEM
 """)
