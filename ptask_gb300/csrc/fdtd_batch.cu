@@ -4,7 +4,7 @@
 // Two time steps of every active instance are ONE launch of the two-step kernel (k_yee_pair, a CTA per
 // tile of the instances' tile lists).  An instance with an odd number of steps takes one of them by the
 // TMA-staged one-step kernel (k_yee_step_bulk) when it joins; a batch that holds an instance too thin for
-// pairs (fewer than 8 planes or 4 rows) takes all its steps by it, or by the register kernel on request.
+// pairs (fewer than 8 planes or 4 rows, or 4 GB a field) takes all its steps by it, or by the register kernel on request.
 // Both take the coefficients from a material index.  Chunks of steps are replayed as captured CUDA graphs
 // (at most kMaxGraphs kept).  Device time of a mix, two steps per pass against one: 64 requests of 32..192
 // 528 ms against 1050, 64 x 32^3 3.4 against 18.0, one 256^3 23 against 40, one 24^3 2.0 against 4.4.

@@ -555,27 +555,27 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
 namespace {
 
-// Bytes of a stage's copies; false when the ids do not fit theirs.
-bool lay_out(PairPlan &p)
+// Bytes of a stage's copies.
+void lay_out(PairPlan &p)
 {
     PairArgs &a = p.args;
-    a.mw = (4 * a.lw + 12 + 15) / 16 * 16;
     a.tx_bytes = 16 * a.lw * (6 * a.rf + 2) + a.mw * a.rf;   // Ex, Ez: one row more
     p.smem = kPairBytes;
     a.one = 1.0f;
-    return a.mw * a.rf <= kIds;
 }
 
 }  // namespace
 
 // The frame of nxt tiles in x and at least `nyt` in y, with no more rows than that needs.  False when no such
-// frame exists; a->nyt may come out larger, where the threads do not allow the rows.
+// frame exists; a->nyt may come out larger, where the threads or the room for the ids do not allow the rows.  Every
+// grid of 4 rows or more has a frame for some nxt.
 static bool pair_frame(int nx, int ny, int nxt, int nyt, int threads, PairArgs *a)
 {
     a->nxt = nxt;
     a->lw = (nx + 1 + 4 * (nxt - 1) + 4 * nxt - 1) / (4 * nxt);
     if (a->lw > kMaxLw || (a->lw < 8 && nxt > 1)) return false;
-    const int most = std::min(std::min(threads / a->lw, 255), ny + 1);
+    a->mw = (4 * a->lw + 12 + 15) / 16 * 16;
+    const int most = std::min(std::min(threads / a->lw, 255), std::min(ny + 1, kIds / a->mw));
     if (most < 5) return false;
     const int least = ny <= most - 1 ? 1 : 1 + (ny - (most - 1) + most - 4) / (most - 3);   // tiles with all those rows
     a->nyt = std::max(nyt, least);
@@ -609,7 +609,8 @@ bool plan_pair(int nx, int ny, int nz, PairPlan *out)
                 p.args.nzt = nzt; p.args.kc = kc; p.args.tiles = (int)tiles;
                 p.grid = (int)std::min<long long>(tiles, sms);
                 const double c = (double)waves * (kc + 3.5) * plane;
-                if (c < best && lay_out(p)) {
+                if (c < best) {
+                    lay_out(p);
                     best = c;
                     *out = p;
                     found = true;
@@ -630,7 +631,8 @@ bool plan_pair_member(int nx, int ny, int nz, PairPlan *out)
     for (int nxt = 1; nxt <= 64; ++nxt) {
         PairPlan p{};
         if (!pair_frame(nx, ny, nxt, 1, kBatchThreads, &p.args)) continue;
-        if (lay_out(p) && (!found || nxt * p.args.nyt < out->args.nxt * out->args.nyt)) {
+        if (!found || nxt * p.args.nyt < out->args.nxt * out->args.nyt) {
+            lay_out(p);
             *out = p;
             found = true;
         }

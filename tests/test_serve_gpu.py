@@ -241,3 +241,21 @@ def test_single_steps_of_odd_counts():
                                           pr.Db, pr.src, pr.wave)
                 for q in range(6):
                     np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{r} chunk {chunk} {P.FIELDS[q]}")
+
+
+@pytest.mark.parametrize("shapes", [[(7, 120, 16), (10, 100, 12)], [(1, 192, 8), (3, 254, 9), (4, 96, 8), (11, 230, 10), (24, 20, 16)]])
+def test_narrow_tall_instances_take_two_steps_per_pass(shapes):
+    """Rows of one to three units: frames end at the room for the material ids, not at the threads."""
+    reqs = [Request(*n, 14, 1 + q, 70 + q, box=(1, 4)) for q, n in enumerate(shapes)]
+    with Server(keep_results=True, chunk_steps=32) as s:
+        tickets = [s.submit(r) for r in reqs]
+        s.run(time_scale=0)
+        assert s.stats()["kernel_launches"] <= 14 // 2 + 4   # a launch per pair of steps, the walls, the clock
+        for t, r in zip(tickets, reqs):
+            got = s.fetch(t)
+            pr = P.Problem.generate(r.nx, r.ny, r.nz, n_boxes=r.n_boxes, eps=r.eps, box=r.box, steps=r.steps,
+                                    source_mode=r.source_mode, seed=r.seed)
+            ref = oracle.step_ext_f32(P.zero_fields(r.nx, r.ny, r.nz), r.steps, pr.params, pr.Ca, pr.Cb, pr.Da,
+                                      pr.Db, pr.src, pr.wave)
+            for q in range(6):
+                np.testing.assert_array_equal(got[q], ref[q], err_msg=f"{r} {P.FIELDS[q]}")
