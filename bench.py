@@ -166,7 +166,7 @@ def hbm_peak():
 def kernel_of(solver, steps: int):
     """(name, time steps per pass over memory) of the kernel that took the solver's last run of `steps`."""
     launches = solver.last_launches()
-    if launches == 1 and steps > 1:
+    if launches == 1:   # the step kernels launch the clock's advance too
         return "k_yee_resident", steps
     if launches < 3 * steps // 4:
         return "k_yee_pair", 2
@@ -175,11 +175,15 @@ def kernel_of(solver, steps: int):
 
 def traffic_per_cell(kernel: str, mat: bool = False, rows: int = 0):
     """DRAM bytes per cell update of the given step kernel from its committed ncu summary (the
-    64-wide 23-row tiles have their own; other staged shapes use the 11-row figure)."""
-    name = {("k_yee_pair", True): "yee_pair_256.md", ("k_yee_step_bulk", True): "yee_step_bulk_mat_256.md", ("k_yee_step_bulk", False): "yee_step_bulk_256.md"}
+    64-wide 23-row tiles have their own; other staged shapes use the 11-row figure); None for a kernel
+    that has no such summary (whole runs on chip; two steps per pass with a Cb per cell)."""
+    name = {("k_yee_pair", True): "yee_pair_256.md", ("k_yee_step_bulk", True): "yee_step_bulk_mat_256.md",
+            ("k_yee_step_bulk", False): "yee_step_bulk_256.md", ("k_yee_step", False): "yee_step_256.md"}
     if kernel == "k_yee_step_bulk" and mat and rows == 23:
         name[(kernel, mat)] = "yee_step_bulk_mat23_256.md"
-    f = ROOT / "profiles" / name.get((kernel, mat), "yee_step_256.md")
+    if (kernel, mat) not in name:
+        return None
+    f = ROOT / "profiles" / name[kernel, mat]
     if not f.exists():
         return None
     for line in f.read_text().splitlines():
@@ -189,6 +193,20 @@ def traffic_per_cell(kernel: str, mat: bool = False, rows: int = 0):
             except ValueError:
                 return None
     return None
+
+
+def bytes_per_update(kernel: str, mat: bool, per_pass: int) -> float:
+    """Algorithmic bytes per cell update: fields once in and once out per pass, and the coefficients as
+    the kernel reads them: ids, or a Cb per cell (the workloads are lossless), or four arrays."""
+    if kernel == "k_yee_resident" or (kernel == "k_yee_pair" and not mat):
+        return (48 + 4) / per_pass
+    return (BYTES_PER_CELL_MAT if mat else BYTES_PER_CELL) / per_pass
+
+
+def served_bytes(reqs) -> float:
+    """Algorithmic bytes of a request set's steps on the server: two per pass, and the odd one of a request
+    whose count is odd by itself."""
+    return sum(BYTES_PER_CELL_MAT * float(r.nx * r.ny * r.nz) * (r.steps // 2 + r.steps % 2) for r in reqs)
 
 
 def cpu_sample(prob, shape, target_s: float = 10.0):
@@ -417,7 +435,7 @@ def run_ours(args, wl, world, rank, local):
     peak, peak_src = hbm_peak()
     run_stages, mat = solver.kernel()
     kernel, per_pass = kernel_of(solver, T)
-    bpc = (BYTES_PER_CELL_MAT if mat else BYTES_PER_CELL) / per_pass
+    bpc = bytes_per_update(kernel, mat, per_pass)
     achieved = bpc * cells / (per_step_ms / 1e3) / 1e9
     by, kc, vec, stages = solver.tiles()
     tpc = traffic_per_cell(kernel, mat, by)
@@ -428,9 +446,10 @@ def run_ours(args, wl, world, rank, local):
         "data": "synthetic (seeded problem generator)",
         "config": workload_config(wl, world),
         "bench_step": "one complete solve (all time steps) from resident initial fields",
-        "kernel": {"tiles": {"rows": by, "z_depth": kc, "cells_per_thread": vec, "staged_planes": run_stages,
-                             "kernel": kernel},
-                   "coefficients": (f"material index: {solver.material_count()} distinct (Ca, Cb, Da, Db) tuples, "
+        "kernel": {"name": kernel,
+                   "single_step_tiles": {"rows": by, "z_depth": kc, "cells_per_thread": vec, "staged_planes": run_stages},
+                   "coefficients": ("Cb per cell, Ca = Da = 1 and one Db" if kernel == "k_yee_resident" or (kernel == "k_yee_pair" and not mat)
+                                    else f"material index: {solver.material_count()} distinct (Ca, Cb, Da, Db) tuples, "
                                     "one byte per node + table; per-cell arrays given at the API" if mat else
                                     "four per-cell FP32 arrays")},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -504,7 +523,7 @@ def serve_arms(reqs, scale: float, rows: int, *, cb_runs: int = 1, cb_warmup: in
         a = {"solves_per_s": len(reqs) / wall, "mcell_updates_per_s": cells / wall / 1e6, "wall_s": wall,
              "p50_latency_s": p50, "p99_latency_s": p99}
         if chunk_dev:
-            a["frac_of_peak_over_device_time"] = BYTES_PER_CELL_MAT / 2 * cells / chunk_dev / 1e9 / peak
+            a["frac_of_peak_over_device_time"] = served_bytes(reqs) / chunk_dev / 1e9 / peak
         return a
 
     for _ in range(cb_warmup):
@@ -527,7 +546,7 @@ def serve_arms(reqs, scale: float, rows: int, *, cb_runs: int = 1, cb_warmup: in
            "plain_fused": arm_of(plain["wall_s"], plain["p50_latency_s"], plain["p99_latency_s"],
                                  plain["chunk_device_s"]),
            "gpu_launches": int(best["launches"]), "clocks": clk,
-           "roofline_basis": "24.5 algorithmic bytes per cell update (material index, two steps per pass) over the device time "
+           "roofline_basis": "49 algorithmic bytes per cell and pass (material index; two steps a pass, the odd one of a request by itself) over the device time "
                              "of the replayed chunks (every step launch, faces, advances) of the whole request set; "
                              f"peak {peak:.1f} GB/s ({peak_src})"}
     for mode in graph_arms:
@@ -561,7 +580,7 @@ def default_rows(kind: str) -> int:
 def large_subrecord(local: int, solves: int = 3) -> dict:
     """The large workload (512x512x384, 32 boxes, 500 steps) solved from resident zero fields with the
     autotuned tiles: Mcell-updates/s over `solves` complete solves (CUDA events) and the step kernel
-    against the measured HBM bandwidth at 49 (material index) or 64 bytes per cell and pass."""
+    against the measured HBM bandwidth at its algorithmic bytes per cell update."""
     import ptask_gb300 as P
     from ptask_gb300.device import DeviceBuffer, Event
     wl = WORKLOADS["large"]
@@ -597,12 +616,12 @@ def large_subrecord(local: int, solves: int = 3) -> dict:
     for b in dev:
         b.free()
     peak, peak_src = hbm_peak()
-    bpc = (BYTES_PER_CELL_MAT if mat else BYTES_PER_CELL) / per_pass
+    bpc = bytes_per_update(kernel, mat, per_pass)
     achieved = bpc * cells * T / (ms / 1e3) / 1e9
     return {"workload": wl["desc"], "grid": list(shape), "time_steps": T, "solves": solves,
             "mcell_updates_per_s": cells * T / (ms / 1e3) / 1e6, "ms_per_solve": ms,
-            "tiles": {"rows": tiles[0], "z_depth": tiles[1], "cells_per_thread": tiles[2], "staged_planes": stages,
-                      "material_index": mat},
+            "single_step_tiles": {"rows": tiles[0], "z_depth": tiles[1], "cells_per_thread": tiles[2], "staged_planes": stages,
+                                  "material_index": mat},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_src, "algorithmic_bytes_per_cell_update": bpc, "kernel": kernel,
                          "basis": "whole solves (step launches, faces, advances) over CUDA-event time"},
