@@ -59,10 +59,11 @@ static void default_tiles(int nx, int ny, int nz, int *by, int *kc, int *vec)
     *kc = k;
 }
 
-// Grids of more than this many cells start with the staged kernel's shape, whose longer runs are one
-// resident launch or take two steps per pass (24^3: 1.6 us per step against 12.8; 32^3: 1.6 against 5.5; 256^3:
-// 87 against 215).  Smaller ones keep the register kernel and a launch per step, which callers count
-// (ptk_solver_last_launches).
+// Grids of more than this many cells start with the staged kernel's shape, whose runs are resident launches or
+// take two steps per pass (24^3: 1.6 us per step against 12.8; 32^3: 1.6 against 5.5; 256^3: 87 against 215).  Smaller
+// ones keep the register kernel and a launch per step not for speed (16^3, 70 steps: 894 us, on chip 112; 6^3: 494 and
+// 102) but because the launches of their default runs are a published figure (ptk_solver_last_launches: the steps, and
+// one per 32).  A caller who wants the speed sets the staged or the tuned shape.
 static constexpr long long kStagedCells = 1 << 12;
 
 // Where the default solver of a larger grid keeps the register kernel for what is not fused: on rows so short that

@@ -587,7 +587,7 @@ static bool pair_fits(int nx, int ny, int nz) { return make_layout(nx, ny, nz).t
 
 // The tile shape with the least estimated time for two steps: rounds of resident CTAs times the planes each
 // streams (its depth, the planes recomputed at its start, the ring's turn at its end) times a plane's time, which
-// grows with the frame's warps (320 threads of 384: 0.89 of the time)
+// grows with the frame's warps (320 threads of 352: taken as 0.94 of the time)
 // and is 7-14 % longer with rows of 9 to 11 units than of 13 and more.
 bool plan_pair(int nx, int ny, int nz, PairPlan *out)
 {
