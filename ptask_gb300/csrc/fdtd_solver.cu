@@ -107,8 +107,8 @@ static constexpr int kChunk = 32, kPairChunk = 64;
 struct ptk_solver {
     ptk_fdtd_params p;
     Layout L;
-    void *block = nullptr;     // the one device allocation that holds the arrays below but wave and d_xch
-    size_t block_bytes = 0, wave_bytes = 0;
+    std::vector<void *> parts; // the device allocations, one as a rule, that hold the arrays below but wave and d_xch
+    size_t held_bytes = 0, wave_bytes = 0;
     float *buf[2][6] = {};
     float *coef[4] = {};
     float *wave = nullptr;
@@ -551,45 +551,62 @@ try {
     default_tiles(p->Nx, p->Ny, p->Nz, &s->by, &s->kc, &s->vec);
     cudaStream_t st = default_stream();
     const size_t bytes = (size_t)s->L.total * sizeof(float);
-    size_t room = 0;
-    auto take = [&room](size_t n) {   // 256-byte aligned places in the block
-        const size_t at = room;
-        room += (n + 255) / 256 * 256;
-        return at;
+    // Everything but the waveform and the exchange buffer: places of one block, 256-byte aligned, those that start at
+    // zero first; allocations of their own where the device has room for each but no block that holds them all.
+    struct Place {
+        void **to;
+        size_t bytes;
+        bool zero;
     };
-    size_t at_buf[2][6], at_coef[4];
+    std::vector<Place> places;
     for (int b = 0; b < 2; ++b)
-        for (int f = 0; f < 6; ++f) at_buf[b][f] = take(bytes);
-    const size_t at_mat = take((size_t)s->L.total), at_err = take(sizeof(int));
-    const size_t cleared = room;      // fields, index and error word start at zero
-    for (int c = 0; c < 4; ++c) at_coef[c] = take(bytes);
-    const size_t at_tab = take(sizeof(float) * 4 * kMaxMaterials), at_desc = take(sizeof(InstDesc));
-    const size_t at_tile0 = take(2 * sizeof(int)), at_tma = take(kTmaSetBytes), at_pair = take(kTmaSetBytes);
-    const size_t at_face0 = take(2 * sizeof(long long)), at_work = take(sizeof(int) * kPairChunk);
-    s->block_bytes = room;
-    rc = pool_alloc(room, st, &s->block);
+        for (int f = 0; f < 6; ++f) places.push_back({(void **)&s->buf[b][f], bytes, true});
+    places.push_back({(void **)&s->mat, (size_t)s->L.total, true});
+    places.push_back({(void **)&s->d_err, sizeof(int), true});
+    for (int c = 0; c < 4; ++c) places.push_back({(void **)&s->coef[c], bytes, false});
+    places.push_back({(void **)&s->mat_tab, sizeof(float) * 4 * kMaxMaterials, false});
+    places.push_back({(void **)&s->d_desc, sizeof(InstDesc), false});
+    places.push_back({(void **)&s->d_tile0, 2 * sizeof(int), false});
+    places.push_back({&s->d_tma, kTmaSetBytes, false});
+    places.push_back({&s->d_tma_pair, kTmaSetBytes, false});
+    places.push_back({(void **)&s->d_face0, 2 * sizeof(long long), false});
+    places.push_back({(void **)&s->d_work, sizeof(int) * kPairChunk, false});
+    size_t cleared = 0;
+    for (Place &q : places) {
+        q.bytes = (q.bytes + 255) / 256 * 256;
+        s->held_bytes += q.bytes;
+        if (q.zero) cleared += q.bytes;
+    }
+    s->parts.reserve(places.size());
+    void *base = nullptr;
+    rc = pool_alloc(s->held_bytes, st, &base);
+    if (rc == PTK_OK) {
+        s->parts.push_back(base);
+        char *at = static_cast<char *>(base);
+        for (const Place &q : places) {
+            *q.to = at;
+            at += q.bytes;
+        }
+        if (cudaMemsetAsync(base, 0, cleared, st) != cudaSuccess) rc = set_error(PTK_ERR_CUDA, "solver initialisation failed");
+    } else if (rc == PTK_ERR_NOMEM) {
+        clear_error();
+        rc = PTK_OK;
+        for (const Place &q : places) {
+            rc = pool_alloc(q.bytes, st, q.to);
+            if (rc) break;
+            s->parts.push_back(*q.to);
+            if (q.zero && cudaMemsetAsync(*q.to, 0, q.bytes, st) != cudaSuccess) rc = set_error(PTK_ERR_CUDA, "solver initialisation failed");
+            if (rc) break;
+        }
+    }
     if (rc) {
         ptk_solver_destroy(s);
         return rc;
     }
-    char *base = static_cast<char *>(s->block);
-    for (int b = 0; b < 2; ++b)
-        for (int f = 0; f < 6; ++f) s->buf[b][f] = (float *)(base + at_buf[b][f]);
-    for (int c = 0; c < 4; ++c) s->coef[c] = (float *)(base + at_coef[c]);
-    s->mat = (unsigned char *)(base + at_mat);
-    s->mat_tab = (float *)(base + at_tab);
-    s->d_err = (int *)(base + at_err);
-    s->d_desc = (InstDesc *)(base + at_desc);
-    s->d_tile0 = (int *)(base + at_tile0);
-    s->d_tma = base + at_tma;
-    s->d_tma_pair = base + at_pair;
-    s->d_face0 = (long long *)(base + at_face0);
-    s->d_work = (int *)(base + at_work);
     s->faces = face_nodes(p->Nx, p->Ny, p->Nz);
     const long long f0[2] = {0, s->faces};   // pageable: staged before the call returns
-    if ((uintptr_t)base & 63) rc = set_error(PTK_ERR_CUDA, "tensor-map buffer is not 64-byte aligned");
-    if (rc == PTK_OK && (cudaMemsetAsync(base, 0, cleared, st) != cudaSuccess ||
-                         cudaMemcpyAsync(s->d_face0, f0, sizeof f0, cudaMemcpyHostToDevice, st) != cudaSuccess))
+    if (((uintptr_t)s->d_tma | (uintptr_t)s->d_tma_pair) & 63) rc = set_error(PTK_ERR_CUDA, "tensor-map buffer is not 64-byte aligned");
+    if (rc == PTK_OK && cudaMemcpyAsync(s->d_face0, f0, sizeof f0, cudaMemcpyHostToDevice, st) != cudaSuccess)
         rc = set_error(PTK_ERR_CUDA, "solver initialisation failed");
     if (rc == PTK_OK) rc = uniform_vacuum(s, st, /*clear_index=*/false);
     if (rc == PTK_OK && (long long)p->Nx * p->Ny * p->Nz > kStagedCells) {
@@ -615,7 +632,7 @@ int ptk_solver_destroy(ptk_solver *s)
     {
         std::lock_guard<std::mutex> lk(s->mu);
         drop_graphs(s);
-        pool_free(s->block, st);
+        for (void *q : s->parts) pool_free(q, st);
         pool_free(s->wave, st);
         pool_free(s->d_xch, st);
         if (s->cap) cudaStreamDestroy(s->cap);
@@ -872,7 +889,7 @@ int ptk_selftest_solver_expiry(ptk_solver *s, void *stream)
 int ptk_solver_bytes(const ptk_solver *s, size_t *bytes)
 {
     PTK_CHECK_ARG(s && bytes, "NULL argument");
-    *bytes = s->block_bytes + s->wave_bytes + (s->d_xch ? s->rplan.xch_bytes : 0);
+    *bytes = s->held_bytes + s->wave_bytes + (s->d_xch ? s->rplan.xch_bytes : 0);
     return PTK_OK;
 }
 

@@ -122,3 +122,39 @@ with P.Solver(pr.params) as s:
         except _lib.PtkError as e:
             assert e.code == 3, e.code   # PTK_ERR_NOMEM
 """)
+
+
+@pytest.mark.parametrize("shape,steps", [((40, 33, 21), 9), ((128, 96, 120), 19)])
+def test_a_solver_in_pieces_where_no_block_holds_it(tmp_path, shape, steps):
+    """No allocation larger than one padded array: the solver's arrays come one by one, and go again."""
+    child(tmp_path, f"""
+shape, steps = {shape}, {steps}
+pr, f, ref = problem(shape, steps)
+def used():
+    _lib.call("ptk_device_sync")
+    r, u = C.c_size_t(), C.c_size_t()
+    _lib.call("ptk_pool_stats", C.byref(r), C.byref(u))
+    return u.value
+with P.Solver(pr.params) as s:   # what a first solver sets up once
+    s.set_problem(pr)
+    s.run(steps)
+base = used()
+array = 4 * (-(-(shape[0] + 1) // 32) * 32) * (shape[1] + 1) * (shape[2] + 1)
+limit.value = -(-array // 256) * 256
+with P.Solver(pr.params) as s:
+    assert starved.value >= 2
+    s.set_problem(pr)
+    s.set_fields(f)
+    s.run(steps)
+    same(s.get_fields(), ref)
+    taken = used() - base
+    assert s.nbytes() <= taken <= s.nbytes() + 30 * (2 << 20)
+assert used() == base
+limit.value = limit.value - 256
+try:
+    P.Solver(pr.params)
+    raise SystemExit("no error")
+except _lib.PtkError as e:
+    assert e.code == 3, e.code   # PTK_ERR_NOMEM
+assert used() == base
+""")
