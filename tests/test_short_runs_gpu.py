@@ -73,6 +73,10 @@ def test_default_shape_of_narrow_and_thin_grids(shape, register, dense):
         s.set_problem(pr)
         s.set_fields(f)
         for n in parts:
+            fused = n == 19 and shape[2] >= 8 and not dense
+            staged = fused or not (n in register or 15 in register)   # a launch more, for the walls
+            before = P.launch_count()
             s.run(n)
-            assert s.last_launches() == (n // 2 + 2 if n == 19 and shape[2] >= 8 and not dense else n + 1)
+            assert s.last_launches() == (n // 2 + 2 if fused else n + 1)
+            assert P.launch_count() - before == s.last_launches() + staged + 2   # two set the run up
         check(s, pr, f, sum(parts), shape)
